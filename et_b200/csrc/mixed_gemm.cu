@@ -891,6 +891,15 @@ void split(Exec &ex, const double *src, int64_t sr, int64_t sk, int64_t R, int64
     split_view(ex, matrix_view(src, R, sr, K, sk), R, K, Rp, Kp, planes, out);
 }
 
+// The split count that `splits` cuts nkt K blocks into: the launch gives every slice ceil(nkt / splits)
+// blocks, and a slice that would start at or past the end is left out (nothing would write its
+// partial product).
+int used_splits(int splits, int64_t nkt) {
+    const int64_t s = std::max<int64_t>(1, std::min<int64_t>(splits, nkt));
+    const int64_t per = (nkt + s - 1) / s;
+    return (int)((nkt + per - 1) / per);
+}
+
 int check_planes(int planes) {
     REQUIRE(planes == 2 || planes == 3, CCSD_GPU_EINVAL, "split-bf16 planes must be 2 or 3");
     return planes;
@@ -935,6 +944,7 @@ std::vector<int> tc_split_candidates(int64_t m, int64_t n, int64_t k, int planes
     std::vector<int> out{1};
     auto add = [&](int64_t s, int64_t min_blocks) {
         if (s < 2 || s > 64 || nkt / s < min_blocks) return;
+        s = used_splits((int)s, nkt);
         if (std::find(out.begin(), out.end(), (int)s) == out.end()) out.push_back((int)s);
     };
     add(tc_default_splits(m, n, k, planes), 1);
@@ -963,7 +973,7 @@ void mixed_gemm_views(Exec &ex, const SplitView &A, const SplitView &B, int64_t 
     const bool pair = splits >= PAIR_ROUTE;
     if (pair) splits -= PAIR_ROUTE;
     if (splits <= 0) splits = tc_default_splits(m, n, k, np);
-    splits = std::max(1, std::min<int>(splits, (int)(Kp / BK)));
+    splits = used_splits(splits, Kp / BK);
     const double mnk = double(m) * double(n) * double(k);
     if (splits <= 1) {
         EpiF64 epi{C, (long long)ldc, (int)m, (int)n, alpha, beta};
@@ -1020,7 +1030,7 @@ void tc_gemm_f64(Exec &ex, const __nv_bfloat16 *A, int64_t Mp, const __nv_bfloat
     const bool pair = splits >= PAIR_ROUTE;
     if (pair) splits -= PAIR_ROUTE;
     if (splits <= 0) splits = wave_splits(Mp / BM * (round_up(n, n_tile(np)) / n_tile(np)), Kp / BK);
-    splits = std::max(1, std::min<int>(splits, (int)(Kp / BK)));
+    splits = used_splits(splits, Kp / BK);
     if (splits == 1) {
         EpiF64 epi{C, (long long)ldc, (int)m, (int)n, alpha, beta};
         launch_tc(ex, np, A, Mp, Mp * Kp, m, B, Np, Np * Kp, n, Kp, epi, mnk, 1, pair);
