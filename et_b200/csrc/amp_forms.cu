@@ -1,0 +1,185 @@
+// Bandwidth kernels between the packed doubles and full (v,o,v,o) arrays (FP64).
+//
+// For a fixed occupied pair i <= j the packed element of (ai, bj) is T_ij[a, b], contiguous along a
+// (ai never exceeds bj for i < j), and everything the full forms need of it lies in the same pair:
+// S_aibj = T[a, b], S_ajbi = T[b, a], and the mirrored block (bj, ai) is the transpose.  A block of
+// threads therefore takes one occupied pair and a 32 x 32 tile of (a, b) with its mirror tile: each
+// packed element is read once, each full element written (or read) once, all along a.
+#include <algorithm>
+#include <type_traits>
+
+#include "amp_forms.cuh"
+
+namespace ccsd {
+
+namespace {
+
+constexpr int TILE = 32, ROWS = 8;
+// 48 warps of sym_pack on an SM: 0.35 ms at o=32, v=320 where its natural 78 registers (24 warps) take 0.51 ms
+constexpr int MIN_BLOCKS = 6;
+
+// (M, m) with M >= m from M(M+1)/2 + m
+__device__ __forceinline__ void untri32(unsigned idx, int &M, int &m) {
+    int r = (int)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
+    while ((unsigned)r * (unsigned)(r + 1) / 2 > idx) r--;
+    while ((unsigned)(r + 1) * (unsigned)(r + 2) / 2 <= idx) r++;
+    M = r;
+    m = (int)(idx - (unsigned)r * (unsigned)(r + 1) / 2);
+}
+
+__device__ __forceinline__ int64_t packed_at(int64_t x, int64_t y) {
+    const int64_t M = x > y ? x : y, m = x > y ? y : x;
+    return M * (M + 1) / 2 + m;
+}
+
+__device__ __forceinline__ void put(double *p, double v, int acc) { *p = acc ? *p + v : v; }
+
+// Bound by HBM: n_t2 read, 2 (o v)^2 written.  At o=32, v=320 it takes 0.41 ms (5.1 TB/s) where the
+// element-wise square-up and the two exchange passes that formed u took 1.19 ms.
+__global__ void __launch_bounds__(TILE * ROWS)
+square_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec, double c1, double c2,
+                    double *__restrict__ S, double *__restrict__ U, int acc_s, int acc_u) {
+    __shared__ double t1[TILE][TILE + 1], t2[TILE][TILE + 1];   // T[a0 + x, b0 + r], T[b0 + x, a0 + r] at [r][x]
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int64_t nov = (int64_t)no * nv, nt2 = nov * (nov + 1) / 2;
+    const int64_t npair = (int64_t)no * (no + 1) / 2;
+    int at, bt, i, j;
+    untri32(blockIdx.x, bt, at);
+    const int a0 = TILE * at, b0 = TILE * bt;
+    const bool mirror = at != bt;
+    for (int64_t w = blockIdx.y; w < npair * nvec; w += gridDim.y) {
+        const int64_t n = w / npair, vec = nov * nov * n;
+        untri32((unsigned)(w - n * npair), j, i);
+        const double *p = packed + nt2 * n;
+        for (int r = ty; r < TILE; r += ROWS) {
+            if (a0 + tx < nv && b0 + r < nv) t1[r][tx] = p[packed_at(a0 + tx + (int64_t)nv * i, b0 + r + (int64_t)nv * j)];
+            if (mirror && b0 + tx < nv && a0 + r < nv)
+                t2[r][tx] = p[packed_at(b0 + tx + (int64_t)nv * i, a0 + r + (int64_t)nv * j)];
+        }
+        __syncthreads();
+        double(*m2)[TILE + 1] = mirror ? t2 : t1;
+        for (int r = ty; r < TILE; r += ROWS) {
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+                if (side && !mirror) break;
+                const int x = (side ? b0 : a0) + tx, y = (side ? a0 : b0) + r;
+                if (x >= nv || y >= nv) continue;
+                const double d = side ? m2[r][tx] : t1[r][tx];       // T[x, y]
+                const double e = side ? t1[tx][r] : m2[tx][r];       // T[y, x]
+                const int64_t ij = vec + x + (int64_t)nv * i + nov * (y + (int64_t)nv * j);
+                const int64_t ji = vec + x + (int64_t)nv * j + nov * (y + (int64_t)nv * i);
+                if (S) put(S + ij, d, acc_s);
+                if (U) put(U + ij, c1 * d + c2 * e, acc_u);
+                if (i != j) {
+                    if (S) put(S + ji, e, acc_s);
+                    if (U) put(U + ji, c1 * e + c2 * d, acc_u);
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Bound by HBM: F and X read once, n_t2 written.  At o=32, v=320 0.35 ms (5.9 TB/s); adding the two
+// forms of X to F in passes of their own and packing the sum took 1.26 ms.
+template <bool HAS_F, bool HAS_X, bool ACC>
+__global__ void __launch_bounds__(TILE * ROWS, MIN_BLOCKS)
+sym_pack_kernel(const double *__restrict__ F, const double *__restrict__ X, int no, int nv, int64_t nvec, double c1,
+                double c2, double *__restrict__ packed) {
+    constexpr int N = TILE / ROWS;
+    __shared__ double s1[TILE][TILE + 1], s2[TILE][TILE + 1];   // Z_ji of the tile and of its mirror
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int64_t nov = (int64_t)no * nv, nt2 = nov * (nov + 1) / 2;
+    const int64_t npair = (int64_t)no * (no + 1) / 2;
+    int at, bt, i, j;
+    untri32(blockIdx.x, bt, at);
+    const int a0 = TILE * at, b0 = TILE * bt;
+    const bool mirror = at != bt;
+    for (int64_t w = blockIdx.y; w < npair * nvec; w += gridDim.y) {
+        const int64_t n = w / npair, vec = nov * nov * n;
+        untri32((unsigned)(w - n * npair), j, i);
+        double *p = packed + nt2 * n;
+        double z[2][N];     // Z_ij of the two tiles
+        double old[2][N];   // what the results are added to, loaded before any store
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            if (side && !mirror) break;
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                const int r = ty + ROWS * k;
+                const int x = (side ? b0 : a0) + tx, y = (side ? a0 : b0) + r;
+                double zij = 0.0, zji = 0.0;
+                if (x < nv && y < nv) {
+                    if (ACC) {
+                        const int64_t M = y + (int64_t)nv * j;   // i == j: the other triangle is not stored
+                        old[side][k] = i == j && x > y ? 0.0 : p[M * (M + 1) / 2 + x + (int64_t)nv * i];
+                    }
+                    const int64_t ij = vec + x + (int64_t)nv * i + nov * (y + (int64_t)nv * j);
+                    const int64_t ji = vec + x + (int64_t)nv * j + nov * (y + (int64_t)nv * i);
+                    if (HAS_F) {
+                        zij = F[ij];
+                        zji = F[ji];
+                    }
+                    if (HAS_X) {
+                        const double xij = X[ij], xji = X[ji];
+                        zij += c1 * xij + c2 * xji;
+                        zji += c1 * xji + c2 * xij;
+                    }
+                }
+                z[side][k] = zij;
+                if (side) s2[r][tx] = zji;
+                else s1[r][tx] = zji;
+            }
+        }
+        __syncthreads();
+        double(*m2)[TILE + 1] = mirror ? s2 : s1;
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            if (side && (!mirror || i == j)) break;   // i == j: the mirror tile is the other triangle
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                const int r = ty + ROWS * k;
+                const int x = (side ? b0 : a0) + tx, y = (side ? a0 : b0) + r;
+                if (x >= nv || y >= nv || (i == j && x > y)) continue;
+                double v = z[side][k] + (side ? s1[tx][r] : m2[tx][r]);
+                if (i == j && x == y) v *= 0.5;
+                const int64_t M = y + (int64_t)nv * j;
+                p[M * (M + 1) / 2 + x + (int64_t)nv * i] = ACC ? old[side][k] + v : v;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+dim3 pair_grid(int64_t no, int64_t nv, int64_t nvec) {
+    const int64_t nt = (nv + TILE - 1) / TILE;
+    return dim3((unsigned)(nt * (nt + 1) / 2), (unsigned)std::min<int64_t>(no * (no + 1) / 2 * nvec, 65535));
+}
+
+}  // namespace
+
+void square_forms(Exec &ex, const double *p, int64_t no, int64_t nv, int64_t nvec, double c1, double c2, double *S,
+                  double *U, bool acc_s, bool acc_u) {
+    square_forms_kernel<<<pair_grid(no, nv, nvec), dim3(TILE, ROWS), 0, ex.stream>>>(p, (int)no, (int)nv, nvec, c1, c2, S,
+                                                                                    U, acc_s, acc_u);
+    ex.launches++;
+    CU_CHECK(cudaGetLastError());
+}
+
+void sym_pack(Exec &ex, const double *F, const double *X, int64_t no, int64_t nv, int64_t nvec, double c1, double c2,
+              double *p, bool accumulate) {
+    auto run = [&](auto f, auto x, auto acc) {
+        sym_pack_kernel<decltype(f)::value, decltype(x)::value, decltype(acc)::value>
+            <<<pair_grid(no, nv, nvec), dim3(TILE, ROWS), 0, ex.stream>>>(F, X, (int)no, (int)nv, nvec, c1, c2, p);
+    };
+    const std::true_type yes;
+    const std::false_type none;
+    auto pick = [&](auto f, auto x) { accumulate ? run(f, x, yes) : run(f, x, none); };
+    if (F && X) pick(yes, yes);
+    else if (F) pick(yes, none);
+    else pick(none, yes);
+    ex.launches++;
+    CU_CHECK(cudaGetLastError());
+}
+
+}  // namespace ccsd

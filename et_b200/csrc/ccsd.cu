@@ -11,6 +11,7 @@
 #include <cstring>
 #include <memory>
 
+#include "amp_forms.cuh"
 #include "autotune.cuh"
 #include "ccsd.cuh"
 #include "ccsd_kernels.cuh"
@@ -700,7 +701,7 @@ void Context::ladder_y_t1(const double *t1, const double *Ltvv, const double *tf
              tv(Y, {no, no, nv, no}));
 }
 
-// The A2 ladder of the residual on the tensor cores, without forming T1-transformed integrals.
+// The A2 ladder of the residual without forming T1-transformed integrals.
 // With L~_vv = L_vv - t1 L_ov (the T1 transformation of the vv block),
 //   g~_acbd = g_acbd - sum_k t_ak g_kcbd - sum_l t_bl g_acld + sum_kl t_ak t_bl g_kcld,
 // so X_aibj = sum_cd g~_acbd t_cidj (symmetric in ai <-> bj) is
@@ -708,35 +709,22 @@ void Context::ladder_y_t1(const double *t1, const double *Ltvv, const double *tf
 //   Y_kibj = sum_cd g_kcbd t_cidj,   T4_aibj = sum_kl t_ak t_bl Q_kilj,   Q_kilj = sum_cd g_kcld t_cidj,
 // (the A^T term uses sum_cd g_acld t_cidj = Y_ljai), all with untransformed integrals: the v^4
 // integrals are formed once per Cholesky set instead of every iteration, the corrections cost
-// o^2 v^3 N_J + o^3 v^3.  The ladder adds pack(X) with the doubles diagonal halved to om2.
-void Context::ladder_residual_mixed(const double *t1, const double *tf, const double *t2, double *om2) {
+// o^2 v^3 N_J + o^3 v^3.  om is packed as om + om^T, so the corrections enter it as -A + T4/2.
+void Context::ladder_t1_corrections(const double *t1, const double *tf, double *om) {
     cudaStream_t s = ex.stream;
-    ladder_tc(L_vv.d(), t2, om2, 1, true);
-    DBuf Y = dalloc(no * no * nv * no, s);
-    if (ovvv_resident()) ladder_y0(tf, Y.d());
-    else ladder_y(L_vv.d(), tf, Y.d());
-    ladder_t1_corrections(t1, tf, Y.d(), om2);
-}
-
-void Context::ladder_t1_corrections(const double *t1, const double *tf, const double *Y0, double *om2) {
-    cudaStream_t s = ex.stream;
-    // the terms below are A_aibj (not symmetric); omega gets pack(A + A^T) with the diagonal halved
-    DBuf A = dalloc(nov * nov, s);
-    contract(ex, "ak,kibj->aibj", -1.0, tv(t1, {nv, no}), tv(Y0, {no, no, nv, no}), 0.0,
-             tv(A.d(), {nv, no, nv, no}));
-    {
-        DBuf Q = dalloc(no * no * no * no, s), B = dalloc(nv * no * no * no, s);
-        contract(ex, "kcld,cidj->kilj", 1.0, tv(g_ovov_const(), {no, nv, no, nv}), tv(tf, {nv, no, nv, no}), 0.0,
-                 tv(Q.d(), {no, no, no, no}));
-        contract(ex, "ak,kilj->ailj", 1.0, tv(t1, {nv, no}), tv(Q.d(), {no, no, no, no}), 0.0,
-                 tv(B.d(), {nv, no, no, no}));
-        // the symmetric term sum_l t_bl B_ailj enters at half weight (pack(A + A^T) adds it twice), in
-        // its mirrored form sum_l t_al B_bjli, whose output index order (a | i, b, j) lies in A's own
-        // layout, so the product writes A in place instead of through a reordered copy
-        contract(ex, "al,bjli->aibj", 0.5, tv(t1, {nv, no}), tv(B.d(), {nv, no, no, no}), 1.0,
-                 tv(A.d(), {nv, no, nv, no}));
-    }
-    pack_sym_add(ex, A.d(), om2, nov);
+    DBuf Y0 = dalloc(no * no * nv * no, s);
+    ladder_y_plain(tf, Y0.d());
+    contract(ex, "ak,kibj->aibj", -1.0, tv(t1, {nv, no}), tv(Y0.d(), {no, no, nv, no}), 1.0,
+             tv(om, {nv, no, nv, no}));
+    DBuf Q = dalloc(no * no * no * no, s), B = dalloc(nv * no * no * no, s);
+    contract(ex, "kcld,cidj->kilj", 1.0, tv(g_ovov_const(), {no, nv, no, nv}), tv(tf, {nv, no, nv, no}), 0.0,
+             tv(Q.d(), {no, no, no, no}));
+    contract(ex, "ak,kilj->ailj", 1.0, tv(t1, {nv, no}), tv(Q.d(), {no, no, no, no}), 0.0,
+             tv(B.d(), {nv, no, no, no}));
+    // the symmetric term sum_l t_bl B_ailj enters at half weight, in its mirrored form sum_l t_al B_bjli,
+    // whose output index order (a | i, b, j) lies in om's own layout
+    contract(ex, "al,bjli->aibj", 0.5, tv(t1, {nv, no}), tv(B.d(), {nv, no, no, no}), 1.0,
+             tv(om, {nv, no, nv, no}));
 }
 
 // FP64 integrals of the untransformed vectors, resident while they fit in half of the free memory
@@ -820,39 +808,52 @@ int Context::f64_digit_planes(int digits) {
     return f64_dig_level;
 }
 
-void Context::ladder_residual_f64(const double *t1, const double *tf, const double *t2, double *om2) {
+// The int8 digit GEMM takes the FP64 ladder products under the same size rule as gemm(); their constant
+// operands then come as digit planes kept per Cholesky set
+int Context::f64_ladder_digits() {
+    const int64_t nop = no * (no + 1) / 2, nvp = nv * (nv + 1) / 2;
+    const bool big = ex.fp64_digits > 0 && 2.0 * double(nop) * double(nvp) * double(nvp) >= ex.fp64_digits_min_flops &&
+                     (ex.fp64_digits_min_flops <= 1 || (nop >= 256 && nvp >= 256));
+    return big ? ex.fp64_digits : 0;
+}
+
+void Context::ladder_f64(const double *t2, double *om2) {
     f64_integrals();
     cudaStream_t s = ex.stream;
     const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
     const int64_t ldm = std::max<int64_t>(nom, 1);
-    // on the digit GEMM the constant operands come as digit planes kept per Cholesky set (products
-    // big enough for it, as gemm() decides)
-    const int digits = ex.fp64_digits;
-    const bool big = digits > 0 && 2.0 * double(nop) * double(nvp) * double(nvp) >= ex.fp64_digits_min_flops &&
-                     (ex.fp64_digits_min_flops <= 1 || (nop >= 256 && nvp >= 256));
-    const int level = big ? f64_digit_planes(digits) : 0;
+    const int digits = f64_ladder_digits();
+    const int level = digits ? f64_digit_planes(digits) : 0;
     // X0 = sum_cd g_acbd t_cidj of the untransformed integrals, all pairs in two GEMMs
-    {
-        DBuf tp = dalloc(nop * nvp, s), tm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
-        build_tpm(ex, t2, tp.d(), tm.d(), no, nv, nop, ldm);
-        DBuf wp = dalloc(nop * nvp, s), wm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
-        if (level >= 1) {
-            ozaki_gemm(ex, false, false, nop, nvp, nvp, 0.5, tp.d(), nop, f64_gp.d(), nvp, 0.0, wp.d(), nop, digits,
-                       nullptr, &f64_gp_dig);
-            if (nom > 0 && nvm > 0)
-                ozaki_gemm(ex, false, false, nom, nvm, nvm, 0.5, tm.d(), ldm, f64_gm.d(), nvm, 0.0, wm.d(), ldm,
-                           digits, nullptr, &f64_gm_dig);
-            ex.flops += 2.0 * (double(nop) * nvp * nvp + double(nom) * nvm * nvm);
-        } else {
-            gemm(ex, false, false, nop, nvp, nvp, 0.5, tp.d(), nop, f64_gp.d(), nvp, 0.0, wp.d(), nop, false);
-            if (nom > 0 && nvm > 0)
-                gemm(ex, false, false, nom, nvm, nvm, 0.5, tm.d(), ldm, f64_gm.d(), nvm, 0.0, wm.d(), ldm, false);
-        }
-        add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, 0, nv, nop, ldm);
+    DBuf tp = dalloc(nop * nvp, s), tm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
+    build_tpm(ex, t2, tp.d(), tm.d(), no, nv, nop, ldm);
+    DBuf wp = dalloc(nop * nvp, s), wm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
+    if (level >= 1) {
+        ozaki_gemm(ex, false, false, nop, nvp, nvp, 0.5, tp.d(), nop, f64_gp.d(), nvp, 0.0, wp.d(), nop, digits,
+                   nullptr, &f64_gp_dig);
+        if (nom > 0 && nvm > 0)
+            ozaki_gemm(ex, false, false, nom, nvm, nvm, 0.5, tm.d(), ldm, f64_gm.d(), nvm, 0.0, wm.d(), ldm, digits,
+                       nullptr, &f64_gm_dig);
+        ex.flops += 2.0 * (double(nop) * nvp * nvp + double(nom) * nvm * nvm);
+    } else {
+        gemm(ex, false, false, nop, nvp, nvp, 0.5, tp.d(), nop, f64_gp.d(), nvp, 0.0, wp.d(), nop, false);
+        if (nom > 0 && nvm > 0)
+            gemm(ex, false, false, nom, nvm, nvm, 0.5, tm.d(), ldm, f64_gm.d(), nvm, 0.0, wm.d(), ldm, false);
     }
-    DBuf Y = dalloc(no * no * nv * no, s);
-    if (level == 2) {
+    add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, 0, nv, nop, ldm);
+}
+
+void Context::ladder_y_plain(const double *tf, double *Y) {
+    if (ex.prec == Prec::MIXED) {
+        if (ovvv_resident()) ladder_y0(tf, Y);
+        else ladder_y(L_vv.d(), tf, Y);
+        return;
+    }
+    f64_integrals();
+    cudaStream_t s = ex.stream;
+    const int digits = f64_ladder_digits();
+    if (digits && f64_digit_planes(digits) == 2) {
         // Y_kibj = sum_cd g_kbcd t_cidj: t as [(c, d), (i, j)], the product [(k, b), (i, j)], then Y
         DBuf TT = dalloc(nv * nv * no * no, s), W = dalloc(nov * no * no, s);
         TV tt = tv(TT.d(), {nv, no, nv, no});   // (c, i, d, j) at c + nv d + nv^2 (i + no j)
@@ -867,12 +868,11 @@ void Context::ladder_residual_f64(const double *t1, const double *tf, const doub
         w.s[1] = no * nv;
         w.s[2] = no;
         w.s[3] = no * nv * no;
-        permute_add(ex, 1.0, w, 0.0, tv(Y.d(), {no, no, nv, no}));
+        permute_add(ex, 1.0, w, 0.0, tv(Y, {no, no, nv, no}));
     } else {
         contract(ex, "kbcd,cidj->kibj", 1.0, tv(f64_ovvv.d(), {no, nv, nv, nv}), tv(tf, {nv, no, nv, no}), 0.0,
-                 tv(Y.d(), {no, no, nv, no}));
+                 tv(Y, {no, no, nv, no}));
     }
-    ladder_t1_corrections(t1, tf, Y.d(), om2);
 }
 
 // ---------------------------------------------------------------------------

@@ -142,7 +142,8 @@ struct Context {
     // const_t1: take the T1-transformed blocks and the Fock matrix from the context (only when no
     // derivative will be taken and t1_current holds)
     OmegaNodes record_omega(Graph &g, bool const_ovov = true, bool const_t1 = false);
-    void record_ladder(Graph &g, int om2, int Lvv, int t2, int t1, int L_vv_in, int tf);
+    void record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, int tf);
+    void record_ladder(Graph &g, int om2, int Lvv, int t2);
     void ladder_y(const double *Lvv, const double *tfull, double *Y);
     // mixed precision: whether the resident ovvv planes fit, their construction, and
     // Y0_kibj = sum_cd g_kcbd tau_cidj from them
@@ -181,14 +182,17 @@ struct Context {
     TPlanes t_planes(const double *t2, int64_t nvec);
     void ladder_pm_block(const TPlanes &T, int64_t nvec, const __nv_bfloat16 *Pp, int64_t prow, const __nv_bfloat16 *Pm,
                          int64_t mrow, int64_t a0, int64_t a1, double *om2);
-    // the residual's ladder in mixed precision from untransformed integrals plus t1 corrections
-    void ladder_residual_mixed(const double *t1, const double *tf, const double *t2, double *om2);
-    // om2 += pack(-(A + A^T) + T4) with A_aibj = sum_k t_ak Y0_kibj, T4 = sum_kl t_ak t_bl Q_kilj
-    void ladder_t1_corrections(const double *t1, const double *tf, const double *Y0, double *om2);
-    // the same ladder in FP64 from resident FP64 integrals (f64_resident() must hold)
+    // Y0_kibj = sum_cd g_kcbd tau_cidj of the untransformed vectors, from whatever integrals the
+    // current precision keeps
+    void ladder_y_plain(const double *tfull, double *Y);
+    // om += -A + T4/2 with A_aibj = sum_k t_ak Y0_kibj, T4 = sum_kl t_ak t_bl Q_kilj (om is packed as
+    // om + om^T)
+    void ladder_t1_corrections(const double *t1, const double *tf, double *om);
+    // the t2 ladder in FP64 from resident FP64 integrals (f64_resident() must hold)
     bool f64_resident();
     void f64_integrals();
-    void ladder_residual_f64(const double *t1, const double *tf, const double *t2, double *om2);
+    int f64_ladder_digits();                 // digits of its products on the digit GEMM, 0: DGEMM
+    void ladder_f64(const double *t2, double *om2);
     // digit planes of the resident FP64 integrals for FP64 evaluations on the int8 digit GEMM: the
     // +/- ladder integrals (B operands) and g_kcbd (A operand of Y), kept per Cholesky set and digit
     // count while they fit (levels: 2 all three, 1 the ladder pair only, 0 none)

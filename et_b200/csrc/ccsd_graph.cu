@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <memory>
 
+#include "amp_forms.cuh"
 #include "ccsd.cuh"
 #include "ccsd_kernels.cuh"
 #include "graph.cuh"
@@ -68,7 +69,8 @@ __global__ void join_amp_kernel(const double *__restrict__ x1, const double *__r
 // ---------------------------------------------------------------------------
 OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
     OmegaNodes n{};
-    g.nov = nov;
+    g.no = no;
+    g.nv = nv;
     const std::vector<int64_t> V4 = {nv, no, nv, no};
     n.t1 = g.input("t1", {nv, no}, t.d());
     n.t2 = g.input("t2", {nt2}, t.d() + nt1);
@@ -149,9 +151,7 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
     const int u = g.zeros("u_aibj", V4);                             // construct_u_aibj (omega_ccsd.F90:881)
     {
         TermTimer tt(ex, "Construct u_aibj");
-        g.squareup(tf, n.t2);                                        // squareup (reordering.F90:4174)
-        g.permute(u, "aibj->aibj", 2.0, tf);
-        g.permute(u, "ajbi->aibj", -1.0, tf);
+        g.square_forms(tf, u, n.t2, 2.0, -1.0);                      // squareup (reordering.F90:4174), 2 t_aibj - t_ajbi
     }
     {
         // omega_doubles_a1 (src/wavefunctions/doubles/omega_doubles.F90:36-138)
@@ -182,7 +182,7 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         g.contract(G4, "Jia,Jjb->iajb", 1.0, Lt_ov, Lt_ov);
     }
     // omega_ccsd_e2 (omega_ccsd.F90:712-878); Fock parts in FP64
-    const int om = g.zeros("omega_aibj", V4);
+    const int om = g.zeros("omega_aibj", V4), x = g.zeros("x_c2", V4);
     {
         TermTimer tt(ex, "omega ccsd e2");
         const int Xbc = g.zeros("X_bc", {nv, nv}), Ykj = g.zeros("Y_kj", {no, no});
@@ -195,8 +195,9 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         g.contract(om, "bc,cjai->bjai", 1.0, Xbc, tf, true);
         g.contract(om, "aibk,kj->aibj", -1.0, tf, Ykj, true);
     }
-    // om collects the terms that eT symmetrises (symmetric_sum, reordering.F90:416): the doubles
-    // residual is pack(om + om^T) with the diagonal halved, formed in one pass at the end.  Terms
+    // om collects the terms that eT symmetrises (symmetric_sum, reordering.F90:416), x the C2 term whose
+    // third and exchanged two thirds join them: the doubles residual is pack(z + z^T), z = om + x_aibj/3
+    // + 2 x_ajbi/3, with the diagonal halved, formed in one pass at the end.  Terms
     // that are symmetric already enter with weight 1/2.
     // omega_ccsd_b2 (omega_ccsd.F90:483-583); g_aibj in FP64
     {
@@ -225,16 +226,14 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
             g.permute(H, "kcld->lckd", -0.5, G4);
         }
         g.contract(D, "lckd,dkaj->claj", 1.0, H, u);
-        const int x = g.zeros("x_c2", V4);
         g.contract(x, "akci,ckbj->aibj", -1.5, tf, C);
         g.contract(om, "aick,ckbj->aibj", 0.5, u, D);
-        g.permute(om, "aibj->aibj", 1.0 / 3.0, x);
-        g.permute(om, "ajbi->aibj", 2.0 / 3.0, x);
     }
+    // omega_ccsd_a2 (omega_ccsd.F90:113-480) as custom ops: its t1 part joins om, its t2 part the packed residual
+    record_ladder_t1(g, om, Lt_vv, t1, n.L_vv, tf);
     const int om2 = g.zeros("omega2", {nt2});
-    g.pack_sym(om2, om);                     // symmetric_sum + scale_diagonal(1/2) + packin
-    // omega_ccsd_a2 (omega_ccsd.F90:113-480) as a custom op
-    record_ladder(g, om2, Lt_vv, n.t2, t1, n.L_vv, tf);
+    g.sym_pack(om2, om, x, 1.0 / 3.0, 2.0 / 3.0);   // symmetric_sum + scale_diagonal(1/2) + packin
+    record_ladder(g, om2, Lt_vv, n.t2);
     n.om1 = om1;
     n.om2 = om2;
     return n;
@@ -261,9 +260,12 @@ void Context::ladder_y(const double *Lvv, const double *tfull, double *Y) {
     }
 }
 
-void Context::record_ladder(Graph &g, int om2, int Lvv, int t2, int t1, int L_vv_in, int tf) {
+// The part of the A2 ladder that depends on t1, as terms A_aibj of om (which is packed as A + A^T): in
+// the residual the corrections that turn integrals of the untransformed vectors into T1-transformed
+// ones (nothing when the integrals are formed from transformed vectors); in the derivative passes the
+// t1 derivative through Y.
+void Context::record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, int tf) {
     auto Ycache = std::make_shared<DBuf>();
-    auto LTcache = std::make_shared<DBuf>();
     auto getY = [this, &g, Lvv, t1, tf, Ycache]() -> const double * {
         if (!*Ycache) {
             *Ycache = dalloc(no * no * nv * no, ex.stream);
@@ -271,6 +273,54 @@ void Context::record_ladder(Graph &g, int om2, int Lvv, int t2, int t1, int L_vv
         }
         return Ycache->d();
     };
+    CustomOp op;
+    op.forward = [this, &g, om, t1, tf]() {
+        TermTimer tt(ex, "omega ccsd a2");
+        if (ex.prec == Prec::MIXED || f64_resident()) ladder_t1_corrections(g.value(t1), g.value(tf), g.node(om).v);
+    };
+    op.tangent = [this, &g, om, Lvv, t1, getY](int nvec) {
+        REQUIRE(!g.node(Lvv).active || g.node(t1).active, CCSD_GPU_EINVAL,
+                "ladder tangent: L_vv directions are not supported");
+        if (!g.node(t1).active) return;
+        // d L~_ac = -sum_k c_ak L_kc: A_aibj = -sum_k c_ak Y_kibj
+        double *out = g.tangent(om, nvec);
+        const double *Y = getY(), *c1 = g.tangent(t1, nvec);
+        for (int n = 0; n < nvec; n++)
+            contract(ex, "ak,kibj->aibj", -1.0, tv(c1 + n * nt1, {nv, no}), tv(Y, {no, no, nv, no}), 1.0,
+                     tv(out + n * nov * nov, {nv, no, nv, no}));
+    };
+    op.adjoint = [this, &g, om, Lvv, t1, tf, L_vv_in, getY](int nvec) {
+        // adjoint into the Cholesky vectors requested: dense route through L~_vv (its adjoint also
+        // reaches t1 through the recorded T1 transformation); otherwise the rank-n_o route via Y.  The
+        // adjoint of om is the symmetric square-up S of the packed residual's adjoint.
+        const bool dense = g.node(L_vv_in).active;
+        if (!g.node(t1).active && !dense) return;
+        const double *S = g.adjoint(om, nvec);
+        for (int n = 0; n < nvec; n++) {
+            const TV B = tv(S + n * nov * nov, {nv, no, nv, no});
+            if (!dense) {
+                // t1bar_ak -= sum_ibj S_aibj Y_kibj
+                contract(ex, "aibj,kibj->ak", -1.0, B, tv(getY(), {no, no, nv, no}), 1.0,
+                         tv(g.adjoint(t1, nvec) + n * nt1, {nv, no}));
+            } else {
+                // Lbar_J,ac += sum_bd L_J,bd Z_acbd, Z_acbd = sum_ij S_aibj t_cidj
+                REQUIRE((double)nv * nv * nv * nv * 8.0 < 24e9, CCSD_GPU_EINVAL,
+                        "ladder adjoint into L_vv needs v^4 doubles of scratch; system too large");
+                DBuf Z = dalloc(nv * nv * nv * nv, ex.stream);
+                contract(ex, "aibj,cidj->acbd", 1.0, B, tv(g.value(tf), {nv, no, nv, no}), 0.0,
+                         tv(Z.d(), {nv, nv, nv, nv}));
+                contract(ex, "Jbd,acbd->Jac", 1.0, tv(g.value(Lvv), {nJ, nv, nv}), tv(Z.d(), {nv, nv, nv, nv}), 1.0,
+                         tv(g.adjoint(Lvv, nvec) + n * nJ * nv * nv, {nJ, nv, nv}));
+            }
+        }
+    };
+    g.custom(std::move(op), om, {Lvv, t1, tf});
+}
+
+// sum_cd g_acbd t_cidj into the packed residual: in the residual with integrals of the untransformed
+// vectors where they are kept, in the derivative passes with the T1-transformed ones
+void Context::record_ladder(Graph &g, int om2, int Lvv, int t2) {
+    auto LTcache = std::make_shared<DBuf>();
     auto getLT = [this, &g, Lvv, LTcache]() -> const double * {
         if (!*LTcache) {
             *LTcache = dalloc(nJ * nv * nv, ex.stream);
@@ -283,69 +333,23 @@ void Context::record_ladder(Graph &g, int om2, int Lvv, int t2, int t1, int L_vv
         return LTcache->d();
     };
     CustomOp op;
-    op.forward = [this, &g, om2, Lvv, t2, t1, tf]() {
+    op.forward = [this, &g, om2, Lvv, t2]() {
         TermTimer tt(ex, "omega ccsd a2");
         if (ex.prec == Prec::MIXED)
-            ladder_residual_mixed(g.value(t1), g.value(tf), g.value(t2), g.node(om2).v);
+            ladder_tc(L_vv.d(), g.value(t2), g.node(om2).v, 1, true);
         else if (f64_resident())
-            ladder_residual_f64(g.value(t1), g.value(tf), g.value(t2), g.node(om2).v);
+            ladder_f64(g.value(t2), g.node(om2).v);
         else
             ladder(g.value(Lvv), g.value(t2), g.node(om2).v);
     };
-    op.tangent = [this, &g, om2, Lvv, t2, t1, getY](int nvec) {
-        REQUIRE(!g.node(Lvv).active || g.node(t1).active, CCSD_GPU_EINVAL,
-                "ladder tangent: L_vv directions are not supported");
-        double *out = g.tangent(om2, nvec);
-        if (g.node(t2).active) {
-            const double *c2 = g.tangent(t2, nvec);
-            ladder(g.value(Lvv), c2, out, nvec);
-        }
-        if (g.node(t1).active) {
-            // d L~_ac = -sum_k c_ak L_kc: term -P(sum_k c_ak Y_kibj + (ai <-> bj))
-            const double *Y = getY();
-            const double *c1 = g.tangent(t1, nvec);
-            DBuf A = dalloc(nov * nov, ex.stream);
-            for (int n = 0; n < nvec; n++) {
-                contract(ex, "ak,kibj->aibj", -1.0, tv(c1 + n * nt1, {nv, no}), tv(Y, {no, no, nv, no}), 0.0,
-                         tv(A.d(), {nv, no, nv, no}));
-                pack_sym_add(ex, A.d(), out + n * nt2, nov);   // pack(A + A^T), diagonal halved
-            }
-        }
+    op.tangent = [this, &g, om2, Lvv, t2](int nvec) {
+        if (g.node(t2).active) ladder(g.value(Lvv), g.tangent(t2, nvec), g.tangent(om2, nvec), nvec);
     };
-    op.adjoint = [this, &g, om2, Lvv, t2, t1, tf, L_vv_in, getY, getLT](int nvec) {
-        // adjoint into the Cholesky vectors requested: dense route through L~_vv (its adjoint also
-        // reaches t1 through the recorded T1 transformation); otherwise the rank-n_o route via Y
-        const bool dense = g.node(L_vv_in).active;
-        const double *pbar = g.adjoint(om2, nvec);
-        if (g.node(t2).active) {
-            // the transpose of the packed ladder is the same ladder with L~_vv transposed
-            const double *LT = getLT();
-            double *t2bar = g.adjoint(t2, nvec);
-            ladder(LT, pbar, t2bar, nvec);
-        }
-        if (g.node(t1).active || dense) {
-            DBuf B = dalloc(nov * nov, ex.stream);
-            for (int n = 0; n < nvec; n++) {
-                squareup(ex, pbar + n * nt2, B.d(), nov);
-                if (g.node(t1).active && !dense) {
-                    // t1bar_ak -= sum_ibj S(pbar)_aibj Y_kibj
-                    contract(ex, "aibj,kibj->ak", -1.0, tv(B.d(), {nv, no, nv, no}), tv(getY(), {no, no, nv, no}),
-                             1.0, tv(g.adjoint(t1, nvec) + n * nt1, {nv, no}));
-                }
-                if (dense) {
-                    // Lbar_J,ac += sum_bd L_J,bd Z_acbd, Z_acbd = sum_ij S(pbar)_aibj t_cidj
-                    REQUIRE((double)nv * nv * nv * nv * 8.0 < 24e9, CCSD_GPU_EINVAL,
-                            "ladder adjoint into L_vv needs v^4 doubles of scratch; system too large");
-                    DBuf Z = dalloc(nv * nv * nv * nv, ex.stream);
-                    contract(ex, "aibj,cidj->acbd", 1.0, tv(B.d(), {nv, no, nv, no}), tv(g.value(tf), {nv, no, nv, no}),
-                             0.0, tv(Z.d(), {nv, nv, nv, nv}));
-                    contract(ex, "Jbd,acbd->Jac", 1.0, tv(g.value(Lvv), {nJ, nv, nv}), tv(Z.d(), {nv, nv, nv, nv}), 1.0,
-                             tv(g.adjoint(Lvv, nvec) + n * nJ * nv * nv, {nJ, nv, nv}));
-                }
-            }
-        }
+    op.adjoint = [this, &g, om2, t2, getLT](int nvec) {
+        // the transpose of the packed ladder is the same ladder with L~_vv transposed
+        if (g.node(t2).active) ladder(getLT(), g.adjoint(om2, nvec), g.adjoint(t2, nvec), nvec);
     };
-    g.custom(std::move(op), om2, {Lvv, t2, t1, tf});
+    g.custom(std::move(op), om2, {Lvv, t2});
 }
 
 void Context::omega_eager(double *om_out) {

@@ -1,6 +1,7 @@
 // Recorded tensor computation with forward- and reverse-mode derivative passes.
 #include <algorithm>
 
+#include "amp_forms.cuh"
 #include "graph.cuh"
 #include "tensor_ops.cuh"
 
@@ -16,81 +17,6 @@ constexpr char BATCH = '#';   // label of the trailing trial index of tangents /
 inline int grid_for(int64_t total, int block) {
     int64_t g = (total + block - 1) / block;
     return (int)std::max<int64_t>(1, std::min<int64_t>(g, 148 * 64));
-}
-
-__device__ __forceinline__ void untri(int64_t idx, int64_t &M, int64_t &m) {
-    int64_t r = (int64_t)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
-    while (r * (r + 1) / 2 > idx) r--;
-    while ((r + 1) * (r + 2) / 2 <= idx) r++;
-    M = r;
-    m = idx - r * (r + 1) / 2;
-}
-
-// packed += S^T full over nbatch columns: p[(M,m)] += F[M,m] + F[m,M] (M > m), F[M,M] (M == m)
-__global__ void squareup_adj_kernel(const double *__restrict__ full, double *__restrict__ packed, int64_t nov,
-                                    int64_t nbatch) {
-    const int64_t np = nov * (nov + 1) / 2;
-    GRID_STRIDE(idx, np * nbatch) {
-        int64_t n = idx / np, p = idx - n * np, M, m;
-        untri(p, M, m);
-        const double *F = full + n * nov * nov;
-        double v = F[M + nov * m];
-        if (M != m) v += F[m + nov * M];
-        packed[idx] += v;
-    }
-}
-
-// full(m, M) += p[(M, m)] * (1/2 if M == m)  (adjoint of the packing read of pack_half_diag_add)
-__global__ void pack_half_adj_kernel(const double *__restrict__ packed, double *__restrict__ full, int64_t nov,
-                                     int64_t nbatch) {
-    const int64_t np = nov * (nov + 1) / 2;
-    GRID_STRIDE(idx, np * nbatch) {
-        int64_t n = idx / np, p = idx - n * np, M, m;
-        untri(p, M, m);
-        double v = packed[idx];
-        if (M == m) v *= 0.5;
-        full[n * nov * nov + m + nov * M] += v;
-    }
-}
-
-__global__ void pack_half_batch_kernel(const double *__restrict__ full, double *__restrict__ packed, int64_t nov,
-                                       int64_t nbatch) {
-    const int64_t np = nov * (nov + 1) / 2;
-    GRID_STRIDE(idx, np * nbatch) {
-        int64_t n = idx / np, p = idx - n * np, M, m;
-        untri(p, M, m);
-        double v = full[n * nov * nov + m + nov * M];
-        if (M == m) v *= 0.5;
-        packed[idx] += v;
-    }
-}
-
-// packed[(M, m)] += (F[m, M] + F[M, m]) * (1/2 if M == m): consecutive threads take consecutive m
-// of one M, so the F[m, M] reads are coalesced and the F[M, m] reads of neighbouring M share sectors
-// in L2
-__global__ void pack_sym_batch_kernel(const double *__restrict__ full, double *__restrict__ packed, int64_t nov,
-                                      int64_t nbatch) {
-    const int64_t np = nov * (nov + 1) / 2;
-    GRID_STRIDE(idx, np * nbatch) {
-        int64_t n = idx / np, p = idx - n * np, M, m;
-        untri(p, M, m);
-        const double *F = full + n * nov * nov;
-        const double v = F[m + nov * M] + F[M + nov * m];
-        packed[idx] += M == m ? 0.5 * v : v;
-    }
-}
-
-// full (+)= the symmetric square of packed (accumulate = 0: overwrite)
-__global__ void squareup_batch_kernel(const double *__restrict__ packed, double *__restrict__ full, int64_t nov,
-                                      int64_t nbatch, int accumulate) {
-    const int64_t nf = nov * nov, np = nov * (nov + 1) / 2;
-    GRID_STRIDE(idx, nf * nbatch) {
-        int64_t n = idx / nf, r = idx - n * nf;
-        int64_t x = r % nov, y = r / nov;
-        int64_t M = x > y ? x : y, m = x > y ? y : x;
-        const double v = packed[n * np + M * (M + 1) / 2 + m];
-        full[idx] = accumulate ? full[idx] + v : v;
-    }
 }
 
 // out[J, n] += sum_k a[J, k, k, n]  /  adjoint: a[J, k, k, n] += out[J, n]
@@ -213,10 +139,14 @@ void Graph::run_forward(const GOp &op) {
     if (op.b >= 0) materialize(op.b);
     if (op.kind == OpKind::Custom)
         for (int i : custom_ins_[op.custom]) materialize(i);
-    const bool fresh = nodes_[op.out].zero &&
-                       (op.kind == OpKind::Contract || op.kind == OpKind::Permute || op.kind == OpKind::Squareup);
-    if (fresh) nodes_[op.out].zero = false;
-    else materialize(op.out);
+    const auto first_write = [&](int i) {
+        const bool zero = nodes_[i].zero;
+        nodes_[i].zero = false;
+        return zero;
+    };
+    const bool overwrites = op.kind != OpKind::Trace && op.kind != OpKind::Custom;
+    if (!overwrites) materialize(op.out);
+    const bool fresh = first_write(op.out);
     const double beta = fresh ? 0.0 : 1.0;
     switch (op.kind) {
     case OpKind::Contract:
@@ -238,20 +168,14 @@ void Graph::run_forward(const GOp &op) {
         permute_add(ex_, op.alpha, pin, beta, out);
         break;
     }
-    case OpKind::Squareup:
-        squareup_batch_kernel<<<grid_for(nov * nov, 256), 256, 0, ex_.stream>>>(nodes_[op.a].v, nodes_[op.out].v, nov,
-                                                                                1, fresh ? 0 : 1);
-        ex_.launches++;
+    case OpKind::SquareForms: {
+        const bool fresh_u = first_write(op.out2);
+        ccsd::square_forms(ex_, nodes_[op.a].v, no, nv, 1, op.c1, op.c2, nodes_[op.out].v, nodes_[op.out2].v, !fresh,
+                           !fresh_u);
         break;
-    case OpKind::PackHalf:
-        pack_half_batch_kernel<<<grid_for(nov * (nov + 1) / 2, 256), 256, 0, ex_.stream>>>(
-            nodes_[op.a].v, nodes_[op.out].v, nov, 1);
-        ex_.launches++;
-        break;
-    case OpKind::PackSym:
-        pack_sym_batch_kernel<<<grid_for(nov * (nov + 1) / 2, 256), 256, 0, ex_.stream>>>(
-            nodes_[op.a].v, nodes_[op.out].v, nov, 1);
-        ex_.launches++;
+    }
+    case OpKind::SymPack:
+        ccsd::sym_pack(ex_, nodes_[op.a].v, nodes_[op.b].v, no, nv, 1, op.c1, op.c2, nodes_[op.out].v, !fresh);
         break;
     case OpKind::Trace: {
         const GNode &a = nodes_[op.a];
@@ -293,33 +217,29 @@ void Graph::permute(int out, const char *spec, double alpha, int a) {
     ops_.push_back(op);
 }
 
-void Graph::squareup(int out, int a) {
+void Graph::square_forms(int t, int u, int a, double c1, double c2) {
     GOp op;
-    op.kind = OpKind::Squareup;
-    op.out = out;
+    op.kind = OpKind::SquareForms;
+    op.out = t;
+    op.out2 = u;
     op.a = a;
+    op.c1 = c1;
+    op.c2 = c2;
     run_forward(op);
     nodes_[a].last_use = (int)ops_.size();
     ops_.push_back(op);
 }
 
-void Graph::pack_sym(int out, int a) {
+void Graph::sym_pack(int out, int a, int x, double c1, double c2) {
     GOp op;
-    op.kind = OpKind::PackSym;
+    op.kind = OpKind::SymPack;
     op.out = out;
     op.a = a;
+    op.b = x;
+    op.c1 = c1;
+    op.c2 = c2;
     run_forward(op);
-    nodes_[a].last_use = (int)ops_.size();
-    ops_.push_back(op);
-}
-
-void Graph::pack_half(int out, int a) {
-    GOp op;
-    op.kind = OpKind::PackHalf;
-    op.out = out;
-    op.a = a;
-    run_forward(op);
-    nodes_[a].last_use = (int)ops_.size();
+    nodes_[a].last_use = nodes_[x].last_use = (int)ops_.size();
     ops_.push_back(op);
 }
 
@@ -357,6 +277,7 @@ void Graph::mark_active(const std::vector<int> &inputs) {
             act = nodes_[op.a].active || (op.b >= 0 && nodes_[op.b].active);
         }
         if (act) nodes_[op.out].active = true;
+        if (act && op.out2 >= 0) nodes_[op.out2].active = true;
     }
 }
 
@@ -410,24 +331,16 @@ void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *
             permute_add(ex_, op.alpha, pin, 1.0, out);
             break;
         }
-        case OpKind::Squareup:
-            if (!nodes_[op.a].active) break;
-            squareup_batch_kernel<<<grid_for(nov * nov * nvec, 256), 256, 0, ex_.stream>>>(
-                tangent(op.a, nvec), tangent(op.out, nvec), nov, nvec, 1);
-            ex_.launches++;
+        case OpKind::SquareForms:
+            ccsd::square_forms(ex_, tangent(op.a, nvec), no, nv, nvec, op.c1, op.c2, tangent(op.out, nvec),
+                               tangent(op.out2, nvec), true, true);
             break;
-        case OpKind::PackHalf:
-            if (!nodes_[op.a].active) break;
-            pack_half_batch_kernel<<<grid_for(nov * (nov + 1) / 2 * nvec, 256), 256, 0, ex_.stream>>>(
-                tangent(op.a, nvec), tangent(op.out, nvec), nov, nvec);
-            ex_.launches++;
+        case OpKind::SymPack: {
+            const double *fa = nodes_[op.a].active ? tangent(op.a, nvec) : nullptr;
+            const double *xa = nodes_[op.b].active ? tangent(op.b, nvec) : nullptr;
+            ccsd::sym_pack(ex_, fa, xa, no, nv, nvec, op.c1, op.c2, tangent(op.out, nvec), true);
             break;
-        case OpKind::PackSym:
-            if (!nodes_[op.a].active) break;
-            pack_sym_batch_kernel<<<grid_for(nov * (nov + 1) / 2 * nvec, 256), 256, 0, ex_.stream>>>(
-                tangent(op.a, nvec), tangent(op.out, nvec), nov, nvec);
-            ex_.launches++;
-            break;
+        }
         case OpKind::Trace: {
             if (!nodes_[op.a].active) break;
             const GNode &a = nodes_[op.a];
@@ -462,7 +375,8 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
     }
     for (int oi = (int)ops_.size() - 1; oi >= 0; --oi) {
         const GOp &op = ops_[oi];
-        if (!nodes_[op.out].active || !nodes_[op.out].adj) continue;
+        if (!nodes_[op.out].active) continue;
+        if (!nodes_[op.out].adj && !(op.out2 >= 0 && nodes_[op.out2].adj)) continue;
         Fp64Scope fp64(ex_, op.fp64);
         switch (op.kind) {
         case OpKind::Contract: {
@@ -496,25 +410,20 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
             permute_add(ex_, op.alpha, pin, 1.0, abar);
             break;
         }
-        case OpKind::Squareup:
-            if (!nodes_[op.a].active) break;
-            squareup_adj_kernel<<<grid_for(nov * (nov + 1) / 2 * nvec, 256), 256, 0, ex_.stream>>>(
-                adjoint(op.out, nvec), adjoint(op.a, nvec), nov, nvec);
-            ex_.launches++;
+        case OpKind::SquareForms: {
+            // p enters S_aibj and S_bjai (its diagonal once) and both through the exchanged form: the
+            // transpose is the symmetrised packing of the two adjoints
+            const double *sa = has_adjoint(op.out) ? adjoint(op.out, nvec) : nullptr;
+            const double *ua = has_adjoint(op.out2) ? adjoint(op.out2, nvec) : nullptr;
+            ccsd::sym_pack(ex_, sa, ua, no, nv, nvec, op.c1, op.c2, adjoint(op.a, nvec), true);
             break;
-        case OpKind::PackHalf:
-            if (!nodes_[op.a].active) break;
-            pack_half_adj_kernel<<<grid_for(nov * (nov + 1) / 2 * nvec, 256), 256, 0, ex_.stream>>>(
-                adjoint(op.out, nvec), adjoint(op.a, nvec), nov, nvec);
-            ex_.launches++;
-            break;
-        case OpKind::PackSym:
-            // d packed[(M, m)] / d F[x, y] = 1 for {x, y} = {M, m} (the diagonal's 1/2 meets two
+        }
+        case OpKind::SymPack:
+            // d packed[(M, m)] / d z[x, y] = 1 for {x, y} = {M, m} (the diagonal's 1/2 meets two
             // equal entries): the adjoint is the full symmetric square-up of the packed adjoint
-            if (!nodes_[op.a].active) break;
-            squareup_batch_kernel<<<grid_for(nov * nov * nvec, 256), 256, 0, ex_.stream>>>(
-                adjoint(op.out, nvec), adjoint(op.a, nvec), nov, nvec, 1);
-            ex_.launches++;
+            ccsd::square_forms(ex_, adjoint(op.out, nvec), no, nv, nvec, op.c1, op.c2,
+                               nodes_[op.a].active ? adjoint(op.a, nvec) : nullptr,
+                               nodes_[op.b].active ? adjoint(op.b, nvec) : nullptr, true, true);
             break;
         case OpKind::Trace: {
             if (!nodes_[op.a].active) break;
@@ -538,12 +447,6 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
         else
             fill(ex_, results[k], n.size * nvec, 0.0);
     }
-}
-
-void pack_sym_add(Exec &ex, const double *full, double *packed, int64_t nov) {
-    pack_sym_batch_kernel<<<grid_for(nov * (nov + 1) / 2, 256), 256, 0, ex.stream>>>(full, packed, nov, 1);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
 }
 
 }  // namespace ccsd

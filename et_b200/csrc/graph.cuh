@@ -26,7 +26,7 @@ struct GNode {
     int last_use = -1;           // index of the last op reading this node
 };
 
-enum class OpKind { Contract, Permute, Squareup, PackHalf, PackSym, Trace, Custom };
+enum class OpKind { Contract, Permute, SquareForms, SymPack, Trace, Custom };
 
 // A custom op supplies its own forward / tangent / adjoint callbacks.
 struct CustomOp {
@@ -38,15 +38,13 @@ struct CustomOp {
 struct GOp {
     OpKind kind;
     int out = -1, a = -1, b = -1;
+    int out2 = -1;               // SquareForms: the exchanged form
     double alpha = 1.0;
+    double c1 = 0.0, c2 = 0.0;   // SquareForms, SymPack: weights of a form and of its exchange
     std::string spec;            // contract: "la,lb->lc"; permute: "lin->lout"
     bool fp64 = false;           // force FP64 (first-order terms)
     int custom = -1;
 };
-
-// packed[(M, m)] += (full[M, m] + full[m, M]) * (1/2 if M == m) over M >= m: the symmetrised full
-// doubles array packed as eT's symmetric_sum + scale_diagonal(1/2) + packin do, in one pass
-void pack_sym_add(Exec &ex, const double *full, double *packed, int64_t nov);
 
 class Graph {
   public:
@@ -63,13 +61,10 @@ class Graph {
     void contract(int out, const char *spec, double alpha, int a, int b, bool fp64 = false);
     // out += alpha * permute(a), spec "ajbi->aibj" (labels name the dims of a / out)
     void permute(int out, const char *spec, double alpha, int a);
-    // out(full (v,o,v,o) symmetric) += squareup(a packed)
-    void squareup(int out, int a);
-    // out(packed) += pack with the diagonal halved of a (full; read triangle (m, M))
-    void pack_half(int out, int a);
-    // out(packed) += pack with the diagonal halved of a + a^T (a full, not symmetric): eT's
-    // symmetric_sum, scale_diagonal(1/2) and packin in one pass
-    void pack_sym(int out, int a);
+    // t (full (v,o,v,o)) += squareup(a packed), u += c1 t_aibj + c2 t_ajbi
+    void square_forms(int t, int u, int a, double c1, double c2);
+    // out(packed) += pack with the diagonal halved of z + z^T, z = a + c1 x_aibj + c2 x_ajbi (a, x full)
+    void sym_pack(int out, int a, int x, double c1, double c2);
     // out[J] += sum_k a[J, k, k]
     void trace(int out, int a);
     // custom op over existing nodes
@@ -83,7 +78,7 @@ class Graph {
         materialize(i);
         return nodes_[i].v;
     }
-    int64_t nov = 0;               // for squareup / pack_half
+    int64_t no = 0, nv = 0;        // for square_forms / sym_pack
 
     // derivative passes; seeds are [size x nvec] device arrays for the listed nodes.  Each pass
     // starts from zero tangents / adjoints, so a recording can serve several passes.

@@ -551,52 +551,6 @@ void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B
 }
 
 // ---------------------------------------------------------------------------
-// packing
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ int64_t pk(int64_t x, int64_t y) {
-    int64_t M = x > y ? x : y, m = x > y ? y : x;
-    return M * (M + 1) / 2 + m;
-}
-
-__global__ void squareup_kernel(const double *__restrict__ packed, double *__restrict__ full, int64_t nov) {
-    int64_t total = nov * nov;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int64_t r = idx % nov, c = idx / nov;
-        full[idx] = packed[pk(r, c)];
-    }
-}
-
-void squareup(Exec &ex, const double *packed, double *full, int64_t nov) {
-    squareup_kernel<<<grid_for(nov * nov, 256), 256, 0, ex.stream>>>(packed, full, nov);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
-}
-
-// one thread per packed element; element (M, m) with M >= m reads full(m, M) = full[m + nov*M]
-__global__ void pack_half_diag_add_kernel(double alpha, const double *__restrict__ full, double *__restrict__ packed,
-                                          int64_t nov) {
-    int64_t total = nov * (nov + 1) / 2;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int64_t M = (int64_t)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
-        while (M * (M + 1) / 2 > idx) M--;
-        while ((M + 1) * (M + 2) / 2 <= idx) M++;
-        int64_t m = idx - M * (M + 1) / 2;
-        double v = full[m + nov * M];
-        if (m == M) v *= 0.5;
-        packed[idx] += alpha * v;
-    }
-}
-
-void pack_half_diag_add(Exec &ex, double alpha, const double *full, double *packed, int64_t nov) {
-    pack_half_diag_add_kernel<<<grid_for(nov * (nov + 1) / 2, 256), 256, 0, ex.stream>>>(alpha, full, packed, nov);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
-}
-
-// ---------------------------------------------------------------------------
 // reductions
 // ---------------------------------------------------------------------------
 

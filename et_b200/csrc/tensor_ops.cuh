@@ -27,12 +27,6 @@ void gemm_batched_f64(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, 
                       const double *A, int64_t lda, int64_t strideA, const double *B, int64_t ldb, int64_t strideB,
                       double beta, double *C, int64_t ldc, int64_t strideC, int64_t batch);
 
-// packed doubles <-> full symmetric (v,o,v,o)
-void squareup(Exec &ex, const double *packed, double *full, int64_t nov);
-// packed += alpha * full(M,m) * (1/2 if M == m) over M >= m (eT's scale_diagonal(1/2) + packin);
-// reads the symmetric counterpart full(m, M) for coalescing, so `full` must be symmetric.
-void pack_half_diag_add(Exec &ex, double alpha, const double *full, double *packed, int64_t nov);
-
 // reductions (deterministic two-pass)
 void dot(Exec &ex, const double *x, const double *y, int64_t n, double *d_result);
 void multi_dot(Exec &ex, const double *x, const double *const *ys, int nys, int64_t n, double *d_results);
