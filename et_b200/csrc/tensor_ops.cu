@@ -255,53 +255,67 @@ Route lookup_route(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int
 
 }  // namespace
 
-void gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha, const double *A,
-          int64_t lda, const double *B, int64_t ldb, double beta, double *C, int64_t ldc, bool allow_mixed) {
-    if (m == 0 || n == 0) return;
-    double fl = 2.0 * double(m) * double(n) * double(k);
-    ex.flops += fl;
-    Route rt = lookup_route(ex, transA, transB, m, n, k, fl, allow_mixed);
-    if (!rt.known) {
-        std::vector<int> routes;
-        if (fl <= 4e11) routes.push_back(0);   // larger products never favour FP64
-        for (int sp : tc_split_candidates(m, n, k, ex.planes)) routes.push_back(sp);
-        DBuf scratch = dalloc(m * n, ex.stream);
-        const int route = tune_measure(ex, rt.key, routes, [&](int r) {
-            if (r == 0) {
-                const double zero = 0.0;
-                BLAS_CHECK(cublasDgemm_64(ex.blas, transA ? CUBLAS_OP_T : CUBLAS_OP_N,
-                                          transB ? CUBLAS_OP_T : CUBLAS_OP_N, m, n, k, &alpha, A, lda, B, ldb,
-                                          &zero, scratch.d(), m));
-            } else {
-                mixed_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, 0.0, scratch.d(), m, r);
-            }
-        });
-        if (route < 0) {
-            // not timed now (another thread is timing, or the stream is being captured): the fixed rule
-            rt = fixed_route(ex, m, n, k, fl, allow_mixed);
+namespace {
+
+// The route of a product that lookup_route does not know yet: every candidate timed on these operands
+// (the fixed rule when that cannot be done now: another thread is timing, or the stream is captured).
+Route measure_route(Exec &ex, const Route &unknown, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha,
+                    const double *A, int64_t lda, const double *B, int64_t ldb, double fl, bool allow_mixed) {
+    std::vector<int> routes;
+    if (fl <= 4e11) routes.push_back(0);   // larger products never favour FP64
+    for (int sp : tc_split_candidates(m, n, k, ex.planes)) routes.push_back(sp);
+    DBuf scratch = dalloc(m * n, ex.stream);
+    const int route = tune_measure(ex, unknown.key, routes, [&](int r) {
+        if (r == 0) {
+            const double zero = 0.0;
+            BLAS_CHECK(cublasDgemm_64(ex.blas, transA ? CUBLAS_OP_T : CUBLAS_OP_N, transB ? CUBLAS_OP_T : CUBLAS_OP_N, m,
+                                      n, k, &alpha, A, lda, B, ldb, &zero, scratch.d(), m));
         } else {
-            rt.known = true;
-            rt.mixed = route > 0;
-            rt.splits = route;
+            mixed_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, 0.0, scratch.d(), m, r);
         }
-    }
-    const bool mixed = rt.mixed;
-    const int route = rt.splits;
+    });
+    if (route < 0) return fixed_route(ex, m, n, k, fl, allow_mixed);
+    Route rt;
+    rt.mixed = route > 0;
+    rt.splits = route;
+    return rt;
+}
+
+// whether an FP64 product goes to the int8 digit GEMM
+bool takes_digits(const Exec &ex, int64_t m, int64_t n, int64_t k, double fl) {
+    return ex.fp64_digits > 0 && fl >= ex.fp64_digits_min_flops &&
+           (ex.fp64_digits_min_flops <= 1 || (m >= 256 && n >= 256 && k >= 512));
+}
+
+void run_gemm(Exec &ex, const Route &rt, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha,
+              const double *A, int64_t lda, const double *B, int64_t ldb, double beta, double *C, int64_t ldc) {
+    const double fl = 2.0 * double(m) * double(n) * double(k);
     if (trace_level() >= 2)
         std::fprintf(stderr, "ccsd_gpu gemm [%s] %s m %lld n %lld k %lld  %.3g flop  splits %d\n",
-                     g_perm_tag ? g_perm_tag : "direct", mixed ? "bf16x3" : "fp64", (long long)m, (long long)n,
-                     (long long)k, fl, route);
-    if (mixed) {
-        mixed_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, route);
+                     g_perm_tag ? g_perm_tag : "direct", rt.mixed ? "bf16x3" : "fp64", (long long)m, (long long)n,
+                     (long long)k, fl, rt.splits);
+    if (rt.mixed) {
+        mixed_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, rt.splits);
         return;
     }
-    if (ex.fp64_digits > 0 && fl >= ex.fp64_digits_min_flops &&
-        (ex.fp64_digits_min_flops <= 1 || (m >= 256 && n >= 256 && k >= 512))) {
+    if (takes_digits(ex, m, n, k, fl)) {
         ozaki_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ex.fp64_digits);
         return;
     }
     BLAS_CHECK(cublasDgemm_64(ex.blas, transA ? CUBLAS_OP_T : CUBLAS_OP_N, transB ? CUBLAS_OP_T : CUBLAS_OP_N, m,
                               n, k, &alpha, A, lda, B, ldb, &beta, C, ldc));
+}
+
+}  // namespace
+
+void gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha, const double *A,
+          int64_t lda, const double *B, int64_t ldb, double beta, double *C, int64_t ldc, bool allow_mixed) {
+    if (m == 0 || n == 0) return;
+    const double fl = 2.0 * double(m) * double(n) * double(k);
+    ex.flops += fl;
+    Route rt = lookup_route(ex, transA, transB, m, n, k, fl, allow_mixed);
+    if (!rt.known) rt = measure_route(ex, rt, transA, transB, m, n, k, alpha, A, lda, B, ldb, fl, allow_mixed);
+    run_gemm(ex, rt, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
 }
 
 void gemm_batched_f64(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha,
@@ -420,6 +434,139 @@ bool gather_view(const TV &v, const std::vector<int> &rows, const std::vector<in
     return true;
 }
 
+// bytes that the reordering copies of a product move (each read and written once; an output that is
+// scattered also reads its old values)
+double copy_bytes(const TV &A, bool packA, const TV &B, bool packB, const TV &C, bool scatter) {
+    return 16.0 * ((packA ? (double)A.size() : 0.0) + (packB ? (double)B.size() : 0.0)) +
+           (scatter ? 24.0 * (double)C.size() : 0.0);
+}
+
+// A contraction as a strided batch of GEMMs: one or two output labels of one operand are taken out (z the
+// batch, w a loop on the host; -1: none), what is left of A, B and C are matrices as they lie.
+struct BatchPlan {
+    bool swap = false;            // C' is N x M: the operands change places
+    bool tA = false, tB = false;
+    int64_t m = 0, n = 0, k = 0, lda = 0, ldb = 0, ldc = 0;
+    int64_t nz = 1, zA = 0, zB = 0, zC = 0;   // batch count and strides
+    int64_t nw = 1, wA = 0, wB = 0, wC = 0;   // loop count and strides
+    bool copyA = false, copyB = false;        // an operand still needs its copy (the one without z, w)
+    std::vector<int> a1, a2, b1, b2;          // its dims as (first group, second group)
+};
+
+// The plan that spares the most copying of those whose launches cost less than that: a copy of 16 MB takes
+// about as long as two launches.  False when none beats `base` bytes.
+bool find_batch(const TV &A, const TV &B, const TV &C, const std::map<char, LabelInfo> &info, const std::vector<char> &K,
+                const std::vector<char> &oM, const std::vector<char> &oN, double base, BatchPlan *best) {
+    bool found = false;
+    double best_gain = 0.0;
+    // a product bound by its flops gains little from the copies it is spared and loses more when the batch
+    // falls on a narrower DGEMM tile (2048^3 with a batch of 16: 1.02 ms, 0.55 ms with both copies)
+    const double fl = 2.0 * (double)prod(oM, info) * (double)prod(oN, info) * (double)prod(K, info);
+    if (fl / 35e12 > 3.0 * base / 4e12) return false;
+    auto without = [](const std::vector<char> &v, char z, char w) {
+        std::vector<char> o;
+        for (char c : v)
+            if (c != z && c != w) o.push_back(c);
+        return o;
+    };
+    std::vector<char> outs = oM;
+    outs.insert(outs.end(), oN.begin(), oN.end());
+    auto try_plan = [&](char z, char w) {
+        BatchPlan p;
+        const auto M = without(oM, z, w), N = without(oN, z, w);
+        const LabelInfo &iz = info.at(z);
+        p.nz = iz.n;
+        p.zA = iz.dA >= 0 ? A.s[iz.dA] : 0;
+        p.zB = iz.dB >= 0 ? B.s[iz.dB] : 0;
+        p.zC = C.s[iz.dC];
+        if (w) {
+            const LabelInfo &iw = info.at(w);
+            p.nw = iw.n;
+            p.wA = iw.dA >= 0 ? A.s[iw.dA] : 0;
+            p.wB = iw.dB >= 0 ? B.s[iw.dB] : 0;
+            p.wC = C.s[iw.dC];
+            if (p.wA == p.zA * p.nz && p.wB == p.zB * p.nz && p.wC == p.zC * p.nz) {   // one longer batch
+                p.nz *= p.nw;
+                p.nw = 1;
+                p.wA = p.wB = p.wC = 0;
+            }
+        }
+        const auto cM = dims_of(M, info, 2), cN = dims_of(N, info, 2);
+        if (groupable(C, cM, cN, &p.ldc)) p.swap = false;
+        else if (groupable(C, cN, cM, &p.ldc)) p.swap = true;
+        else return;
+        p.m = prod(M, info);
+        p.n = prod(N, info);
+        p.k = prod(K, info);
+        // the output tiles of what is left must stay full (cuBLAS runs a batch of thin products, or one of
+        // gemv shape, several times slower than one product over copies)
+        if ((p.m < 64 && p.m < prod(oM, info)) || (p.n < 64 && p.n < prod(oN, info)) || p.m == 1 || p.n == 1) return;
+        // a strided batch runs without K splits: a long K needs enough 64 x 64 output tiles for the SMs
+        if (p.k > 4096 && ((p.m + 63) / 64) * ((p.n + 63) / 64) * p.nz < 148) return;
+        const bool freeA = p.zA == 0 && p.wA == 0, freeB = p.zB == 0 && p.wB == 0;
+        for (int which = 0; which < 2; which++) {   // the K order of A, then of B
+            BatchPlan q = p;
+            const auto oK = natural_order(which == 0 ? A : B, K, info, which);
+            const auto aK = dims_of(oK, info, 0), aM = dims_of(M, info, 0), bK = dims_of(oK, info, 1), bN = dims_of(N, info, 1);
+            if (groupable(A, aM, aK, &q.lda)) q.tA = false;
+            else if (groupable(A, aK, aM, &q.lda)) q.tA = true;
+            else if (freeA) {
+                q.copyA = q.tA = true;
+                q.lda = q.k;
+                q.a1 = aK;
+                q.a2 = aM;
+            } else continue;
+            if (groupable(B, bK, bN, &q.ldb)) q.tB = false;
+            else if (groupable(B, bN, bK, &q.ldb)) q.tB = true;
+            else if (freeB) {
+                q.copyB = true;
+                q.tB = false;
+                q.ldb = q.k;
+                q.b1 = bK;
+                q.b2 = bN;
+            } else continue;
+            const double gain = base - copy_bytes(A, q.copyA, B, q.copyB, C, false);
+            // of equal plans the one with the larger products
+            if (gain < best_gain || (gain == best_gain && found && q.m * q.n <= best->m * best->n)) continue;
+            if (gain <= 0.0 || (double)(q.nw - 1) * 16e6 > gain) continue;
+            best_gain = gain;
+            *best = q;
+            found = true;
+        }
+    };
+    for (char z : outs) {
+        const LabelInfo &iz = info.at(z);
+        if (iz.n < 2) continue;
+        try_plan(z, 0);
+        for (char w : outs) {
+            const LabelInfo &iw = info.at(w);
+            if (w == z || iw.n < 2 || (iw.dA >= 0) != (iz.dA >= 0)) continue;
+            try_plan(z, w);
+        }
+    }
+    return found;
+}
+
+void run_batch(Exec &ex, const BatchPlan &p, const TV &A, const TV &B, const TV &C, double alpha, double beta) {
+    DBuf bufA, bufB;
+    const TV Au = p.copyA ? make_contiguous(ex, A, p.a1, p.a2, bufA) : A;
+    const TV Bu = p.copyB ? make_contiguous(ex, B, p.b1, p.b2, bufB) : B;
+    if (trace_level() >= 2)
+        std::fprintf(stderr, "ccsd_gpu gemm [%s] fp64 batch %lld x %lld m %lld n %lld k %lld\n",
+                     g_perm_tag ? g_perm_tag : "direct", (long long)p.nw, (long long)p.nz, (long long)p.m, (long long)p.n,
+                     (long long)p.k);
+    for (int64_t w = 0; w < p.nw; w++) {
+        const double *a = Au.p + w * p.wA, *b = Bu.p + w * p.wB;
+        double *c = C.p + w * p.wC;
+        if (p.swap)
+            gemm_batched_f64(ex, !p.tB, !p.tA, p.n, p.m, p.k, alpha, b, p.ldb, p.zB, a, p.lda, p.zA, beta, c, p.ldc, p.zC,
+                             p.nz);
+        else
+            gemm_batched_f64(ex, p.tA, p.tB, p.m, p.n, p.k, alpha, a, p.lda, p.zA, b, p.ldb, p.zB, beta, c, p.ldc, p.zC,
+                             p.nz);
+    }
+}
+
 }  // namespace
 
 void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B, double beta, const TV &C) {
@@ -512,33 +659,47 @@ void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B
         }
         permute_add(ex, 1.0, t, beta, C);
     };
-    if (packA || packB) {
-        SplitView va, vb;
-        if (gather_view(A, aM, aK, &va) && gather_view(B, bN, bK, &vb)) {
-            // the route of the product as the reordered copies would present it
-            const double fl = 2.0 * double(mM) * double(mN) * double(mK);
-            const Route rt = cmode == 1 ? lookup_route(ex, !tB, !tA, mN, mM, mK, fl, true)
-                                        : lookup_route(ex, tA, tB, mM, mN, mK, fl, true);
-            if (rt.known && rt.mixed) {
-                ex.flops += fl;
-                if (trace_level() >= 2)
-                    std::fprintf(stderr, "ccsd_gpu gemm [%s] bf16x3 gather m %lld n %lld k %lld  %.3g flop  splits %d\n",
-                                 spec, (long long)mM, (long long)mN, (long long)mK, fl, rt.splits);
-                if (cmode == 0) {
-                    mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, beta, C.p, ldc, rt.splits);
-                } else if (cmode == 1) {
-                    mixed_gemm_views(ex, vb, va, mN, mM, mK, alpha, beta, C.p, ldc, rt.splits);
-                } else {
-                    bufC = dalloc(mM * mN, ex.stream);
-                    mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, 0.0, bufC.d(), mM, rt.splits);
-                    scatter_C();
-                }
-                return;
-            }
+    const double fl = 2.0 * double(mM) * double(mN) * double(mK);
+    Route rt = cmode == 1 ? lookup_route(ex, !tB, !tA, mN, mM, mK, fl, true)
+                          : lookup_route(ex, tA, tB, mM, mN, mK, fl, true);
+    SplitView va, vb;
+    if ((packA || packB) && rt.known && rt.mixed && gather_view(A, aM, aK, &va) && gather_view(B, bN, bK, &vb)) {
+        ex.flops += fl;
+        if (trace_level() >= 2)
+            std::fprintf(stderr, "ccsd_gpu gemm [%s] bf16x3 gather m %lld n %lld k %lld  %.3g flop  splits %d\n", spec,
+                         (long long)mM, (long long)mN, (long long)mK, fl, rt.splits);
+        if (cmode == 0) {
+            mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, beta, C.p, ldc, rt.splits);
+        } else if (cmode == 1) {
+            mixed_gemm_views(ex, vb, va, mN, mM, mK, alpha, beta, C.p, ldc, rt.splits);
+        } else {
+            bufC = dalloc(mM * mN, ex.stream);
+            mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, 0.0, bufC.d(), mM, rt.splits);
+            scatter_C();
         }
-        if (packA) Au = make_contiguous(ex, A, aK, aM, bufA);
-        if (packB) Bu = make_contiguous(ex, B, bK, bN, bufB);
+        return;
     }
+    // a product for cuBLAS whose operands or output are not matrices as they lie: as a strided batch of
+    // GEMMs over an output index (the trial index, or one that sits between the others) where that spares
+    // the copies
+    BatchPlan bp;
+    const bool batch = (packA || packB || cmode == 2) && !takes_digits(ex, mM, mN, mK, fl) &&
+                       find_batch(A, B, C, info, K, oM, oN, copy_bytes(A, packA, B, packB, C, cmode == 2), &bp);
+    auto copies = [&]() {
+        if (packA && Au.p == A.p) Au = make_contiguous(ex, A, aK, aM, bufA);
+        if (packB && Bu.p == B.p) Bu = make_contiguous(ex, B, bK, bN, bufB);
+    };
+    if (batch && !rt.known) {
+        // time the candidates on the copies the tensor-core routes would be compared with
+        copies();
+        rt = cmode == 1 ? measure_route(ex, rt, !tB, !tA, mN, mM, mK, alpha, Bu.p, ldb, Au.p, lda, fl, true)
+                        : measure_route(ex, rt, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, fl, true);
+    }
+    if (batch && !rt.mixed) {
+        run_batch(ex, bp, A, B, C, alpha, beta);
+        return;
+    }
+    copies();
     if (cmode == 0) {
         gemm(ex, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, beta, C.p, ldc);
     } else if (cmode == 1) {
