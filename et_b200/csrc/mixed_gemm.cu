@@ -57,7 +57,7 @@ struct Mode {
     static constexpr int A_TILE = BM * KB * 2;       // bytes per plane
     static constexpr int B_TILE = BN * KB * 2;
     static constexpr int STAGE_BYTES = NP * (A_TILE + B_TILE);
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 4 * BN * 8 /*column offsets*/;
     static constexpr uint32_t TMEM_COLS = 2 * BN;    // two FP32 accumulators of 128 lanes x BN columns
     // kind::f16 instruction descriptor: BF16 x BF16 -> F32, both K-major, M = 128, N = BN
     static constexpr uint32_t IDESC =
@@ -73,9 +73,10 @@ static_assert(B_ROW_PAD % ModeX3::BN == 0 && B_ROW_PAD % ModeX6::BN == 0, "B pad
 
 }  // namespace
 
-// FP64 column-major output with alpha/beta
+// FP64 output with alpha/beta: a column-major matrix.
 struct EpiF64 {
     static constexpr bool kChunked = true;   // can accumulate K chunks into the output
+    static constexpr bool kTable = false;
     double *C;
     long long ldc;
     int M, N;
@@ -87,7 +88,7 @@ struct EpiF64 {
     // 16 consecutive columns of one row.  first: the first K chunk of the tile (beta applies);
     // later chunks add to what is there, in FP64.  The 16 old values are loaded before any store so
     // their L2 latencies overlap.
-    __device__ __forceinline__ void apply16(int row, int col0, const float (&v)[16], bool first) const {
+    __device__ __forceinline__ void apply16(int row, int col0, const float (&v)[16], bool first, const long long *) const {
         if (row >= M) return;
         double *base = C + zoff + (long long)col0 * ldc + row;
         const bool need_old = !first || beta != 0.0;
@@ -101,6 +102,42 @@ struct EpiF64 {
                 if (!first) r += old[j];
                 else if (beta != 0.0) r += beta * old[j];
                 base[(long long)j * ldc] = r;
+            }
+        }
+    }
+};
+
+// The same into a tensor of interleaved index groups: each element at its row's plus its column's offset.
+// The column offsets of a tile stand in shared memory (one table per epilogue warp), so the scatter costs
+// one division chain per row and per column of the tile, not per element.  Matrices keep the form above:
+// its address arithmetic is cheaper, and through the table they lost 2-4 % of the residual.
+// Four transposes at o=16, v=128: 8.51 ms with a matrix scratch and a reordering pass, 8.41 so; six
+// transformations at o=24, v=240: 130.7 and 128.4 ms.
+struct EpiScatter {
+    static constexpr bool kChunked = true;
+    static constexpr bool kTable = true;
+    OutView C;
+    int M, N;
+    double alpha, beta;
+    long long off = 0;
+    __device__ __forceinline__ void tile_setup(int) {}
+    __device__ __forceinline__ void row_setup(int row) { off = OutView::offset(row, C.nr, C.rn, C.rs); }
+    __device__ __forceinline__ long long col_offset(int col) const { return OutView::offset(col, C.nc, C.cn, C.cs); }
+    __device__ __forceinline__ void apply16(int row, int col0, const float (&v)[16], bool first,
+                                            const long long *coff) const {
+        if (row >= M) return;
+        double *base = C.p + off;
+        const bool need_old = !first || beta != 0.0;
+        double old[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) old[j] = (need_old && col0 + j < N) ? __ldcg(base + coff[j]) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            if (col0 + j < N) {
+                double r = alpha * (double)v[j];
+                if (!first) r += old[j];
+                else if (beta != 0.0) r += beta * old[j];
+                base[coff[j]] = r;
             }
         }
     }
@@ -123,6 +160,7 @@ __device__ __forceinline__ void store_split_planes(__nv_bfloat16 *out, size_t pl
 // take consecutive c and store to consecutive addresses).
 struct EpiOvvv {
     static constexpr bool kChunked = false;
+    static constexpr bool kTable = false;
     __nv_bfloat16 *out;
     size_t plane;
     long long ldk;
@@ -133,7 +171,7 @@ struct EpiOvvv {
         k = row / nv;
         c = row - k * nv;
     }
-    __device__ __forceinline__ void apply16(int row, int col0, const float (&v)[16], bool) const {
+    __device__ __forceinline__ void apply16(int row, int col0, const float (&v)[16], bool, const long long *) const {
         if (row >= M) return;
 #pragma unroll
         for (int j = 0; j < 16; j++) {
@@ -305,11 +343,17 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     } else {
         // epilogue: warp w reads TMEM lanes 32*(w % 4) .. +31
         const int quarter = warp & 3;
+        long long *coff = reinterpret_cast<long long *>(smem + STAGES * STAGE_BYTES + 256) + quarter * BN;
         int tc = 0;
         bool aborted = false;
         for (int t = blockIdx.x; t < num_tiles && !aborted; t += gridDim.x) {
             int m0, n0, z, kt0, nk;
             map.decode(t, m0, n0, z, kt0, nk);
+            if constexpr (Epi::kTable) {
+                __syncwarp();
+                for (int c = lane; c < BN; c += 32) coff[c] = n0 + c < epi.N ? epi.col_offset(n0 + c) : 0;
+                __syncwarp();
+            }
             for (int c0 = 0; c0 < nk; c0 += map.kc, tc++) {
             const int acc = tc & 1;
             bool ok = !*abort_flag && mbar_wait(&acc_full[acc], (tc >> 1) & 1, map.wait_cycles);
@@ -329,7 +373,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             for (int cc = 0; cc < BN; cc += 16) {
                 float v[16];
                 tmem_ld16(base + (uint32_t)cc, v);
-                epi.apply16(row, n0 + cc, v, c0 == 0);
+                epi.apply16(row, n0 + cc, v, c0 == 0, coff + cc);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[acc])) : "memory");
@@ -359,7 +403,7 @@ struct PairMode {
     static constexpr int A_TILE = BM * KB * 2;          // 128 rows of one plane
     static constexpr int B_TILE = (BN / 2) * KB * 2;    // this CTA's half of the B tile
     static constexpr int STAGE_BYTES = NP * (A_TILE + B_TILE);
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 4 * BN * 8;
     static constexpr uint32_t TMEM_COLS = 2 * BN;
     static constexpr uint32_t IDESC =
         (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -506,11 +550,17 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     } else {
         // epilogue: this CTA's 128 rows; warp w reads TMEM lanes 32*(w % 4) .. +31
         const int quarter = warp & 3;
+        long long *coff = reinterpret_cast<long long *>(smem + STAGES * STAGE_BYTES + 256) + quarter * BN;
         int tc = 0;
         bool aborted = false;
         for (int t = pair; t < num_tiles && !aborted; t += npairs) {
             int m0, n0, z, kt0, nk;
             map.decode(t, m0, n0, z, kt0, nk);
+            if constexpr (Epi::kTable) {
+                __syncwarp();
+                for (int c = lane; c < BN; c += 32) coff[c] = n0 + c < epi.N ? epi.col_offset(n0 + c) : 0;
+                __syncwarp();
+            }
             for (int c0 = 0; c0 < nk; c0 += map.kc, tc++) {
                 const int acc = tc & 1;
                 bool ok = !*abort_flag && mbar_wait(&acc_full[acc], (tc >> 1) & 1, map.wait_cycles);
@@ -530,7 +580,7 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                 for (int cc = 0; cc < BN; cc += 16) {
                     float v[16];
                     tmem_ld16(base + (uint32_t)cc, v);
-                    epi.apply16(row, n0 + cc, v, c0 == 0);
+                    epi.apply16(row, n0 + cc, v, c0 == 0, coff + cc);
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -632,13 +682,13 @@ __global__ void __launch_bounds__(GS_WARPS * 32) gather_split_kernel(GatherPlan 
 
 // C = beta C + sum_z P_z  (P_z dense m x n, z-major)
 __global__ void sum_splits_kernel(const double *__restrict__ P, int splits, int64_t m, int64_t n, double beta,
-                                  double *__restrict__ C, int64_t ldc) {
+                                  OutView C) {
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < m * n;
          idx += (int64_t)gridDim.x * blockDim.x) {
         int64_t r = idx % m, c = idx / m;
         double acc = 0.0;
         for (int z = 0; z < splits; z++) acc += P[(int64_t)z * m * n + idx];
-        double *dst = C + r + ldc * c;
+        double *dst = C.p + OutView::offset((int)r, C.nr, C.rn, C.rs) + OutView::offset((int)c, C.nc, C.cn, C.cs);
         *dst = beta != 0.0 ? beta * *dst + acc : acc;
     }
 }
@@ -799,7 +849,7 @@ template <class Epi>
 void launch_tc(Exec &ex, int planes, const __nv_bfloat16 *A, int64_t a_rows, int64_t a_plane, int64_t m_out,
                const __nv_bfloat16 *B, int64_t b_rows, int64_t b_plane, int64_t n_out, int64_t Kp, const Epi &epi,
                double mnk, int splits = 1, bool pair = false) {
-    if constexpr (std::is_same<Epi, EpiF64>::value) {
+    if constexpr (Epi::kChunked) {
         if (planes == 2 && m_out >= 2 * BM && (pair || pair_gemm_on())) {
             launch_pair(ex, A, a_rows, a_plane, m_out, B, b_rows, b_plane, n_out, Kp, epi, mnk, splits);
             return;
@@ -963,7 +1013,7 @@ std::vector<int> tc_split_candidates(int64_t m, int64_t n, int64_t k, int planes
 }
 
 void mixed_gemm_views(Exec &ex, const SplitView &A, const SplitView &B, int64_t m, int64_t n, int64_t k, double alpha,
-                      double beta, double *C, int64_t ldc, int splits) {
+                      double beta, const OutView &C, int splits) {
     REQUIRE(m < (1ll << 31) && n < (1ll << 31) && k < (1ll << 31), CCSD_GPU_EINVAL, "mixed_gemm: size too large");
     const int np = check_planes(ex.planes);
     const int64_t Kp = round_up(k, BK), Mp = round_up(m, BM), Np = round_up(n, B_ROW_PAD);
@@ -976,9 +1026,12 @@ void mixed_gemm_views(Exec &ex, const SplitView &A, const SplitView &B, int64_t 
     splits = used_splits(splits, Kp / BK);
     const double mnk = double(m) * double(n) * double(k);
     if (splits <= 1) {
-        EpiF64 epi{C, (long long)ldc, (int)m, (int)n, alpha, beta};
-        launch_tc(ex, np, a.as<__nv_bfloat16>(), Mp, Mp * Kp, m, b.as<__nv_bfloat16>(), Np, Np * Kp, n, Kp, epi, mnk, 1,
-                  pair);
+        auto launch = [&](const auto &epi) {
+            launch_tc(ex, np, a.as<__nv_bfloat16>(), Mp, Mp * Kp, m, b.as<__nv_bfloat16>(), Np, Np * Kp, n, Kp, epi, mnk,
+                      1, pair);
+        };
+        if (C.nr == 1 && C.nc == 1 && (C.rs[0] == 1 || m == 1)) launch(EpiF64{C.p, C.cs[0], (int)m, (int)n, alpha, beta});
+        else launch(EpiScatter{C, (int)m, (int)n, alpha, beta});
         return;
     }
     DBuf part = dalloc((int64_t)splits * m * n, ex.stream);
@@ -986,9 +1039,20 @@ void mixed_gemm_views(Exec &ex, const SplitView &A, const SplitView &B, int64_t 
     launch_tc(ex, np, a.as<__nv_bfloat16>(), Mp, Mp * Kp, m, b.as<__nv_bfloat16>(), Np, Np * Kp, n, Kp, epi, mnk,
               splits, pair);
     sum_splits_kernel<<<(unsigned)std::min<int64_t>((m * n + 255) / 256, 148 * 64), 256, 0, ex.stream>>>(
-        part.d(), splits, m, n, beta, C, ldc);
+        part.d(), splits, m, n, beta, C);
     ex.launches++;
     CU_CHECK(cudaGetLastError());
+}
+
+OutView matrix_out(double *p, int64_t m, int64_t n, int64_t ldc) {
+    OutView v{};
+    v.p = p;
+    v.nr = v.nc = 1;
+    v.rn[0] = (int)m;
+    v.cn[0] = (int)n;
+    v.rs[0] = 1;
+    v.cs[0] = ldc;
+    return v;
 }
 
 SplitView matrix_view(const double *p, int64_t rows, int64_t sr, int64_t K, int64_t sk) {
@@ -1008,7 +1072,7 @@ void mixed_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     // op(B)(kk, c) = B[kk + ldb c] (N) or B[c + ldb kk] (T)
     const SplitView a = transA ? matrix_view(A, m, lda, k, 1) : matrix_view(A, m, 1, k, lda);
     const SplitView b = transB ? matrix_view(B, n, 1, k, ldb) : matrix_view(B, n, ldb, k, 1);
-    mixed_gemm_views(ex, a, b, m, n, k, alpha, beta, C, ldc, splits);
+    mixed_gemm_views(ex, a, b, m, n, k, alpha, beta, matrix_out(C, m, n, ldc), splits);
 }
 
 int64_t tc_pad_rows_a(int64_t m) { return round_up(m, BM); }
@@ -1040,7 +1104,7 @@ void tc_gemm_f64(Exec &ex, const __nv_bfloat16 *A, int64_t Mp, const __nv_bfloat
     EpiF64 epi{part.d(), (long long)m, (int)m, (int)n, alpha, 0.0, (long long)m * n};
     launch_tc(ex, np, A, Mp, Mp * Kp, m, B, Np, Np * Kp, n, Kp, epi, mnk, splits, pair);
     sum_splits_kernel<<<(unsigned)std::min<int64_t>((m * n + 255) / 256, 148 * 64), 256, 0, ex.stream>>>(
-        part.d(), splits, m, n, beta, C, ldc);
+        part.d(), splits, m, n, beta, matrix_out(C, m, n, ldc));
     ex.launches++;
     CU_CHECK(cudaGetLastError());
 }

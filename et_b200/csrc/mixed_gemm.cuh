@@ -25,12 +25,31 @@ struct SplitView {
     int nr, nk;
     long long rn[4], rs[4], kn[4], ks[4];
 };
+// FP64 output of the tensor-core GEMM as a strided scatter, digits as above: element (r, c) at
+// p[sum_d digit_d(r) rs[d] + sum_d digit_d(c) cs[d]].  The epilogue writes (and accumulates) a tensor whose
+// index groups interleave where it lies; rows whose first digit has unit stride are written coalesced.
+struct OutView {
+    double *p;
+    int nr, nc;
+    int rn[4], cn[4];
+    long long rs[4], cs[4];
+    __host__ __device__ static long long offset(int x, int nd, const int *n, const long long *s) {
+        long long off = 0;
+        for (int d = 0; d + 1 < nd; d++) {
+            const int q = x / n[d];
+            off += (long long)(x - q * n[d]) * s[d];
+            x = q;
+        }
+        return off + (long long)x * s[nd - 1];
+    }
+};
+OutView matrix_out(double *p, int64_t m, int64_t n, int64_t ldc);
 SplitView matrix_view(const double *p, int64_t rows, int64_t sr, int64_t K, int64_t sk);
 
-// C (m x n, col-major, ldc) = alpha A B^T + beta C for operands given as views: A's rows are the m
-// output rows, B's rows the n output columns, both with the same k contraction indices.
+// C (m x n) = alpha A B^T + beta C for operands and output given as views: A's rows are the m output
+// rows, B's rows the n output columns, both with the same k contraction indices.
 void mixed_gemm_views(Exec &ex, const SplitView &A, const SplitView &B, int64_t m, int64_t n, int64_t k, double alpha,
-                      double beta, double *C, int64_t ldc, int splits = -1);
+                      double beta, const OutView &C, int splits = -1);
 
 // Routes (the `splits` argument of the GEMMs below and of mixed_gemm): s in 1..99 runs the
 // single-CTA kernel with s K splits, PAIR_ROUTE + s the CTA-pair kernel (cta_group::2, 256 x 256

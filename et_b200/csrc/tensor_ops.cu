@@ -434,6 +434,32 @@ bool gather_view(const TV &v, const std::vector<int> &rows, const std::vector<in
     return true;
 }
 
+// C as the output of a GEMM with rows over the dims `rows` and columns over `cols` (first fastest)
+bool out_view(const TV &C, const std::vector<int> &rows, const std::vector<int> &cols, OutView *out) {
+    OutView v{};
+    v.p = C.p;
+    // neighbouring dims that are one run of memory become one (a matrix then is one by one)
+    auto add = [&](int d, int &n, int *ext, long long *str) {
+        if (C.n[d] == 1) return true;
+        if (n > 0 && C.s[d] == str[n - 1] * ext[n - 1]) {
+            ext[n - 1] *= (int)C.n[d];
+            return true;
+        }
+        if (n == 4) return false;
+        ext[n] = (int)C.n[d];
+        str[n++] = C.s[d];
+        return true;
+    };
+    for (int d : rows)
+        if (!add(d, v.nr, v.rn, v.rs)) return false;
+    for (int d : cols)
+        if (!add(d, v.nc, v.cn, v.cs)) return false;
+    if (v.nr == 0) v.rn[v.nr++] = 1;
+    if (v.nc == 0) v.cn[v.nc++] = 1;
+    *out = v;
+    return true;
+}
+
 // bytes that the reordering copies of a product move (each read and written once; an output that is
 // scattered also reads its old values)
 double copy_bytes(const TV &A, bool packA, const TV &B, bool packB, const TV &C, bool scatter) {
@@ -660,53 +686,52 @@ void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B
         permute_add(ex, 1.0, t, beta, C);
     };
     const double fl = 2.0 * double(mM) * double(mN) * double(mK);
-    Route rt = cmode == 1 ? lookup_route(ex, !tB, !tA, mN, mM, mK, fl, true)
-                          : lookup_route(ex, tA, tB, mM, mN, mK, fl, true);
-    SplitView va, vb;
-    if ((packA || packB) && rt.known && rt.mixed && gather_view(A, aM, aK, &va) && gather_view(B, bN, bK, &vb)) {
-        ex.flops += fl;
-        if (trace_level() >= 2)
-            std::fprintf(stderr, "ccsd_gpu gemm [%s] bf16x3 gather m %lld n %lld k %lld  %.3g flop  splits %d\n", spec,
-                         (long long)mM, (long long)mN, (long long)mK, fl, rt.splits);
-        if (cmode == 0) {
-            mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, beta, C.p, ldc, rt.splits);
-        } else if (cmode == 1) {
-            mixed_gemm_views(ex, vb, va, mN, mM, mK, alpha, beta, C.p, ldc, rt.splits);
-        } else {
-            bufC = dalloc(mM * mN, ex.stream);
-            mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, 0.0, bufC.d(), mM, rt.splits);
-            scatter_C();
-        }
-        return;
-    }
-    // a product for cuBLAS whose operands or output are not matrices as they lie: as a strided batch of
-    // GEMMs over an output index (the trial index, or one that sits between the others) where that spares
-    // the copies
-    BatchPlan bp;
-    const bool batch = (packA || packB || cmode == 2) && !takes_digits(ex, mM, mN, mK, fl) &&
-                       find_batch(A, B, C, info, K, oM, oN, copy_bytes(A, packA, B, packB, C, cmode == 2), &bp);
+    // the operands change places when C lies the other way round; a scattered C takes the group that holds
+    // its unit stride as the rows, so that the epilogue writes along it
+    const bool swap = cmode == 1 || (cmode == 2 && !cM.empty() && !cN.empty() && C.s[cN[0]] < C.s[cM[0]]);
+    Route rt = swap ? lookup_route(ex, !tB, !tA, mN, mM, mK, fl, true)
+                    : lookup_route(ex, tA, tB, mM, mN, mK, fl, true);
+    // a product whose operands or output are not matrices as they lie: the tensor-core GEMM gathers and
+    // scatters them itself; for cuBLAS a strided batch of GEMMs over an output index (the trial index, or
+    // one that sits between the others) may spare the copies
+    const bool strided = packA || packB || cmode == 2;
     auto copies = [&]() {
         if (packA && Au.p == A.p) Au = make_contiguous(ex, A, aK, aM, bufA);
         if (packB && Bu.p == B.p) Bu = make_contiguous(ex, B, bK, bN, bufB);
     };
-    if (batch && !rt.known) {
-        // time the candidates on the copies the tensor-core routes would be compared with
+    if (!rt.known) {
+        // timed on the operands as matrices, then dispatched like every later product of this shape
         copies();
-        rt = cmode == 1 ? measure_route(ex, rt, !tB, !tA, mN, mM, mK, alpha, Bu.p, ldb, Au.p, lda, fl, true)
+        rt = swap ? measure_route(ex, rt, !tB, !tA, mN, mM, mK, alpha, Bu.p, ldb, Au.p, lda, fl, true)
                         : measure_route(ex, rt, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, fl, true);
     }
-    if (batch && !rt.mixed) {
+    SplitView va, vb;
+    OutView vc;
+    if (strided && rt.mixed && gather_view(A, aM, aK, &va) && gather_view(B, bN, bK, &vb) &&
+        out_view(C, swap ? cN : cM, swap ? cM : cN, &vc)) {
+        ex.flops += fl;
+        if (trace_level() >= 2)
+            std::fprintf(stderr, "ccsd_gpu gemm [%s] bf16x3 strided m %lld n %lld k %lld  %.3g flop  splits %d\n", spec,
+                         (long long)mM, (long long)mN, (long long)mK, fl, rt.splits);
+        if (swap) mixed_gemm_views(ex, vb, va, mN, mM, mK, alpha, beta, vc, rt.splits);
+        else mixed_gemm_views(ex, va, vb, mM, mN, mK, alpha, beta, vc, rt.splits);
+        return;
+    }
+    BatchPlan bp;
+    if (strided && !rt.mixed && !takes_digits(ex, mM, mN, mK, fl) &&
+        find_batch(A, B, C, info, K, oM, oN, copy_bytes(A, packA, B, packB, C, cmode == 2), &bp)) {
         run_batch(ex, bp, A, B, C, alpha, beta);
         return;
     }
     copies();
+    ex.flops += fl;
     if (cmode == 0) {
-        gemm(ex, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, beta, C.p, ldc);
+        run_gemm(ex, rt, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, beta, C.p, ldc);
     } else if (cmode == 1) {
-        gemm(ex, !tB, !tA, mN, mM, mK, alpha, Bu.p, ldb, Au.p, lda, beta, C.p, ldc);
+        run_gemm(ex, rt, !tB, !tA, mN, mM, mK, alpha, Bu.p, ldb, Au.p, lda, beta, C.p, ldc);
     } else {
         bufC = dalloc(mM * mN, ex.stream);
-        gemm(ex, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, 0.0, bufC.d(), mM);
+        run_gemm(ex, rt, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, 0.0, bufC.d(), mM);
         scatter_C();
     }
 }
