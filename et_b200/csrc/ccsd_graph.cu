@@ -136,7 +136,11 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         g.contract(F_oo, "Jpq,J->pq", 2.0, Lt_oo, X, true);
         g.contract(F_ov, "Jpq,J->pq", 2.0, Lt_ov, X, true);
         g.contract(F_vo, "Jpq,J->pq", 2.0, Lt_vo, X, true);
-        g.contract(F_vv, "Jpq,J->pq", 2.0, Lt_vv, X, true);
+        // 2 sum_J L~_vv X_J through L~_vv = L_vv - t1 L_ov, so that no derivative of L~_vv is formed
+        g.contract(F_vv, "Jpq,J->pq", 2.0, n.L_vv, X, true);
+        const int V = g.zeros("V_jb", {no, nv});
+        g.contract(V, "Jjb,J->jb", 1.0, n.L_ov, X, true);
+        g.contract(F_vv, "aj,jb->ab", -2.0, t1, V, true);
         g.contract(F_oo, "Jpk,Jkq->pq", -1.0, Lt_oo, Lt_oo, true);
         g.contract(F_ov, "Jpk,Jkq->pq", -1.0, Lt_oo, Lt_ov, true);
         g.contract(F_vo, "Jpk,Jkq->pq", -1.0, Lt_vo, Lt_oo, true);
@@ -158,7 +162,14 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         TermTimer tt(ex, "omega doubles a1");
         const int XJ = g.zeros("X_Jbi", {nJ, nv, no});
         g.contract(XJ, "Jcj,cjbi->Jbi", 1.0, n.L_vo, u);
-        g.contract(om1, "Jab,Jbi->ai", 1.0, Lt_vv, XJ);
+        if (const_t1) {
+            g.contract(om1, "Jab,Jbi->ai", 1.0, Lt_vv, XJ);
+        } else {
+            g.contract(om1, "Jab,Jbi->ai", 1.0, n.L_vv, XJ);
+            const int W = g.zeros("W_ji", {no, no});
+            g.contract(W, "Jjb,Jbi->ji", 1.0, n.L_ov, XJ);
+            g.contract(om1, "aj,ji->ai", -1.0, t1, W);
+        }
     }
     {
         // omega_doubles_b1 (:141-204)
@@ -202,7 +213,7 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
     // omega_ccsd_b2 (omega_ccsd.F90:483-583); g_aibj in FP64
     {
         TermTimer tt(ex, "omega ccsd b2");
-        g.contract(om, "Jai,Jbj->aibj", 0.5, Lt_vo, Lt_vo, true);
+        g.contract_sym(om, "Jai,Jbj->aibj", 0.5, Lt_vo, true);
         const int X4 = g.zeros("X_klij", {no, no, no, no});
         g.contract(X4, "Jki,Jlj->klij", 1.0, Lt_oo, Lt_oo);
         g.contract(X4, "kcld,cidj->klij", 1.0, G4, tf);
@@ -212,7 +223,16 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
     {
         TermTimer tt(ex, "omega ccsd c2 and d2");
         const int C = g.zeros("C_term", V4), D = g.zeros("D_term", V4);
-        g.contract(C, "Jac,Jkj->ckaj", 1.0, Lt_vv, Lt_oo);
+        if (const_t1) {
+            g.contract(C, "Jac,Jkj->ckaj", 1.0, Lt_vv, Lt_oo);
+        } else {
+            // g_ackj through L~_vv = L_vv - t1 L_ov: a derivative in t1 costs a product over n_o instead of
+            // one over N_J with an n_v^2 N_J tangent of L~_vv
+            g.contract(C, "Jac,Jkj->ckaj", 1.0, n.L_vv, Lt_oo);
+            const int G = g.zeros("g_lckj", {no, nv, no, no});
+            g.contract(G, "Jlc,Jkj->lckj", 1.0, n.L_ov, Lt_oo);
+            g.contract(C, "al,lckj->ckaj", -1.0, t1, G);
+        }
         g.permute(D, "ckaj->ckaj", -1.0, C);
         g.contract(D, "Jai,Jkc->ckai", 2.0, Lt_vo, Lt_ov);
         g.contract(C, "kcld,djak->claj", -0.5, G4, tf);
@@ -278,6 +298,7 @@ void Context::record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, i
         TermTimer tt(ex, "omega ccsd a2");
         if (ex.prec == Prec::MIXED || f64_resident()) ladder_t1_corrections(g.value(t1), g.value(tf), g.node(om).v);
     };
+    op.tangent_reads = {t1};
     op.tangent = [this, &g, om, Lvv, t1, getY](int nvec) {
         REQUIRE(!g.node(Lvv).active || g.node(t1).active, CCSD_GPU_EINVAL,
                 "ladder tangent: L_vv directions are not supported");
@@ -342,6 +363,7 @@ void Context::record_ladder(Graph &g, int om2, int Lvv, int t2) {
         else
             ladder(g.value(Lvv), g.value(t2), g.node(om2).v);
     };
+    op.tangent_reads = {t2};
     op.tangent = [this, &g, om2, Lvv, t2](int nvec) {
         if (g.node(t2).active) ladder(g.value(Lvv), g.tangent(t2, nvec), g.tangent(om2, nvec), nvec);
     };

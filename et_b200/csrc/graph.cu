@@ -104,6 +104,30 @@ TV Graph::view(int i) const {
     return v;
 }
 
+double *Graph::derivative(int i, int nvec, bool adj) {
+    GNode &n = nodes_[i];
+    DBuf &buf = adj ? n.adj : n.tan;
+    if (!buf) {
+        buf = dalloc(n.size * nvec, ex_.stream);
+        (adj ? n.adj_zero : n.tan_zero) = true;
+    }
+    return buf.d();
+}
+
+double *Graph::tangent(int i, int nvec) {
+    double *p = derivative(i, nvec, false);
+    if (nodes_[i].tan_zero) fill(ex_, p, nodes_[i].size * nvec, 0.0);
+    nodes_[i].tan_zero = false;
+    return p;
+}
+
+double *Graph::adjoint(int i, int nvec) {
+    double *p = derivative(i, nvec, true);
+    if (nodes_[i].adj_zero) fill(ex_, p, nodes_[i].size * nvec, 0.0);
+    nodes_[i].adj_zero = false;
+    return p;
+}
+
 TV Graph::tview(int i, int nvec, bool adj) {
     TV v = view(i);
     v.p = adj ? adjoint(i, nvec) : tangent(i, nvec);
@@ -113,22 +137,12 @@ TV Graph::tview(int i, int nvec, bool adj) {
     return v;
 }
 
-double *Graph::tangent(int i, int nvec) {
-    GNode &n = nodes_[i];
-    if (!n.tan) {
-        n.tan = dalloc(n.size * nvec, ex_.stream);
-        fill(ex_, n.tan.d(), n.size * nvec, 0.0);
-    }
-    return n.tan.d();
-}
-
-double *Graph::adjoint(int i, int nvec) {
-    GNode &n = nodes_[i];
-    if (!n.adj) {
-        n.adj = dalloc(n.size * nvec, ex_.stream);
-        fill(ex_, n.adj.d(), n.size * nvec, 0.0);
-    }
-    return n.adj.d();
+TV Graph::twrite(int i, int nvec, bool adj, double *beta) {
+    derivative(i, nvec, adj);
+    bool &zero = adj ? nodes_[i].adj_zero : nodes_[i].tan_zero;
+    *beta = zero ? 0.0 : 1.0;
+    zero = false;
+    return tview(i, nvec, adj);
 }
 
 void Graph::run_forward(const GOp &op) {
@@ -200,9 +214,26 @@ void Graph::contract(int out, const char *spec, double alpha, int a, int b, bool
     op.alpha = alpha;
     op.spec = spec;
     op.fp64 = fp64;
+    record(std::move(op));
+}
+
+void Graph::contract_sym(int out, const char *spec, double alpha, int a, bool fp64) {
+    GOp op;
+    op.kind = OpKind::Contract;
+    op.out = out;
+    op.a = op.b = a;
+    op.alpha = alpha;
+    op.spec = spec;
+    op.fp64 = fp64;
+    op.sym = true;
+    record(std::move(op));
+}
+
+void Graph::record(GOp op) {
     run_forward(op);
-    nodes_[a].last_use = nodes_[b].last_use = (int)ops_.size();
-    ops_.push_back(op);
+    for (int i : {op.a, op.b})
+        if (i >= 0) nodes_[i].last_use = (int)ops_.size();
+    ops_.push_back(std::move(op));
 }
 
 void Graph::permute(int out, const char *spec, double alpha, int a) {
@@ -212,9 +243,7 @@ void Graph::permute(int out, const char *spec, double alpha, int a) {
     op.a = a;
     op.alpha = alpha;
     op.spec = spec;
-    run_forward(op);
-    nodes_[a].last_use = (int)ops_.size();
-    ops_.push_back(op);
+    record(std::move(op));
 }
 
 void Graph::square_forms(int t, int u, int a, double c1, double c2) {
@@ -225,9 +254,7 @@ void Graph::square_forms(int t, int u, int a, double c1, double c2) {
     op.a = a;
     op.c1 = c1;
     op.c2 = c2;
-    run_forward(op);
-    nodes_[a].last_use = (int)ops_.size();
-    ops_.push_back(op);
+    record(std::move(op));
 }
 
 void Graph::sym_pack(int out, int a, int x, double c1, double c2) {
@@ -238,9 +265,7 @@ void Graph::sym_pack(int out, int a, int x, double c1, double c2) {
     op.b = x;
     op.c1 = c1;
     op.c2 = c2;
-    run_forward(op);
-    nodes_[a].last_use = nodes_[x].last_use = (int)ops_.size();
-    ops_.push_back(op);
+    record(std::move(op));
 }
 
 void Graph::trace(int out, int a) {
@@ -248,9 +273,7 @@ void Graph::trace(int out, int a) {
     op.kind = OpKind::Trace;
     op.out = out;
     op.a = a;
-    run_forward(op);
-    nodes_[a].last_use = (int)ops_.size();
-    ops_.push_back(op);
+    record(std::move(op));
 }
 
 int Graph::custom(CustomOp c, int out, std::vector<int> ins) {
@@ -285,6 +308,7 @@ void Graph::clear_derivatives() {
     for (auto &n : nodes_) {
         n.tan.release();
         n.adj.release();
+        n.tan_zero = n.adj_zero = false;
     }
 }
 
@@ -293,26 +317,42 @@ void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *
     clear_derivatives();
     mark_active(inputs);
     for (size_t k = 0; k < inputs.size(); k++) {
-        double *t = tangent(inputs[k], nvec);
+        double *t = derivative(inputs[k], nvec, false);
+        nodes_[inputs[k]].tan_zero = false;
         CU_CHECK(cudaMemcpyAsync(t, seeds[k], sizeof(double) * nodes_[inputs[k]].size * nvec,
                                  cudaMemcpyDeviceToDevice, ex_.stream));
     }
+    // the tangents that the outputs depend on: an op feeding only others is skipped
+    std::vector<char> needed(nodes_.size(), 0);
+    for (int i : outputs) needed[i] = 1;
+    for (int oi = (int)ops_.size() - 1; oi >= 0; --oi) {
+        const GOp &op = ops_[oi];
+        if (!needed[op.out] && !(op.out2 >= 0 && needed[op.out2])) continue;
+        if (op.kind == OpKind::Custom) {
+            for (int i : customs_[op.custom].tangent_reads) needed[i] = 1;
+        } else {
+            for (int i : {op.a, op.b})
+                if (i >= 0) needed[i] = 1;
+        }
+    }
+    double beta = 1.0;
     for (const GOp &op : ops_) {
-        if (!nodes_[op.out].active) continue;
+        if (!nodes_[op.out].active || !(needed[op.out] || (op.out2 >= 0 && needed[op.out2]))) continue;
         Fp64Scope fp64(ex_, op.fp64);
         switch (op.kind) {
         case OpKind::Contract: {
             std::string s = op.spec;
             size_t comma = s.find(','), ar = s.find("->");
             std::string la = s.substr(0, comma), lb = s.substr(comma + 1, ar - comma - 1), lc = s.substr(ar + 2);
-            TV out = tview(op.out, nvec, false);
-            if (nodes_[op.a].active) {
+            if (nodes_[op.a].active && !op.sym) {
                 std::string sp = with_batch(la) + "," + lb + "->" + with_batch(lc);
-                ccsd::contract(ex_, sp.c_str(), op.alpha, tview(op.a, nvec, false), view(op.b), 1.0, out);
+                const TV in = tview(op.a, nvec, false), out = twrite(op.out, nvec, false, &beta);
+                ccsd::contract(ex_, sp.c_str(), op.alpha, in, view(op.b), beta, out);
             }
             if (nodes_[op.b].active) {
                 std::string sp = la + "," + with_batch(lb) + "->" + with_batch(lc);
-                ccsd::contract(ex_, sp.c_str(), op.alpha, view(op.a), tview(op.b, nvec, false), 1.0, out);
+                const TV in = tview(op.b, nvec, false), out = twrite(op.out, nvec, false, &beta);
+                ccsd::contract(ex_, sp.c_str(), op.sym ? 2.0 * op.alpha : op.alpha, view(op.a), in, beta, out);
             }
             break;
         }
@@ -320,7 +360,7 @@ void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *
             if (!nodes_[op.a].active) break;
             size_t ar = op.spec.find("->");
             std::string lin = op.spec.substr(0, ar) + BATCH, lout = op.spec.substr(ar + 2) + BATCH;
-            TV in = tview(op.a, nvec, false), out = tview(op.out, nvec, false), pin;
+            TV in = tview(op.a, nvec, false), out = twrite(op.out, nvec, false, &beta), pin;
             pin.p = in.p;
             pin.nd = out.nd;
             for (int k = 0; k < out.nd; k++) {
@@ -328,17 +368,20 @@ void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *
                 pin.n[k] = in.n[pos];
                 pin.s[k] = in.s[pos];
             }
-            permute_add(ex_, op.alpha, pin, 1.0, out);
+            permute_add(ex_, op.alpha, pin, beta, out);
             break;
         }
-        case OpKind::SquareForms:
-            ccsd::square_forms(ex_, tangent(op.a, nvec), no, nv, nvec, op.c1, op.c2, tangent(op.out, nvec),
-                               tangent(op.out2, nvec), true, true);
+        case OpKind::SquareForms: {
+            double beta_u = 1.0;
+            const TV t = twrite(op.out, nvec, false, &beta), u = twrite(op.out2, nvec, false, &beta_u);
+            ccsd::square_forms(ex_, tangent(op.a, nvec), no, nv, nvec, op.c1, op.c2, t.p, u.p, beta != 0.0, beta_u != 0.0);
             break;
+        }
         case OpKind::SymPack: {
             const double *fa = nodes_[op.a].active ? tangent(op.a, nvec) : nullptr;
             const double *xa = nodes_[op.b].active ? tangent(op.b, nvec) : nullptr;
-            ccsd::sym_pack(ex_, fa, xa, no, nv, nvec, op.c1, op.c2, tangent(op.out, nvec), true);
+            const TV out = twrite(op.out, nvec, false, &beta);
+            ccsd::sym_pack(ex_, fa, xa, no, nv, nvec, op.c1, op.c2, out.p, beta != 0.0);
             break;
         }
         case OpKind::Trace: {
@@ -357,7 +400,7 @@ void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *
     }
     for (size_t k = 0; k < outputs.size(); k++) {
         const GNode &n = nodes_[outputs[k]];
-        if (n.active && n.tan)
+        if (n.active && n.tan && !n.tan_zero)
             CU_CHECK(cudaMemcpyAsync(results[k], n.tan.d(), sizeof(double) * n.size * nvec, cudaMemcpyDeviceToDevice,
                                      ex_.stream));
         else
@@ -370,27 +413,31 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
     clear_derivatives();
     mark_active(inputs);
     for (size_t k = 0; k < outputs.size(); k++) {
-        double *a = adjoint(outputs[k], nvec);
-        axpby(ex_, nodes_[outputs[k]].size * nvec, 1.0, seeds[k], 1.0, a);
+        double beta;
+        const TV a = twrite(outputs[k], nvec, true, &beta);
+        axpby(ex_, nodes_[outputs[k]].size * nvec, 1.0, seeds[k], beta, a.p);
     }
+    double beta = 1.0;
     for (int oi = (int)ops_.size() - 1; oi >= 0; --oi) {
         const GOp &op = ops_[oi];
         if (!nodes_[op.out].active) continue;
-        if (!nodes_[op.out].adj && !(op.out2 >= 0 && nodes_[op.out2].adj)) continue;
+        if (!has_adjoint(op.out) && !(op.out2 >= 0 && has_adjoint(op.out2))) continue;
         Fp64Scope fp64(ex_, op.fp64);
         switch (op.kind) {
         case OpKind::Contract: {
             std::string s = op.spec;
             size_t comma = s.find(','), ar = s.find("->");
             std::string la = s.substr(0, comma), lb = s.substr(comma + 1, ar - comma - 1), lc = s.substr(ar + 2);
-            TV cbar = tview(op.out, nvec, true);
-            if (nodes_[op.a].active) {
+            const TV cbar = tview(op.out, nvec, true);
+            if (nodes_[op.a].active && !op.sym) {
                 std::string sp = with_batch(lc) + "," + lb + "->" + with_batch(la);
-                ccsd::contract(ex_, sp.c_str(), op.alpha, cbar, view(op.b), 1.0, tview(op.a, nvec, true));
+                const TV out = twrite(op.a, nvec, true, &beta);
+                ccsd::contract(ex_, sp.c_str(), op.alpha, cbar, view(op.b), beta, out);
             }
             if (nodes_[op.b].active) {
                 std::string sp = la + "," + with_batch(lc) + "->" + with_batch(lb);
-                ccsd::contract(ex_, sp.c_str(), op.alpha, view(op.a), cbar, 1.0, tview(op.b, nvec, true));
+                const TV out = twrite(op.b, nvec, true, &beta);
+                ccsd::contract(ex_, sp.c_str(), op.sym ? 2.0 * op.alpha : op.alpha, view(op.a), cbar, beta, out);
             }
             break;
         }
@@ -399,7 +446,7 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
             // a_bar[lin] += alpha * out_bar[lout]
             size_t ar = op.spec.find("->");
             std::string lin = op.spec.substr(0, ar) + BATCH, lout = op.spec.substr(ar + 2) + BATCH;
-            TV obar = tview(op.out, nvec, true), abar = tview(op.a, nvec, true), pin;
+            TV obar = tview(op.out, nvec, true), abar = twrite(op.a, nvec, true, &beta), pin;
             pin.p = obar.p;
             pin.nd = abar.nd;
             for (int k = 0; k < abar.nd; k++) {
@@ -407,7 +454,7 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
                 pin.n[k] = obar.n[pos];
                 pin.s[k] = obar.s[pos];
             }
-            permute_add(ex_, op.alpha, pin, 1.0, abar);
+            permute_add(ex_, op.alpha, pin, beta, abar);
             break;
         }
         case OpKind::SquareForms: {
@@ -415,16 +462,19 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
             // transpose is the symmetrised packing of the two adjoints
             const double *sa = has_adjoint(op.out) ? adjoint(op.out, nvec) : nullptr;
             const double *ua = has_adjoint(op.out2) ? adjoint(op.out2, nvec) : nullptr;
-            ccsd::sym_pack(ex_, sa, ua, no, nv, nvec, op.c1, op.c2, adjoint(op.a, nvec), true);
+            const TV out = twrite(op.a, nvec, true, &beta);
+            ccsd::sym_pack(ex_, sa, ua, no, nv, nvec, op.c1, op.c2, out.p, beta != 0.0);
             break;
         }
-        case OpKind::SymPack:
+        case OpKind::SymPack: {
             // d packed[(M, m)] / d z[x, y] = 1 for {x, y} = {M, m} (the diagonal's 1/2 meets two
             // equal entries): the adjoint is the full symmetric square-up of the packed adjoint
-            ccsd::square_forms(ex_, adjoint(op.out, nvec), no, nv, nvec, op.c1, op.c2,
-                               nodes_[op.a].active ? adjoint(op.a, nvec) : nullptr,
-                               nodes_[op.b].active ? adjoint(op.b, nvec) : nullptr, true, true);
+            double *fa = nullptr, *xa = nullptr, beta_x = 1.0;
+            if (nodes_[op.a].active) fa = twrite(op.a, nvec, true, &beta).p;
+            if (nodes_[op.b].active) xa = twrite(op.b, nvec, true, &beta_x).p;
+            ccsd::square_forms(ex_, adjoint(op.out, nvec), no, nv, nvec, op.c1, op.c2, fa, xa, beta != 0.0, beta_x != 0.0);
             break;
+        }
         case OpKind::Trace: {
             if (!nodes_[op.a].active) break;
             const GNode &a = nodes_[op.a];
@@ -441,7 +491,7 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
     }
     for (size_t k = 0; k < inputs.size(); k++) {
         const GNode &n = nodes_[inputs[k]];
-        if (n.adj)
+        if (n.adj && !n.adj_zero)
             CU_CHECK(cudaMemcpyAsync(results[k], n.adj.d(), sizeof(double) * n.size * nvec, cudaMemcpyDeviceToDevice,
                                      ex_.stream));
         else

@@ -20,6 +20,9 @@ struct GNode {
     double *v = nullptr;         // primal value
     DBuf own;                    // storage when the graph owns the primal
     DBuf tan, adj;               // [size x nvec]
+    // allocated and not written yet: reads as zero, and the first op writing it overwrites (clearing every
+    // derivative first was a pass over each of them: 3 of 128 ms for six trials at o=24, v=240)
+    bool tan_zero = false, adj_zero = false;
     bool active = false;         // depends on a differentiated input
     bool zero = false;           // allocated by zeros() and not written yet: reads as zero, and the
                                  // first op writing it overwrites instead of accumulating
@@ -33,6 +36,7 @@ struct CustomOp {
     std::function<void()> forward;
     std::function<void(int nvec)> tangent;   // reads input tangents, accumulates out tangent
     std::function<void(int nvec)> adjoint;   // reads out adjoint, accumulates input adjoints
+    std::vector<int> tangent_reads;          // the nodes whose tangents `tangent` reads
 };
 
 struct GOp {
@@ -43,6 +47,9 @@ struct GOp {
     double c1 = 0.0, c2 = 0.0;   // SquareForms, SymPack: weights of a form and of its exchange
     std::string spec;            // contract: "la,lb->lc"; permute: "lin->lout"
     bool fp64 = false;           // force FP64 (first-order terms)
+    // contract of a node with itself whose output is only read as out + out^T: one of the two equal halves of
+    // its derivative, 7 of 128 ms for six trials at o=24, v=240
+    bool sym = false;
     int custom = -1;
 };
 
@@ -59,6 +66,9 @@ class Graph {
 
     // out += alpha * einsum(spec, a, b)
     void contract(int out, const char *spec, double alpha, int a, int b, bool fp64 = false);
+    // out += alpha * einsum(spec, a, a), symmetric under exchange of the two factors' indices, where every
+    // reader of out takes its symmetric part (sym_pack): the two terms of its derivative count the same
+    void contract_sym(int out, const char *spec, double alpha, int a, bool fp64 = false);
     // out += alpha * permute(a), spec "ajbi->aibj" (labels name the dims of a / out)
     void permute(int out, const char *spec, double alpha, int a);
     // t (full (v,o,v,o)) += squareup(a packed), u += c1 t_aibj + c2 t_ajbi
@@ -90,10 +100,9 @@ class Graph {
              const std::vector<int> &inputs, const std::vector<double *> &results);
 
     // helpers for custom ops
-    double *tangent(int i, int nvec);   // allocates (zeroed) on first use
+    double *tangent(int i, int nvec);   // allocated on first use; zero where nothing has been written
     double *adjoint(int i, int nvec);
-    bool has_tangent(int i) const { return (bool)nodes_[i].tan; }
-    bool has_adjoint(int i) const { return (bool)nodes_[i].adj; }
+    bool has_adjoint(int i) const { return (bool)nodes_[i].adj && !nodes_[i].adj_zero; }
     Exec &exec() { return ex_; }
 
   private:
@@ -106,7 +115,13 @@ class Graph {
     TV view(int node) const;
     // fills a node that zeros() allocated and nothing has written yet
     void materialize(int node);
+    // the node's tangents / adjoints as a view over (node dims, trial)
     TV tview(int node, int nvec, bool adjoint);
+    // the same for an op that writes every element: *beta is 0 when nothing has been written yet (the op
+    // then overwrites), else 1
+    TV twrite(int node, int nvec, bool adjoint, double *beta);
+    double *derivative(int node, int nvec, bool adjoint);   // allocated, contents undefined while zero
+    void record(GOp op);
 };
 
 }  // namespace ccsd
