@@ -151,6 +151,137 @@ sym_pack_kernel(const double *__restrict__ F, const double *__restrict__ X, int 
     }
 }
 
+struct TpmOut {
+    double *p, *m;                 // FP64 columns
+    __nv_bfloat16 *bp, *bm;        // or bf16 planes
+    int64_t ldp, ldm, plane_p, plane_m;
+    int np;
+};
+
+__device__ __forceinline__ void put_planes(double x, int np, int64_t plane, __nv_bfloat16 *out) {
+    for (int q = 0; q < np; q++) {
+        const __nv_bfloat16 h = __double2bfloat16(x);
+        out[q * plane] = h;
+        x -= (double)__bfloat162float(h);
+    }
+}
+
+// An occupied pair i >= j and a 32 x 32 tile of (c, d), c >= d: t_cidj lies along d in its packed row
+// (c, i), t_cjdi along c in row (d, i), turned in shared memory; both forms are stored along d.  Bound by
+// HBM: n_t2 read, the forms written; each thread of the element-wise version found its four indices by two
+// square roots and read two elements whose neighbours lay a packed row apart.  bf16 planes at o=32, v=320
+// 0.54 ms (1.2 TB/s).
+template <bool PLANES>
+__global__ void __launch_bounds__(TILE * ROWS)
+tpm_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec, TpmOut o) {
+    __shared__ double s[TILE][TILE + 1];   // t_cjdi of (c0 + x, d0 + r) at [r][x]
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int64_t nov = (int64_t)no * nv, nt2 = nov * (nov + 1) / 2;
+    const int64_t nop = (int64_t)no * (no + 1) / 2, nom = (int64_t)no * (no - 1) / 2;
+    int ct, dt, i, j;
+    untri32(blockIdx.x, ct, dt);
+    const int c0 = TILE * ct, d0 = TILE * dt;
+    for (int64_t w = blockIdx.y; w < nop * nvec; w += gridDim.y) {
+        const int64_t n = w / nop;
+        untri32((unsigned)(w - n * nop), i, j);
+        const double *p = packed + nt2 * n;
+        double x[TILE / ROWS];
+#pragma unroll
+        for (int k = 0; k < TILE / ROWS; k++) {
+            const int r = ty + ROWS * k;
+            if (c0 + tx < nv && d0 + r < nv) s[r][tx] = p[packed_at(d0 + r + (int64_t)nv * i, c0 + tx + (int64_t)nv * j)];
+            x[k] = c0 + r < nv && d0 + tx <= c0 + r ? p[packed_at(c0 + r + (int64_t)nv * i, d0 + tx + (int64_t)nv * j)] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < TILE / ROWS; k++) {
+            const int c = c0 + ty + ROWS * k, d = d0 + tx;
+            if (c >= nv || d > c) continue;
+            const double y = s[tx][ty + ROWS * k];
+            const double f = (c == d ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
+            const int64_t at = w * o.ldp + (int64_t)c * (c + 1) / 2 + d;
+            if (PLANES) put_planes(f * (x[k] + y), o.np, o.plane_p, o.bp + at);
+            else o.p[at] = f * (x[k] + y);
+            if (i > j && c > d) {
+                const int64_t am = (n * nom + (int64_t)i * (i - 1) / 2 + j) * o.ldm + (int64_t)c * (c - 1) / 2 + d;
+                if (PLANES) put_planes(x[k] - y, o.np, o.plane_m, o.bm + am);
+                else o.m[am] = x[k] - y;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// An occupied pair i >= j and a 32 x 32 tile of (a, b), a >= b: w+- are read along b, Omega_aibj is added
+// to along b in its packed row (a, i), Omega_ajbi along a in row (b, i) through shared memory.  Bound by
+// HBM: w+- read, n_t2 read and written.  The element-wise version ran along ij, so that neighbouring threads
+// updated packed rows far apart: 1.37 ms at o=32, v=320; so 0.54 (2.3 TB/s).
+__global__ void __launch_bounds__(TILE * ROWS)
+add_omega_pm_kernel(double *__restrict__ om2, const double *__restrict__ wp, const double *__restrict__ wm, int no, int nv,
+                    int64_t nvec, int a0, int a1, int64_t ldwp, int64_t ldwm) {
+    __shared__ double s[TILE][TILE + 1];   // the Omega_ajbi share of (a, b) at [a][b]
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int64_t nov = (int64_t)no * nv, nt2 = nov * (nov + 1) / 2;
+    const int64_t nop = (int64_t)no * (no + 1) / 2, nom = (int64_t)no * (no - 1) / 2;
+    const int at0 = a0 / TILE, nbt = (a1 - 1) / TILE + 1;
+    const int at = at0 + (int)blockIdx.x / nbt, bt = (int)blockIdx.x % nbt;
+    if (bt > at) return;
+    const int64_t row0 = (int64_t)a0 * (a0 + 1) / 2, row0m = (int64_t)a0 * (a0 - 1) / 2;
+    for (int64_t w = blockIdx.y; w < nop * nvec; w += gridDim.y) {
+        const int64_t n = w / nop;
+        int i, j;
+        untri32((unsigned)(w - n * nop), i, j);
+        const int64_t cm = n * nom + (int64_t)i * (i - 1) / 2 + j;
+        double *om = om2 + nt2 * n;
+        double v[TILE / ROWS], old[TILE / ROWS];
+#pragma unroll
+        for (int k = 0; k < TILE / ROWS; k++) {
+            const int a = TILE * at + ty + ROWS * k, b = TILE * bt + tx;
+            double x1 = 0.0, x2 = 0.0;
+            old[k] = 0.0;
+            if (a >= a0 && a < a1 && b <= a) {
+                const int64_t M = a + (int64_t)nv * i;
+                old[k] = om[M * (M + 1) / 2 + b + (int64_t)nv * j];
+                const double p = wp[(int64_t)a * (a + 1) / 2 + b - row0 + ldwp * w] * (a == b ? 0.5 : 1.0);
+                if (i == j || a == b) {
+                    x1 = p + p;   // both shares fall on one element
+                } else {
+                    const double m = wm[(int64_t)a * (a - 1) / 2 + b - row0m + ldwm * cm];
+                    x1 = p + m;
+                    x2 = p - m;
+                }
+            }
+            v[k] = x1;
+            s[ty + ROWS * k][tx] = x2;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < TILE / ROWS; k++) {
+            const int a = TILE * at + ty + ROWS * k, b = TILE * bt + tx;
+            if (a >= a0 && a < a1 && b <= a) {
+                const int64_t M = a + (int64_t)nv * i;
+                om[M * (M + 1) / 2 + b + (int64_t)nv * j] = old[k] + v[k];
+            }
+        }
+        if (i != j) {
+            double e[TILE / ROWS];
+#pragma unroll
+            for (int k = 0; k < TILE / ROWS; k++) {
+                const int b = TILE * bt + ty + ROWS * k, a = TILE * at + tx;
+                const int64_t M = b + (int64_t)nv * i;
+                e[k] = a >= a0 && a < a1 && b < a ? om[M * (M + 1) / 2 + a + (int64_t)nv * j] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < TILE / ROWS; k++) {
+                const int b = TILE * bt + ty + ROWS * k, a = TILE * at + tx;
+                const int64_t M = b + (int64_t)nv * i;
+                if (a >= a0 && a < a1 && b < a) om[M * (M + 1) / 2 + a + (int64_t)nv * j] = e[k] + s[tx][ty + ROWS * k];
+            }
+        }
+        __syncthreads();
+    }
+}
+
 dim3 pair_grid(int64_t no, int64_t nv, int64_t nvec) {
     const int64_t nt = (nv + TILE - 1) / TILE;
     return dim3((unsigned)(nt * (nt + 1) / 2), (unsigned)std::min<int64_t>(no * (no + 1) / 2 * nvec, 65535));
@@ -178,6 +309,41 @@ void sym_pack(Exec &ex, const double *F, const double *X, int64_t no, int64_t nv
     if (F && X) pick(yes, yes);
     else if (F) pick(yes, none);
     else pick(none, yes);
+    ex.launches++;
+    CU_CHECK(cudaGetLastError());
+}
+
+void build_tpm(Exec &ex, const double *t2, int64_t no, int64_t nv, int64_t nvec, double *tp, int64_t ldp, double *tm,
+               int64_t ldm) {
+    const TpmOut o{tp, tm, nullptr, nullptr, ldp, ldm, 0, 0, 0};
+    tpm_forms_kernel<false><<<pair_grid(no, nv, nvec), dim3(TILE, ROWS), 0, ex.stream>>>(t2, (int)no, (int)nv, nvec, o);
+    ex.launches++;
+    CU_CHECK(cudaGetLastError());
+}
+
+void build_tpm_planes(Exec &ex, const double *t2, int64_t no, int64_t nv, int64_t nvec, int np, __nv_bfloat16 *tp,
+                      int64_t rows_p, int64_t ldp, __nv_bfloat16 *tm, int64_t rows_m, int64_t ldm) {
+    const TpmOut o{nullptr, nullptr, tp, tm, ldp, ldm, rows_p * ldp, rows_m * ldm, np};
+    const size_t eb = sizeof(__nv_bfloat16);
+    auto clear = [&](__nv_bfloat16 *t, int64_t rows, int64_t used, int64_t ld, int64_t k) {
+        if (ld > k) CU_CHECK(cudaMemset2DAsync(t + k, ld * eb, 0, (ld - k) * eb, (size_t)np * rows, ex.stream));
+        if (rows > used)
+            CU_CHECK(cudaMemset2DAsync(t + used * ld, rows * ld * eb, 0, (rows - used) * ld * eb, np, ex.stream));
+    };
+    clear(tp, rows_p, nvec * (no * (no + 1) / 2), ldp, nv * (nv + 1) / 2);
+    clear(tm, rows_m, nvec * (no * (no - 1) / 2), ldm, nv * (nv - 1) / 2);
+    tpm_forms_kernel<true><<<pair_grid(no, nv, nvec), dim3(TILE, ROWS), 0, ex.stream>>>(t2, (int)no, (int)nv, nvec, o);
+    ex.launches++;
+    CU_CHECK(cudaGetLastError());
+}
+
+void add_omega_pm(Exec &ex, double *om2, const double *wp, const double *wm, int64_t no, int64_t nv, int64_t nvec,
+                  int64_t a0, int64_t a1, int64_t ldwp, int64_t ldwm) {
+    if (a1 <= a0) return;
+    const int64_t nbt = (a1 - 1) / TILE + 1, nat = nbt - a0 / TILE;
+    const dim3 g((unsigned)(nat * nbt), (unsigned)std::min<int64_t>(no * (no + 1) / 2 * nvec, 65535));
+    add_omega_pm_kernel<<<g, dim3(TILE, ROWS), 0, ex.stream>>>(om2, wp, wm, (int)no, (int)nv, nvec, (int)a0, (int)a1,
+                                                              ldwp, ldwm);
     ex.launches++;
     CU_CHECK(cudaGetLastError());
 }

@@ -328,10 +328,10 @@ void Context::ladder(const double *Lvv, const double *t2, double *om2, int64_t n
     cudaStream_t s = ex.stream;
     const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
-    // the nvec vectors side by side: rows [v n_o_p, (v+1) n_o_p) of t+ belong to vector v
-    const int64_t ldp = nvec * nop, ldm = std::max<int64_t>(nvec * nom, 1);
-    DBuf tp = dalloc(ldp * nvp, s), tm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
-    for (int64_t v = 0; v < nvec; v++) build_tpm(ex, t2 + v * nt2, tp.d() + v * nop, tm.d() + v * nom, no, nv, ldp, ldm);
+    // the nvec vectors side by side: columns [v n_o_p, (v+1) n_o_p) of t+ belong to vector v
+    const int64_t np = nvec * nop, nm = nvec * nom;
+    DBuf tp = dalloc(np * nvp, s), tm = dalloc(std::max<int64_t>(nm * nvm, 1), s);
+    build_tpm(ex, t2, no, nv, nvec, tp.d(), nvp, tm.d(), nvm);
     // L~_vv as (J, c, a): columns (c, a) of one a-block are contiguous
     DBuf LT = dalloc(nJ * nv * nv, s);
     {
@@ -351,7 +351,7 @@ void Context::ladder(const double *Lvv, const double *t2, double *om2, int64_t n
     int64_t nA = ladder_batch;
     if (nA <= 0) {
         const double budget = 6.0e9;   // bytes
-        double per_a = 8.0 * (double)nv * nv * nv + 16.0 * (double)nvp * nv + 16.0 * (double)ldp * nv;
+        double per_a = 8.0 * (double)nv * nv * nv + 16.0 * (double)nvp * nv + 16.0 * (double)np * nv;
         nA = std::max<int64_t>(1, std::min<int64_t>(nv, (int64_t)(budget / per_a)));
     }
     int64_t maxab = 0;
@@ -361,7 +361,7 @@ void Context::ladder(const double *Lvv, const double *t2, double *om2, int64_t n
     }
     DBuf G = dalloc(nv * nA * nv * nv, s);
     DBuf gp = dalloc(nvp * maxab, s), gm = dalloc(std::max<int64_t>(nvm * maxab, 1), s);
-    DBuf wp = dalloc(ldp * maxab, s), wm = dalloc(ldm * maxab, s);
+    DBuf wp = dalloc(np * maxab, s), wm = dalloc(std::max<int64_t>(nm * maxab, 1), s);
     for (int64_t a0 = 0; a0 < nv; a0 += nA) {
         int64_t a1 = std::min(nv, a0 + nA);
         int64_t M = nv * (a1 - a0), N = nv * a1;
@@ -370,11 +370,9 @@ void Context::ladder(const double *Lvv, const double *t2, double *om2, int64_t n
         form_gpm(ex, G.d(), M, gp.d(), gm.d(), nv, a0, a1);
         int64_t nabp = a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2;
         int64_t nabm = a1 * (a1 - 1) / 2 - a0 * (a0 - 1) / 2;
-        gemm(ex, false, false, ldp, nabp, nvp, 0.5, tp.d(), ldp, gp.d(), nvp, 0.0, wp.d(), ldp);
-        if (nom > 0 && nabm > 0)
-            gemm(ex, false, false, nvec * nom, nabm, nvm, 0.5, tm.d(), ldm, gm.d(), nvm, 0.0, wm.d(), ldm);
-        for (int64_t v = 0; v < nvec; v++)
-            add_omega_pm(ex, om2 + v * nt2, wp.d() + v * nop, wm.d() + v * nom, no, nv, a0, a1, ldp, ldm);
+        gemm(ex, true, false, nabp, np, nvp, 0.5, gp.d(), nvp, tp.d(), nvp, 0.0, wp.d(), nabp);
+        if (nom > 0 && nabm > 0) gemm(ex, true, false, nabm, nm, nvm, 0.5, gm.d(), nvm, tm.d(), nvm, 0.0, wm.d(), nabm);
+        add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, nvec, a0, a1, nabp, nabm);
     }
 }
 
@@ -493,37 +491,38 @@ void Context::ladder_pairs(const double *Lvv, bool untransformed) {
     cache_epoch++;
 }
 
-// t+ and t- planes of nvec packed vectors (the A operands of the +/- GEMMs)
+// t+ and t- planes of nvec packed vectors (the B operands of the +/- GEMMs)
 Context::TPlanes Context::t_planes(const double *t2, int64_t nvec) {
     const PairShape ps = pair_shape(nv);
     const int np = ex.planes;
     const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
     TPlanes T;
-    T.rows_p = tc_pad_rows_a(nvec * nop);
-    T.rows_m = tc_pad_rows_a(std::max<int64_t>(nvec * nom, 1));
+    T.rows_p = (nvec * nop + 31) / 32 * 32;
+    T.rows_m = (std::max<int64_t>(nvec * nom, 1) + 31) / 32 * 32;
     T.p = DBuf(sizeof(__nv_bfloat16) * np * T.rows_p * ps.kp, ex.stream);
     T.m = DBuf(sizeof(__nv_bfloat16) * np * T.rows_m * ps.km, ex.stream);
-    build_tpm_planes(ex, t2, nvec, no, nv, true, T.rows_p, ps.kp, np, T.p.as<__nv_bfloat16>());
-    build_tpm_planes(ex, t2, nvec, no, nv, false, T.rows_m, ps.km, np, T.m.as<__nv_bfloat16>());
+    build_tpm_planes(ex, t2, no, nv, nvec, np, T.p.as<__nv_bfloat16>(), T.rows_p, ps.kp, T.m.as<__nv_bfloat16>(), T.rows_m,
+                     ps.km);
     return T;
 }
 
-// om2[v] += the ladder of the pairs a in [a0, a1), whose g+- planes are Pp / Pm (row 0 = the
-// block's first pair, prow / mrow padded rows per plane)
+// om2[v] += the ladder of the pairs a in [a0, a1), whose g+- planes are Pp / Pm (row 0 = the block's first
+// pair, prow / mrow padded rows per plane): W = P t^T with the pairs as the rows, so the few columns ij fit
+// an N tile of their own width and W is read along the pairs.  The K splits depend on the whole ladder, not
+// on the block, so every element is the same sum whatever the block.
 void Context::ladder_pm_block(const TPlanes &T, int64_t nvec, const __nv_bfloat16 *Pp, int64_t prow,
                               const __nv_bfloat16 *Pm, int64_t mrow, int64_t a0, int64_t a1, double *om2) {
     const PairShape ps = pair_shape(nv);
-    const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
+    const int64_t np = nvec * (no * (no + 1) / 2), nm = nvec * (no * (no - 1) / 2);
     const int64_t nabp = a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2, nabm = a1 * (a1 - 1) / 2 - a0 * (a0 - 1) / 2;
-    const int64_t ldp = nvec * nop, ldm = std::max<int64_t>(nvec * nom, 1);
-    DBuf wp = dalloc(ldp * nabp, ex.stream), wm = dalloc(ldm * std::max<int64_t>(nabm, 1), ex.stream);
-    tc_gemm_f64(ex, T.p.as<__nv_bfloat16>(), T.rows_p, Pp, prow, ps.kp, ldp, nabp, ps.nvp, 0.5, 0.0, wp.d(), ldp, 1);
-    if (nom > 0 && nabm > 0)
-        tc_gemm_f64(ex, T.m.as<__nv_bfloat16>(), T.rows_m, Pm, mrow, ps.km, nvec * nom, nabm, ps.nvm, 0.5, 0.0, wm.d(),
-                    ldm, 1);
-    for (int64_t v = 0; v < nvec; v++)
-        add_omega_pm(ex, om2 + v * nt2, wp.d() + v * nop, wm.d() + v * nom, no, nv, a0, a1, ldp, ldm);
-    ex.flops += 2.0 * double(ldp) * double(nabp) * double(ps.nvp) + 2.0 * double(nvec * nom) * double(nabm) * double(ps.nvm);
+    DBuf wp = dalloc(np * nabp, ex.stream), wm = dalloc(std::max<int64_t>(nm * nabm, 1), ex.stream);
+    tc_gemm_f64(ex, Pp, prow, T.p.as<__nv_bfloat16>(), T.rows_p, ps.kp, nabp, np, ps.nvp, 0.5, 0.0, wp.d(), nabp,
+                tc_tall_route(ps.nvp, np, ps.kp, ex.planes));
+    if (nm > 0 && nabm > 0)
+        tc_gemm_f64(ex, Pm, mrow, T.m.as<__nv_bfloat16>(), T.rows_m, ps.km, nabm, nm, ps.nvm, 0.5, 0.0, wm.d(), nabm,
+                    tc_tall_route(ps.nvm, nm, ps.km, ex.planes));
+    add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, nvec, a0, a1, nabp, nabm);
+    ex.flops += 2.0 * double(np) * double(nabp) * double(ps.nvp) + 2.0 * double(nm) * double(nabm) * double(ps.nvm);
 }
 
 void Context::ladder_tc(const double *Lvv, const double *t2, double *om2, int64_t nvec, bool untransformed) {
@@ -552,8 +551,7 @@ void Context::ladder_tc_streamed(const double *Lvv, const double *t2, double *om
     cudaStream_t s = ex.stream;
     const int np = ex.planes;
     const PairShape ps = pair_shape(nv);
-    const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
-    const int64_t ldp = nvec * nop, ldm = std::max<int64_t>(nvec * nom, 1);
+    const int64_t ldp = nvec * (no * (no + 1) / 2), ldm = std::max<int64_t>(nvec * (no * (no - 1) / 2), 1);
     DBuf LT = lvv_jca(Lvv);
     const TPlanes T = t_planes(t2, nvec);
     // blocks: consecutive a whose G, planes and W fit the budget (or a quarter of the free memory),
@@ -822,26 +820,24 @@ void Context::ladder_f64(const double *t2, double *om2) {
     cudaStream_t s = ex.stream;
     const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
-    const int64_t ldm = std::max<int64_t>(nom, 1);
     const int digits = f64_ladder_digits();
     const int level = digits ? f64_digit_planes(digits) : 0;
     // X0 = sum_cd g_acbd t_cidj of the untransformed integrals, all pairs in two GEMMs
-    DBuf tp = dalloc(nop * nvp, s), tm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
-    build_tpm(ex, t2, tp.d(), tm.d(), no, nv, nop, ldm);
-    DBuf wp = dalloc(nop * nvp, s), wm = dalloc(ldm * std::max<int64_t>(nvm, 1), s);
+    DBuf tp = dalloc(nop * nvp, s), tm = dalloc(std::max<int64_t>(nom * nvm, 1), s);
+    build_tpm(ex, t2, no, nv, 1, tp.d(), nvp, tm.d(), nvm);
+    DBuf wp = dalloc(nop * nvp, s), wm = dalloc(std::max<int64_t>(nom * nvm, 1), s);
     if (level >= 1) {
-        ozaki_gemm(ex, false, false, nop, nvp, nvp, 0.5, tp.d(), nop, f64_gp.d(), nvp, 0.0, wp.d(), nop, digits,
-                   nullptr, &f64_gp_dig);
+        ozaki_gemm(ex, true, false, nvp, nop, nvp, 0.5, f64_gp.d(), nvp, tp.d(), nvp, 0.0, wp.d(), nvp, digits, &f64_gp_dig);
         if (nom > 0 && nvm > 0)
-            ozaki_gemm(ex, false, false, nom, nvm, nvm, 0.5, tm.d(), ldm, f64_gm.d(), nvm, 0.0, wm.d(), ldm, digits,
-                       nullptr, &f64_gm_dig);
+            ozaki_gemm(ex, true, false, nvm, nom, nvm, 0.5, f64_gm.d(), nvm, tm.d(), nvm, 0.0, wm.d(), nvm, digits,
+                       &f64_gm_dig);
         ex.flops += 2.0 * (double(nop) * nvp * nvp + double(nom) * nvm * nvm);
     } else {
-        gemm(ex, false, false, nop, nvp, nvp, 0.5, tp.d(), nop, f64_gp.d(), nvp, 0.0, wp.d(), nop, false);
+        gemm(ex, true, false, nvp, nop, nvp, 0.5, f64_gp.d(), nvp, tp.d(), nvp, 0.0, wp.d(), nvp, false);
         if (nom > 0 && nvm > 0)
-            gemm(ex, false, false, nom, nvm, nvm, 0.5, tm.d(), ldm, f64_gm.d(), nvm, 0.0, wm.d(), ldm, false);
+            gemm(ex, true, false, nvm, nom, nvm, 0.5, f64_gm.d(), nvm, tm.d(), nvm, 0.0, wm.d(), nvm, false);
     }
-    add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, 0, nv, nop, ldm);
+    add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, 1, 0, nv, nvp, nvm);
 }
 
 void Context::ladder_y_plain(const double *tf, double *Y) {

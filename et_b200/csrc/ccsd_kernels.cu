@@ -35,24 +35,6 @@ inline int grid_for(int64_t total, int block) {
 #define GRID_STRIDE(i, total) \
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (total); i += (int64_t)gridDim.x * blockDim.x)
 
-__global__ void build_tpm_kernel(const double *__restrict__ t2, double *__restrict__ tp, double *__restrict__ tm,
-                                 int64_t no, int64_t nv, int64_t ldp, int64_t ldm) {
-    const int64_t nop = no * (no + 1) / 2, nvp = nv * (nv + 1) / 2;
-    GRID_STRIDE(idx, nop * nvp) {
-        int64_t ij = idx % nop, cd = idx / nop, i, j, c, d;
-        untri(ij, i, j);
-        untri(cd, c, d);
-        double a = t2[pk(c + nv * i, d + nv * j)];
-        double b = t2[pk(c + nv * j, d + nv * i)];
-        double f = (c == d ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
-        tp[ij + ldp * cd] = f * (a + b);
-        if (i > j && c > d) {
-            int64_t ijm = i * (i - 1) / 2 + j, cdm = c * (c - 1) / 2 + d;
-            tm[ijm + ldm * cdm] = a - b;
-        }
-    }
-}
-
 // G[(c + nv*(a-a0)) + ldg*(d + nv*b)] = g_acbd for a in [a0,a1), b in [0,a1)
 __global__ void form_gpm_kernel(const double *__restrict__ G, int64_t ldg, double *__restrict__ gp,
                                 double *__restrict__ gm, int64_t nv, int64_t a0, int64_t a1) {
@@ -79,36 +61,6 @@ __device__ __forceinline__ void put_planes(double x, int np, size_t plane, __nv_
         const __nv_bfloat16 h = __double2bfloat16(x);
         out[q * plane] = h;
         x -= (double)__bfloat162float(h);
-    }
-}
-
-// t+ (plus) or t- rows of the +/- tensor-core ladder as np bf16 planes [np][rows_pad][kpad]: row
-// vec n_rows + ij (vector vec, ij over i >= j for t+, i > j for t-), column cd over c >= d (t+) or
-// c > d (t-), the values of build_tpm
-__global__ void build_tpm_planes_kernel(const double *__restrict__ t2s, int64_t nvec, int64_t no, int64_t nv,
-                                        int64_t rows_pad, int64_t kpad, int np, int plus,
-                                        __nv_bfloat16 *__restrict__ out) {
-    const int64_t nrow = plus ? no * (no + 1) / 2 : no * (no - 1) / 2;
-    const int64_t ncol = plus ? nv * (nv + 1) / 2 : nv * (nv - 1) / 2;
-    const int64_t nt2 = nv * no * (nv * no + 1) / 2;
-    const size_t plane = (size_t)rows_pad * kpad;
-    GRID_STRIDE(idx, rows_pad * kpad) {
-        const int64_t rr = idx / kpad, k = idx - rr * kpad;
-        const int64_t vec = nrow > 0 ? rr / nrow : nvec, row = nrow > 0 ? rr - vec * nrow : 0;
-        double val = 0.0;
-        if (vec < nvec && k < ncol) {
-            int64_t i, j, c, d;
-            untri(row, i, j);
-            untri(k, c, d);
-            if (!plus) {   // strict triangles: M(M-1)/2 + m maps to (M-1, m)
-                i += 1;
-                c += 1;
-            }
-            const double *t2 = t2s + vec * nt2;
-            const double x = t2[pk(c + nv * i, d + nv * j)], y = t2[pk(c + nv * j, d + nv * i)];
-            val = plus ? (c == d ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0) * (x + y) : x - y;
-        }
-        put_planes(val, np, plane, out + idx);
     }
 }
 
@@ -148,34 +100,6 @@ __global__ void form_pm_planes_kernel(const double *__restrict__ G, int64_t ldg,
             }
         }
         __syncthreads();
-    }
-}
-
-__global__ void add_omega_pm_kernel(double *__restrict__ om2, const double *__restrict__ wp,
-                                    const double *__restrict__ wm, int64_t no, int64_t nv, int64_t a0, int64_t a1,
-                                    int64_t ldwp, int64_t ldwm) {
-    const int64_t nop = no * (no + 1) / 2;
-    const int64_t abp0 = a0 * (a0 + 1) / 2, nabp = a1 * (a1 + 1) / 2 - abp0;
-    const int64_t abm0 = a0 * (a0 - 1) / 2;
-    GRID_STRIDE(idx, nop * nabp) {
-        int64_t ij = idx % nop, loc = idx / nop, i, j, a, b;
-        untri(ij, i, j);
-        untri(abp0 + loc, a, b);
-        double p = wp[ij + ldwp * loc] * (a == b ? 0.5 : 1.0);
-        double x1 = p, x2 = p;
-        if (i != j && a != b) {
-            int64_t ijm = i * (i - 1) / 2 + j, locm = a * (a - 1) / 2 + b - abm0;
-            double m = wm[ijm + ldwm * locm];
-            x1 = p + m;
-            x2 = p - m;
-        }
-        int64_t P1 = pk(a + nv * i, b + nv * j), P2 = pk(a + nv * j, b + nv * i);
-        if (P1 == P2) {
-            om2[P1] += x1 + x2;
-        } else {
-            om2[P1] += x1;
-            om2[P2] += x2;
-        }
     }
 }
 
@@ -457,32 +381,9 @@ __global__ void diis_solve_kernel(double *__restrict__ Gslot, int maxdim, const 
 
 }  // namespace
 
-void build_tpm(Exec &ex, const double *t2, double *tp, double *tm, int64_t no, int64_t nv, int64_t ldp, int64_t ldm) {
-    int64_t total = (no * (no + 1) / 2) * (nv * (nv + 1) / 2);
-    build_tpm_kernel<<<grid_for(total, 256), 256, 0, ex.stream>>>(t2, tp, tm, no, nv, ldp, ldm);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
-}
-
 void form_gpm(Exec &ex, const double *G, int64_t ldg, double *gp, double *gm, int64_t nv, int64_t a0, int64_t a1) {
     int64_t total = (nv * (nv + 1) / 2) * (a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2);
     form_gpm_kernel<<<grid_for(total, 256), 256, 0, ex.stream>>>(G, ldg, gp, gm, nv, a0, a1);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
-}
-
-void add_omega_pm(Exec &ex, double *om2, const double *wp, const double *wm, int64_t no, int64_t nv, int64_t a0,
-                  int64_t a1, int64_t ldwp, int64_t ldwm) {
-    int64_t total = (no * (no + 1) / 2) * (a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2);
-    add_omega_pm_kernel<<<grid_for(total, 256), 256, 0, ex.stream>>>(om2, wp, wm, no, nv, a0, a1, ldwp, ldwm);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
-}
-
-void build_tpm_planes(Exec &ex, const double *t2s, int64_t nvec, int64_t no, int64_t nv, bool plus, int64_t rows_pad,
-                      int64_t kpad, int np, __nv_bfloat16 *out) {
-    build_tpm_planes_kernel<<<grid_for(rows_pad * kpad, 256), 256, 0, ex.stream>>>(t2s, nvec, no, nv, rows_pad, kpad,
-                                                                                  np, plus ? 1 : 0, out);
     ex.launches++;
     CU_CHECK(cudaGetLastError());
 }

@@ -59,9 +59,9 @@ struct Mode {
     static constexpr int STAGE_BYTES = NP * (A_TILE + B_TILE);
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 4 * BN * 8 /*column offsets*/;
     static constexpr uint32_t TMEM_COLS = 2 * BN;    // two FP32 accumulators of 128 lanes x BN columns
-    // kind::f16 instruction descriptor: BF16 x BF16 -> F32, both K-major, M = 128, N = BN
-    static constexpr uint32_t IDESC =
-        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    static constexpr int N_STEP = 16;                // N tiles are multiples of this, up to BN
+    // kind::f16 instruction descriptor: BF16 x BF16 -> F32, both K-major, M = 128; N is the launch's tile
+    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);
     // plane pair (A plane, B plane) of product p, largest products first
     __host__ __device__ static constexpr int pa(int p) { return p == 2 || p == 4 ? 1 : (p == 5 ? 2 : 0); }
     __host__ __device__ static constexpr int pb(int p) { return p == 1 || p == 4 ? 1 : (p == 3 ? 2 : 0); }
@@ -263,6 +263,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     if (warp == 0) {
         if (lane == 0) {
             // TMA producer: one ring of stages across all tiles of this CTA
+            const uint32_t stage_bytes = (uint32_t)(NP * (A_TILE + map.bn * KB * 2));
             int g = 0;
             int issued[STAGES] = {};   // loads issued per stage (at most the last one is in flight)
             for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
@@ -278,7 +279,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                     if (map.stall_test && g == 0) continue;   // stage 0's first phase never completes
                     issued[s]++;
                     uint8_t *st = smem + s * STAGE_BYTES;
-                    mbar_expect_tx(&full[s], STAGE_BYTES);
+                    mbar_expect_tx(&full[s], stage_bytes);
                     const int k0 = (kt0 + i) * KB;
 #pragma unroll
                     for (int p = 0; p < NP; p++) {
@@ -297,6 +298,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     } else if (warp == 1) {
         if (lane == 0) {
             // MMA issuer
+            const uint32_t idesc = MD::IDESC | ((uint32_t)(map.bn >> 3) << 17);
             // one accumulation unit = one K chunk of one tile; units alternate between the two
             // TMEM accumulators
             int g = 0, tc = 0;
@@ -329,7 +331,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                         for (int p = 0; p < MD::NPROD; p++) {
                             const uint8_t *ta = st + MD::pa(p) * A_TILE;
                             const uint8_t *tb = st + NP * A_TILE + MD::pb(p) * B_TILE;
-                            mma_bf16(d, smem_desc_k<MD::ROW_BYTES>(ta, ko), smem_desc_k<MD::ROW_BYTES>(tb, ko), MD::IDESC,
+                            mma_bf16(d, smem_desc_k<MD::ROW_BYTES>(ta, ko), smem_desc_k<MD::ROW_BYTES>(tb, ko), idesc,
                                      (i > c0 || kk > 0 || p > 0) ? 1u : 0u);
                         }
                     }
@@ -351,7 +353,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             map.decode(t, m0, n0, z, kt0, nk);
             if constexpr (Epi::kTable) {
                 __syncwarp();
-                for (int c = lane; c < BN; c += 32) coff[c] = n0 + c < epi.N ? epi.col_offset(n0 + c) : 0;
+                for (int c = lane; c < map.bn; c += 32) coff[c] = n0 + c < epi.N ? epi.col_offset(n0 + c) : 0;
                 __syncwarp();
             }
             for (int c0 = 0; c0 < nk; c0 += map.kc, tc++) {
@@ -370,7 +372,7 @@ split_bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             epi.row_setup(row);
             const uint32_t base = tmem + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int cc = 0; cc < BN; cc += 16) {
+            for (int cc = 0; cc < map.bn; cc += 16) {
                 float v[16];
                 tmem_ld16(base + (uint32_t)cc, v);
                 epi.apply16(row, n0 + cc, v, c0 == 0, coff + cc);
@@ -405,8 +407,8 @@ struct PairMode {
     static constexpr int STAGE_BYTES = NP * (A_TILE + B_TILE);
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 4 * BN * 8;
     static constexpr uint32_t TMEM_COLS = 2 * BN;
-    static constexpr uint32_t IDESC =
-        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+    static constexpr int N_STEP = 32;
+    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 4) << 24);
 };
 static_assert(PairMode::STAGE_BYTES == 64 * 1024, "pair stage size");
 
@@ -470,6 +472,7 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     if (warp == 0) {
         if (lane == 0) {
             // TMA producer of this CTA: its A rows and its half of B; CTA 0 expects both CTAs' bytes
+            const uint32_t stage_bytes = (uint32_t)(MD::NP * (A_TILE + map.bn / 2 * KB * 2));
             int g = 0;
             int issued[STAGES] = {};
             for (int t = pair; t < num_tiles && !*abort_flag; t += npairs) {
@@ -485,13 +488,13 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                     if (map.stall_test && g == 0) continue;   // stage 0's first phase never completes
                     issued[s]++;
                     uint8_t *st = smem + s * STAGE_BYTES;
-                    if (lead) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                    if (lead) mbar_expect_tx(&full[s], 2 * stage_bytes);
                     const int k0 = (kt0 + i) * KB;
 #pragma unroll
                     for (int p = 0; p < MD::NP; p++) {
                         tma_load_3d_pair(&tmA, &full[s], st + p * A_TILE, k0, m0 + BM * (int)rank, p);
-                        tma_load_3d_pair(&tmB, &full[s], st + MD::NP * A_TILE + p * B_TILE, k0, n0 + (BN / 2) * (int)rank,
-                                         p);
+                        tma_load_3d_pair(&tmB, &full[s], st + MD::NP * A_TILE + p * B_TILE, k0,
+                                         n0 + (map.bn / 2) * (int)rank, p);
                     }
                 }
             }
@@ -505,6 +508,7 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     } else if (warp == 1) {
         if (lane == 0 && lead) {
             // MMA issuer of the pair
+            const uint32_t idesc = MD::IDESC | ((uint32_t)(map.bn >> 3) << 17);
             int g = 0, tc = 0;
             for (int t = pair; t < num_tiles && !*abort_flag; t += npairs) {
                 int m0, n0, z, kt0, nk;
@@ -536,7 +540,7 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                                 // hi*hi, hi*lo, lo*hi
                                 const uint8_t *ta = st + (p == 2 ? 1 : 0) * A_TILE;
                                 const uint8_t *tb = st + MD::NP * A_TILE + (p == 1 ? 1 : 0) * B_TILE;
-                                mma_bf16_pair(d, smem_desc_k<128>(ta, ko), smem_desc_k<128>(tb, ko), MD::IDESC,
+                                mma_bf16_pair(d, smem_desc_k<128>(ta, ko), smem_desc_k<128>(tb, ko), idesc,
                                               (i > c0 || kk > 0 || p > 0) ? 1u : 0u);
                             }
                         }
@@ -558,7 +562,7 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             map.decode(t, m0, n0, z, kt0, nk);
             if constexpr (Epi::kTable) {
                 __syncwarp();
-                for (int c = lane; c < BN; c += 32) coff[c] = n0 + c < epi.N ? epi.col_offset(n0 + c) : 0;
+                for (int c = lane; c < map.bn; c += 32) coff[c] = n0 + c < epi.N ? epi.col_offset(n0 + c) : 0;
                 __syncwarp();
             }
             for (int c0 = 0; c0 < nk; c0 += map.kc, tc++) {
@@ -577,7 +581,7 @@ split_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                 epi.row_setup(row);
                 const uint32_t base = tmem + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-                for (int cc = 0; cc < BN; cc += 16) {
+                for (int cc = 0; cc < map.bn; cc += 16) {
                     float v[16];
                     tmem_ld16(base + (uint32_t)cc, v);
                     epi.apply16(row, n0 + cc, v, c0 == 0, coff + cc);
@@ -726,24 +730,64 @@ int sm_count() {
     return v;
 }
 
+// Time of one K block of a tile with an N tile of bn, in SM cycles: the tensor cores take bn / 2 cycles per
+// MMA of a 16-wide slice, and the stage arrives from L2 at about 64 bytes a cycle.
+template <class MD>
+double kblock_cycles(int bn) {
+    constexpr bool pair = std::is_same<MD, PairMode>::value;
+    const double mma = (MD::NP == 2 ? 3 : 6) * (MD::KB / 16) * bn / 2.0;
+    const double fill = MD::NP * (BM + (pair ? bn / 2 : bn)) * MD::KB * 2 / 64.0;
+    return std::max(mma, fill);
+}
+
+// Time of the whole product on the persistent grid, in K-block cycles of one slice
+template <class MD>
+double tiles_cycles(int64_t mt, int64_t n, int64_t splits, int bn) {
+    constexpr bool pair = std::is_same<MD, PairMode>::value;
+    const int64_t slots = pair ? sm_count() / 2 : sm_count();
+    const int64_t units = mt * ((n + bn - 1) / bn) * splits;
+    return double((units + slots - 1) / slots) * kblock_cycles<MD>(bn) / double(splits);
+}
+
+// N tile of a product with mt row tiles: of the equal cuts of n into tiles of at most BN the one whose
+// waves over the SMs cost least, the widest of equals.  Full 256-wide tiles left 35 % of the columns of a
+// 169-column product empty, and a few-column product ran on as many CTAs as it had row tiles: one mixed
+// residual at o=13, v=107 (91 and 78 columns of the ladder) 1.76 ms with them, 1.55 with its own widths.
+template <class MD>
+int n_tile_for(int64_t mt, int64_t n, int64_t splits) {
+    int best = MD::BN;
+    double best_cost = tiles_cycles<MD>(mt, n, splits, best);
+    for (int64_t nt = (n + MD::BN - 1) / MD::BN; nt <= (n + MD::BN - 1) / MD::BN + 2; nt++) {
+        const int bn = (int)std::min<int64_t>(MD::BN, round_up((n + nt - 1) / nt, MD::N_STEP));
+        const double c = tiles_cycles<MD>(mt, n, splits, bn);
+        if (c < best_cost * 0.999) {
+            best = bn;
+            best_cost = c;
+        }
+    }
+    return best;
+}
+
 // A: a_rows rows of NP planes with stride a_plane; B likewise; the grid covers m_out x n_out output
 // elements (rounded up to the tile); mnk = m * n * k of the product for the FLOP count.
 template <class MD, class Epi>
 void launch_mode(Exec &ex, const __nv_bfloat16 *A, int64_t a_rows, int64_t a_plane, int64_t m_out,
                  const __nv_bfloat16 *B, int64_t b_rows, int64_t b_plane, int64_t n_out, int64_t Kp, const Epi &epi,
                  double mnk, int splits) {
-    const int64_t Mp = round_up(m_out, BM), Np = round_up(n_out, MD::BN);
+    const int64_t Mp = round_up(m_out, BM);
+    const int bn = n_tile_for<MD>(Mp / BM, n_out, splits);
+    const int64_t Np = round_up(n_out, bn);
     REQUIRE(Kp % BK == 0 && Kp > 0 && Mp > 0 && Np > 0, CCSD_GPU_EINVAL, "tc gemm: bad padding");
     CU_CHECK(cudaFuncSetAttribute(split_bf16_gemm_kernel<MD, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   MD::SMEM_BYTES));
     CUtensorMap ta = make_map(const_cast<__nv_bfloat16 *>(A), a_rows, Kp, BM, a_plane, MD::NP, MD::KB);
-    CUtensorMap tb = make_map(const_cast<__nv_bfloat16 *>(B), b_rows, Kp, MD::BN, b_plane, MD::NP, MD::KB);
+    CUtensorMap tb = make_map(const_cast<__nv_bfloat16 *>(B), b_rows, Kp, bn, b_plane, MD::NP, MD::KB);
     TileMap map;
     map.num_mt = (int)(Mp / BM);
-    map.num_nt = (int)(Np / MD::BN);
+    map.num_nt = (int)(Np / bn);
     map.nk_all = (int)(Kp / MD::KB);
     map.nks = (map.nk_all + splits - 1) / splits;
-    map.bn = MD::BN;
+    map.bn = bn;
     map.group_m = std::min(map.num_mt, 16);
     map.kc = (Epi::kChunked && ex.k_chunk > 0) ? (int)std::max<int64_t>(1, ex.k_chunk / MD::KB) : map.nks;
     REQUIRE(ex.gemm_err != nullptr, CCSD_GPU_EINVAL, "tc gemm: no error word");
@@ -774,20 +818,22 @@ void launch_pair(Exec &ex, const __nv_bfloat16 *A, int64_t a_rows, int64_t a_pla
                  const __nv_bfloat16 *B, int64_t b_rows, int64_t b_plane, int64_t n_out, int64_t Kp, const Epi &epi,
                  double mnk, int splits) {
     using MD = PairMode;
-    const int64_t Mp = round_up(m_out, 2 * BM), Np = round_up(n_out, MD::BN);
+    const int64_t Mp = round_up(m_out, 2 * BM);
+    const int bn = n_tile_for<MD>(Mp / (2 * BM), n_out, splits);
+    const int64_t Np = round_up(n_out, bn);
     REQUIRE(Kp % BK == 0 && Kp > 0 && Mp > 0 && Np > 0, CCSD_GPU_EINVAL, "tc gemm: bad padding");
     auto kernel = split_bf16_pair_kernel<Epi>;
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MD::SMEM_BYTES));
     // rows beyond a buffer's own rows (the second CTA of the last pair tile) read as zero
     CUtensorMap ta = make_map(const_cast<__nv_bfloat16 *>(A), a_rows, Kp, BM, a_plane, MD::NP, MD::KB);
-    CUtensorMap tb = make_map(const_cast<__nv_bfloat16 *>(B), b_rows, Kp, MD::BN / 2, b_plane, MD::NP, MD::KB);
+    CUtensorMap tb = make_map(const_cast<__nv_bfloat16 *>(B), b_rows, Kp, bn / 2, b_plane, MD::NP, MD::KB);
     TileMap map;
     map.bm = 2 * BM;
     map.num_mt = (int)(Mp / (2 * BM));
-    map.num_nt = (int)(Np / MD::BN);
+    map.num_nt = (int)(Np / bn);
     map.nk_all = (int)(Kp / MD::KB);
     map.nks = (map.nk_all + splits - 1) / splits;
-    map.bn = MD::BN;
+    map.bn = bn;
     map.group_m = std::min(map.num_mt, 8);
     map.kc = (Epi::kChunked && ex.k_chunk > 0) ? (int)std::max<int64_t>(1, ex.k_chunk / MD::KB) : map.nks;
     REQUIRE(ex.gemm_err != nullptr, CCSD_GPU_EINVAL, "tc gemm: no error word");
@@ -850,7 +896,7 @@ void launch_tc(Exec &ex, int planes, const __nv_bfloat16 *A, int64_t a_rows, int
                const __nv_bfloat16 *B, int64_t b_rows, int64_t b_plane, int64_t n_out, int64_t Kp, const Epi &epi,
                double mnk, int splits = 1, bool pair = false) {
     if constexpr (Epi::kChunked) {
-        if (planes == 2 && m_out >= 2 * BM && (pair || pair_gemm_on())) {
+        if (planes == 2 && (pair || (m_out >= 2 * BM && pair_gemm_on()))) {
             launch_pair(ex, A, a_rows, a_plane, m_out, B, b_rows, b_plane, n_out, Kp, epi, mnk, splits);
             return;
         }
@@ -988,6 +1034,31 @@ int tc_default_splits(int64_t m, int64_t n, int64_t k, int planes) {
     return (int)((nkt + per - 1) / per);
 }
 
+int tc_tall_route(int64_t m, int64_t n, int64_t kp, int planes) {
+    const int64_t nkt = kp / BK, mt = (m + BM - 1) / BM, pt = (m + 2 * BM - 1) / (2 * BM);
+    int best = 1;
+    double best_cost = 1e300;
+    // every further split writes and sums another m x n partial product; at least 8 K blocks per slice
+    const double per_split = 16.0 * double(m) * double(n) / (double(sm_count()) * 24.0) / double(std::max<int64_t>(nkt, 1));
+    for (int s = 1; s <= 8 && (s == 1 || nkt / s >= 8); s++) {
+        if (used_splits(s, nkt) != s) continue;
+        const double extra = s > 1 ? per_split * s : 0.0;
+        const double c = extra + (planes == 3 ? tiles_cycles<ModeX6>(mt, n, s, n_tile_for<ModeX6>(mt, n, s))
+                                              : tiles_cycles<ModeX3>(mt, n, s, n_tile_for<ModeX3>(mt, n, s)));
+        if (c < best_cost * 0.98) {
+            best = s;
+            best_cost = c;
+        }
+        if (planes != 2 || m < 2 * BM) continue;
+        const double cp = extra + tiles_cycles<PairMode>(pt, n, s, n_tile_for<PairMode>(pt, n, s));
+        if (cp < best_cost * 0.98) {
+            best = PAIR_ROUTE + s;
+            best_cost = cp;
+        }
+    }
+    return best;
+}
+
 std::vector<int> tc_split_candidates(int64_t m, int64_t n, int64_t k, int planes) {
     const int64_t tiles = (round_up(m, BM) / BM) * (round_up(n, n_tile(planes)) / n_tile(planes));
     const int64_t nkt = round_up(k, BK) / BK, nsm = sm_count();
@@ -1088,7 +1159,7 @@ void split_rows(Exec &ex, const double *src, int64_t sr, int64_t sk, int64_t R, 
 void tc_gemm_f64(Exec &ex, const __nv_bfloat16 *A, int64_t Mp, const __nv_bfloat16 *B, int64_t Np, int64_t Kp,
                  int64_t m, int64_t n, int64_t k_true, double alpha, double beta, double *C, int64_t ldc,
                  int splits) {
-    REQUIRE(Mp >= round_up(m, BM) && Np >= round_up(n, B_ROW_PAD), CCSD_GPU_EINVAL, "tc_gemm_f64: bad padding");
+    REQUIRE(Mp >= m && Np >= n, CCSD_GPU_EINVAL, "tc_gemm_f64: bad padding");   // rows past a plane read as zero
     const int np = check_planes(ex.planes);
     const double mnk = double(m) * double(n) * double(k_true);
     const bool pair = splits >= PAIR_ROUTE;

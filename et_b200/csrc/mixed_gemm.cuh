@@ -58,6 +58,10 @@ constexpr int PAIR_ROUTE = 100;
 
 // K-split count of the fixed rule: split only when the output tiles cannot fill the SMs.
 int tc_default_splits(int64_t m, int64_t n, int64_t k, int planes);
+// Route of a product with many rows and few columns on pre-split operands (the A2 ladder's, whose rows may
+// come in blocks): the K-split count that lets the tiles of all m rows fill the SMs best, by the same cost
+// model as the N tile.
+int tc_tall_route(int64_t m, int64_t n, int64_t kp, int planes);
 // K-split counts worth timing for an m x n x k product: 1, the fixed rule's count, and counts whose
 // tile units fill whole waves of the persistent grid; for products of at least 256 rows the same
 // counts again as CTA-pair routes.
