@@ -112,7 +112,7 @@ Context::~Context() {
     if (ex.stream) cudaStreamSynchronize(ex.stream);
     if (graphs_captured) cudaDeviceGraphMemTrim(device);   // the physical memory the residual graphs held
     for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig, &f64_ovvv_dig}) p->buf.release();
-    for (DBuf *b : {&gov, &hov, &L_oo, &L_ov, &L_vo, &L_vv, &Lt_oo, &Lt_ov, &Lt_vo, &Lt_vv, &h, &eps, &F, &t, &epsdiff, &scal,
+    for (DBuf *b : {&gov, &hov, &gex, &L_oo, &L_ov, &L_vo, &L_vv, &Lt_oo, &Lt_ov, &Lt_vo, &Lt_vv, &h, &eps, &F, &t, &epsdiff, &scal,
                     &mbuf, &ybuf, &om_stage, &f64_gp, &f64_gm, &f64_ovvv, &hb_oo, &hb_ov, &hb_vo, &hb_vv,
                     &gemm_err, &digit_arena, &fb_oo, &fb_ov, &fb_vo, &fb_vv})
         b->release();
@@ -267,21 +267,37 @@ const double *Context::g_ovov_const() {
     return gov.d();
 }
 
-// H_lckd = g_lckd - 1/2 g_kcld, the combination of g_ovov that the two u terms of omega_ccsd_d2
-// contract with (one product instead of two), kept beside g_ovov
-const double *Context::h_ovov_const() {
+// The two forms of g_ovov that C2 and D2 contract with, in the pair layout (v,o,v,o) of the amplitudes, so
+// that their products are matrix products as they lie: the exchanged integrals gex[c,l,d,k] = g_kcld, and
+// H_lckd = g_lckd - 1/2 g_kcld of the two u terms of omega_ccsd_d2 (one product instead of two), which also
+// serves the integrals of omega_ccsd_e2 (u g = t (2 g - g^x)).  Read from (o,v,o,v), the operands of these
+// products were gathered across their unit stride: one residual at o=24, v=192 with its energy 13.2 ms so,
+// 12.4 with the two forms and Y0 and Q below in one product; with six digits at o=20, v=200 28.2 and 23.0 ms.
+void Context::g_pairs_const() {
     const double *g = g_ovov_const();
-    if (!hov || hov_id != gov_id) {
-        if (!hov) hov = dalloc(nov * nov, ex.stream);
-        const TV H = tv(hov.d(), {no, nv, no, nv});
-        permute_add(ex, 1.0, tv(g, {no, nv, no, nv}), 0.0, H);
-        TV gt = tv(g, {no, nv, no, nv});   // gt[l, c, k, d] = g[k, c, l, d]
-        std::swap(gt.s[0], gt.s[2]);
-        permute_add(ex, -0.5, gt, 1.0, H);
-        hov_id = gov_id;
-        cache_epoch++;
+    if (hov && gov_pairs_id == gov_id) return;
+    if (!hov) {
+        hov = dalloc(nov * nov, ex.stream);
+        gex = dalloc(nov * nov, ex.stream);
     }
-    return hov.d();
+    TV lckd = tv(g, {no, nv, no, nv});   // as [c, l, d, k] = g[l, c, k, d]
+    lckd.n[0] = lckd.n[2] = nv;
+    lckd.n[1] = lckd.n[3] = no;
+    TV kcld = lckd;                      // as [c, l, d, k] = g[k, c, l, d]
+    lckd.s[0] = no;
+    lckd.s[1] = 1;
+    lckd.s[2] = nov * no;
+    lckd.s[3] = nov;
+    kcld.s[0] = no;
+    kcld.s[1] = nov;
+    kcld.s[2] = nov * no;
+    kcld.s[3] = 1;
+    const TV H = tv(hov.d(), {nv, no, nv, no}), X = tv(gex.d(), {nv, no, nv, no});
+    permute_add(ex, 1.0, kcld, 0.0, X);
+    permute_add(ex, 1.0, lckd, 0.0, H);
+    permute_add(ex, -0.5, X, 1.0, H);
+    gov_pairs_id = gov_id;
+    cache_epoch++;
 }
 
 // calculate_energy_ccsd (src/wavefunctions/ccsd/mean_value_ccsd.F90:36-99), FP64
@@ -592,13 +608,13 @@ void Context::ladder_tc_streamed(const double *Lvv, const double *t2, double *om
     }
 }
 
-// Mixed precision keeps the ovvv integrals of the untransformed Cholesky vectors resident as split
-// bf16, ybuf[plane][k + no*b][c + nv*d] = g_kcbd (o v^3 elements per plane: 4.2 GB for both planes
-// at o = 32, v = 320), formed once per Cholesky set by one tensor-core GEMM whose epilogue writes
-// the planes.  The ladder's Y intermediates then cost one GEMM of o^2 x o v x v^2 per call instead
-// of re-forming g_kcbd in batches (and permuting and splitting it) every time.
+// Mixed precision keeps the ovvv and ovov integrals of the untransformed Cholesky vectors resident as split
+// bf16, ybuf[plane][k + no*p][c + nv*d] = g_kcpd with p over the virtual and then the occupied orbitals
+// (o (o + v) v^2 elements per plane: 4.6 GB for both planes at o = 32, v = 320), formed once per Cholesky set
+// by one tensor-core GEMM whose epilogue writes the planes.  The ladder's Y0 and the Q of its corrections
+// and of omega_ccsd_b2 then cost one GEMM of o^2 x o (o + v) x v^2 per call.
 bool Context::ovvv_resident() {
-    const size_t need = sizeof(__nv_bfloat16) * (size_t)ex.planes * (size_t)tc_pad_rows_a(nov) * tc_pad_k(nv * nv);
+    const size_t need = sizeof(__nv_bfloat16) * (size_t)ex.planes * (size_t)tc_pad_rows_a(no * nmo) * tc_pad_k(nv * nv);
     if (ybuf_bytes >= need) return true;
     if (ybuf_fit < 0 || ybuf_fit_version != l_version || ybuf_fit_planes != ex.planes) {
         size_t free_b = 0, total_b = 0;
@@ -626,18 +642,21 @@ void Context::ovvv_pairs() {
         permute_add(ex, 1.0, tv(L_ov.d(), {nJ, no, nv}), 0.0, dst);
         split_rows(ex, LO.d(), nJ, 1, nov, nJ, o_rows, Jp, LOS.as<__nv_bfloat16>());
     }
-    // L_vv split rows d + nv*b: L_vv[J, b, d] sits at J + nJ*(b + nv*d); copy to (J, d, b)
-    const int64_t v_rows = tc_pad_rows_b(nv2);
+    // rows d + nv*p of L_vv and then of L_ov: L[J, p, d] copied to (J, d, p)
+    const int64_t v_rows = tc_pad_rows_b(nv * nmo);
     DBuf LVS(sizeof(__nv_bfloat16) * np * v_rows * Jp, s);
     {
-        DBuf LV = dalloc(nJ * nv2, s);
+        DBuf LV = dalloc(nJ * nv * nmo, s);
         TV dst = tv(LV.d(), {nJ, nv, nv});   // [J, b, d] at J + nJ*(d + nv*b)
         dst.s[1] = nJ * nv;
         dst.s[2] = nJ;
         permute_add(ex, 1.0, tv(L_vv.d(), {nJ, nv, nv}), 0.0, dst);
-        split_rows(ex, LV.d(), nJ, 1, nv2, nJ, v_rows, Jp, LVS.as<__nv_bfloat16>());
+        dst.p += nJ * nv2;
+        dst.n[1] = no;                       // [J, l, d] behind it
+        permute_add(ex, 1.0, tv(L_ov.d(), {nJ, no, nv}), 0.0, dst);
+        split_rows(ex, LV.d(), nJ, 1, nv * nmo, nJ, v_rows, Jp, LVS.as<__nv_bfloat16>());
     }
-    const int64_t yrows = tc_pad_rows_a(nov);
+    const int64_t yrows = tc_pad_rows_a(no * nmo);
     const size_t need = sizeof(__nv_bfloat16) * (size_t)np * (size_t)yrows * Kq;
     if (ybuf_bytes < need) {
         ybuf = DBuf();
@@ -653,49 +672,20 @@ void Context::ovvv_pairs() {
     cache_epoch++;
 }
 
-void Context::ladder_y0(const double *tf, double *Y) {
-    ovvv_pairs();
-    cudaStream_t s = ex.stream;
-    const int64_t nv2 = nv * nv, oo = no * no, Kq = tc_pad_k(nv2), yrows = tc_pad_rows_a(nov);
-    const int64_t rows_T = tc_pad_rows_b(oo);
-    DBuf TS(sizeof(__nv_bfloat16) * ex.planes * rows_T * Kq, s);
-    {
-        // tau split rows i + no*j, K position c + nv*d: copy tau[c, i, d, j] to (c, d, i, j)
-        DBuf TT = dalloc(oo * nv2, s);
-        TV dst = tv(TT.d(), {nv, no, nv, no});
-        dst.s[1] = nv2;        // i
-        dst.s[2] = nv;         // d
-        dst.s[3] = nv2 * no;   // j
-        permute_add(ex, 1.0, tv(tf, {nv, no, nv, no}), 0.0, dst);
-        split_rows(ex, TT.d(), nv2, 1, oo, nv2, rows_T, Kq, TS.as<__nv_bfloat16>());
-    }
-    // Yt[(k + no*b) + nov*(i + no*j)], then Y[k, i, b, j]
-    DBuf Yt = dalloc(nov * oo, s);
-    tc_gemm_f64_tuned(ex, ybuf.as<__nv_bfloat16>(), yrows, TS.as<__nv_bfloat16>(), rows_T, Kq, nov, oo, nv2, 1.0, 0.0,
-                      Yt.d(), nov, 0);
-    TV src = tv(Yt.d(), {no, no, nv, no});   // (k, i, b, j)
-    src.s[1] = nov;
-    src.s[2] = no;
-    src.s[3] = nov * no;
-    permute_add(ex, 1.0, src, 0.0, tv(Y, {no, no, nv, no}));
-}
-
-void Context::ladder_y_t1(const double *t1, const double *Ltvv, const double *tf, double *Y) {
-    if (ex.prec == Prec::MIXED && ovvv_resident()) {
-        ladder_y0(tf, Y);
-    } else if (ex.prec != Prec::MIXED && f64_resident()) {
-        f64_integrals();
-        contract(ex, "kbcd,cidj->kibj", 1.0, tv(f64_ovvv.d(), {no, nv, nv, nv}), tv(tf, {nv, no, nv, no}), 0.0,
-                 tv(Y, {no, no, nv, no}));
-    } else {
-        ladder_y(Ltvv, tf, Y);
-        return;
+void Context::ladder_y_t1(const double *t1, const double *Ltvv, const double *tf, const LadderY &yq, double *Y) {
+    LadderY own;
+    const LadderY *src = &yq;
+    if (!yq.Y) {
+        if (!(ex.prec == Prec::MIXED ? ovvv_resident() : f64_resident())) {
+            ladder_y(Ltvv, tf, Y);
+            return;
+        }
+        own = ladder_y_plain(tf);
+        src = &own;
     }
     // L~_bd = L_bd - sum_l t_bl L_ld, so g_kc~bd = g_kcbd - sum_l t_bl g_kcld
-    DBuf Q = dalloc(no * no * no * no, ex.stream);
-    contract(ex, "kcld,cidj->kilj", 1.0, tv(g_ovov_const(), {no, nv, no, nv}), tv(tf, {nv, no, nv, no}), 0.0,
-             tv(Q.d(), {no, no, no, no}));
-    contract(ex, "bl,kilj->kibj", -1.0, tv(t1, {nv, no}), tv(Q.d(), {no, no, no, no}), 1.0,
+    CU_CHECK(cudaMemcpyAsync(Y, src->Y.d(), src->Y.bytes(), cudaMemcpyDeviceToDevice, ex.stream));
+    contract(ex, "bl,kilj->kibj", -1.0, tv(t1, {nv, no}), tv(src->Q.d(), {no, no, no, no}), 1.0,
              tv(Y, {no, no, nv, no}));
 }
 
@@ -708,16 +698,11 @@ void Context::ladder_y_t1(const double *t1, const double *Ltvv, const double *tf
 // (the A^T term uses sum_cd g_acld t_cidj = Y_ljai), all with untransformed integrals: the v^4
 // integrals are formed once per Cholesky set instead of every iteration, the corrections cost
 // o^2 v^3 N_J + o^3 v^3.  om is packed as om + om^T, so the corrections enter it as -A + T4/2.
-void Context::ladder_t1_corrections(const double *t1, const double *tf, double *om) {
-    cudaStream_t s = ex.stream;
-    DBuf Y0 = dalloc(no * no * nv * no, s);
-    ladder_y_plain(tf, Y0.d());
-    contract(ex, "ak,kibj->aibj", -1.0, tv(t1, {nv, no}), tv(Y0.d(), {no, no, nv, no}), 1.0,
+void Context::ladder_t1_corrections(const double *t1, const LadderY &yq, double *om) {
+    contract(ex, "ak,kibj->aibj", -1.0, tv(t1, {nv, no}), tv(yq.Y.d(), {no, no, nv, no}), 1.0,
              tv(om, {nv, no, nv, no}));
-    DBuf Q = dalloc(no * no * no * no, s), B = dalloc(nv * no * no * no, s);
-    contract(ex, "kcld,cidj->kilj", 1.0, tv(g_ovov_const(), {no, nv, no, nv}), tv(tf, {nv, no, nv, no}), 0.0,
-             tv(Q.d(), {no, no, no, no}));
-    contract(ex, "ak,kilj->ailj", 1.0, tv(t1, {nv, no}), tv(Q.d(), {no, no, no, no}), 0.0,
+    DBuf B = dalloc(nv * no * no * no, ex.stream);
+    contract(ex, "ak,kilj->ailj", 1.0, tv(t1, {nv, no}), tv(yq.Q.d(), {no, no, no, no}), 0.0,
              tv(B.d(), {nv, no, no, no}));
     // the symmetric term sum_l t_bl B_ailj enters at half weight, in its mirrored form sum_l t_al B_bjli,
     // whose output index order (a | i, b, j) lies in om's own layout
@@ -733,10 +718,10 @@ bool Context::f64_resident() {
     if (f64_version == l_version) return true;
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
     // buffers of this shape already held (integrals of earlier Cholesky vectors) are reused
-    if (f64_gp.bytes() == sizeof(double) * nvp * nvp && f64_ovvv.bytes() == sizeof(double) * nov * nv * nv)
+    if (f64_gp.bytes() == sizeof(double) * nvp * nvp && f64_ovvv.bytes() == sizeof(double) * no * nmo * nv * nv)
         return true;
     if (f64_fit < 0 || f64_fit_version != l_version) {
-        const double need = 8.0 * (double(nvp) * nvp + double(nvm) * nvm + double(nov) * nv * nv);
+        const double need = 8.0 * (double(nvp) * nvp + double(nvm) * nvm + double(no) * nmo * nv * nv);
         size_t free_b = 0, total_b = 0;
         CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
         f64_fit = need < 0.5 * double(free_b) ? 1 : 0;
@@ -758,7 +743,7 @@ void Context::f64_integrals() {
     };
     hold(f64_gp, nvp * nvp);
     hold(f64_gm, std::max<int64_t>(nvm * nvm, 1));
-    hold(f64_ovvv, nov * nv * nv);
+    hold(f64_ovvv, no * nmo * nv * nv);
     {
         // L_vv as (J, c, a): columns (c, a) of one a-block are contiguous
         DBuf LT = dalloc(nJ * nv * nv, s);
@@ -775,35 +760,57 @@ void Context::f64_integrals() {
                      f64_gm.d() + nvm * std::max<int64_t>(a0 * (a0 - 1) / 2, 0), nv, a0, a1);
         }
     }
-    // g_kcbd as [k, b, c, d]
-    contract(ex, "Jkc,Jbd->kbcd", 1.0, tv(L_ov.d(), {nJ, no, nv}), tv(L_vv.d(), {nJ, nv, nv}), 0.0,
-             tv(f64_ovvv.d(), {no, nv, nv, nv}));
+    // g_kcpd as [k, p, c, d]: the virtual p, then the occupied
+    TV g = tv(f64_ovvv.d(), {no, nv, nv, nv});
+    g.s[2] = no * nmo;
+    g.s[3] = no * nmo * nv;
+    contract(ex, "Jkc,Jbd->kbcd", 1.0, tv(L_ov.d(), {nJ, no, nv}), tv(L_vv.d(), {nJ, nv, nv}), 0.0, g);
+    g.p += nov;
+    g.n[1] = no;
+    contract(ex, "Jkc,Jld->klcd", 1.0, tv(L_ov.d(), {nJ, no, nv}), tv(L_ov.d(), {nJ, no, nv}), 0.0, g);
     ex.prec = keep;
     f64_version = l_version;
     cache_epoch++;
 }
 
-int Context::f64_digit_planes(int digits) {
-    if (f64_dig_version == f64_version && f64_dig_digits == digits) return f64_dig_level;
+namespace {
+double digit_bytes(int digits, int64_t rows, int64_t k) {
+    return (double)digits * (double)((rows + 127) / 128 * 128) * (double)((k + 63) / 64 * 64);
+}
+}  // namespace
+
+bool Context::f64_ladder_planes(int digits) {
+    DigitFit &f = f64_ladder_fit;
+    if (f.version == f64_version && f.digits == digits) return f.held;
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
-    auto planes = [&](int64_t rows, int64_t k) {
-        return (double)digits * (double)((rows + 127) / 128 * 128) * (double)((k + 63) / 64 * 64);
-    };
-    const double ladder = planes(nvp, nvp) + (nvm > 0 ? planes(nvm, nvm) : 0.0), ovvv = planes(nov, nv * nv);
-    for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig, &f64_ovvv_dig}) p->buf.release();
+    for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig}) p->buf.release();
     size_t free_b = 0, total_b = 0;
     CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    const double room = 0.6 * (double)free_b;
-    f64_dig_level = ladder + ovvv <= room ? 2 : ladder <= room ? 1 : 0;
-    if (f64_dig_level >= 1) {
+    f.held = digit_bytes(digits, nvp, nvp) + (nvm > 0 ? digit_bytes(digits, nvm, nvm) : 0.0) <= 0.6 * (double)free_b;
+    if (f.held) {
         ozaki_prepare(ex, true, nvp, nvp, f64_gp.d(), nvp, digits, f64_gp_dig);
         if (nvm > 0) ozaki_prepare(ex, true, nvm, nvm, f64_gm.d(), nvm, digits, f64_gm_dig);
     }
-    if (f64_dig_level == 2) ozaki_prepare(ex, false, nov, nv * nv, f64_ovvv.d(), nov, digits, f64_ovvv_dig);
-    f64_dig_version = f64_version;
-    f64_dig_digits = digits;
+    f.version = f64_version;
+    f.digits = digits;
     cache_epoch++;
-    return f64_dig_level;
+    return f.held;
+}
+
+bool Context::f64_ovvv_planes(int digits) {
+    DigitFit &f = f64_ovvv_fit;
+    if (f.version == f64_version && f.digits == digits) return f.held;
+    f64_ovvv_dig.buf.release();
+    const bool ladder = f64_ladder_digits() > 0;
+    if (ladder) f64_ladder_planes(digits);   // first claim
+    size_t free_b = 0, total_b = 0;
+    CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    f.held = (!ladder || f64_ladder_fit.held) && digit_bytes(digits, no * nmo, nv * nv) <= 0.6 * (double)free_b;
+    if (f.held) ozaki_prepare(ex, false, no * nmo, nv * nv, f64_ovvv.d(), no * nmo, digits, f64_ovvv_dig);
+    f.version = f64_version;
+    f.digits = digits;
+    cache_epoch++;
+    return f.held;
 }
 
 // The int8 digit GEMM takes the FP64 ladder products under the same size rule as gemm(); their constant
@@ -821,12 +828,12 @@ void Context::ladder_f64(const double *t2, double *om2) {
     const int64_t nop = no * (no + 1) / 2, nom = no * (no - 1) / 2;
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
     const int digits = f64_ladder_digits();
-    const int level = digits ? f64_digit_planes(digits) : 0;
+    const bool planes = digits && f64_ladder_planes(digits);
     // X0 = sum_cd g_acbd t_cidj of the untransformed integrals, all pairs in two GEMMs
     DBuf tp = dalloc(nop * nvp, s), tm = dalloc(std::max<int64_t>(nom * nvm, 1), s);
     build_tpm(ex, t2, no, nv, 1, tp.d(), nvp, tm.d(), nvm);
     DBuf wp = dalloc(nop * nvp, s), wm = dalloc(std::max<int64_t>(nom * nvm, 1), s);
-    if (level >= 1) {
+    if (planes) {
         ozaki_gemm(ex, true, false, nvp, nop, nvp, 0.5, f64_gp.d(), nvp, tp.d(), nvp, 0.0, wp.d(), nvp, digits, &f64_gp_dig);
         if (nom > 0 && nvm > 0)
             ozaki_gemm(ex, true, false, nvm, nom, nvm, 0.5, f64_gm.d(), nvm, tm.d(), nvm, 0.0, wm.d(), nvm, digits,
@@ -840,35 +847,55 @@ void Context::ladder_f64(const double *t2, double *om2) {
     add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, 1, 0, nv, nvp, nvm);
 }
 
-void Context::ladder_y_plain(const double *tf, double *Y) {
-    if (ex.prec == Prec::MIXED) {
-        if (ovvv_resident()) ladder_y0(tf, Y);
-        else ladder_y(L_vv.d(), tf, Y);
-        return;
-    }
-    f64_integrals();
+Context::LadderY Context::ladder_y_plain(const double *tf) {
     cudaStream_t s = ex.stream;
-    const int digits = f64_ladder_digits();
-    if (digits && f64_digit_planes(digits) == 2) {
-        // Y_kibj = sum_cd g_kbcd t_cidj: t as [(c, d), (i, j)], the product [(k, b), (i, j)], then Y
-        DBuf TT = dalloc(nv * nv * no * no, s), W = dalloc(nov * no * no, s);
-        TV tt = tv(TT.d(), {nv, no, nv, no});   // (c, i, d, j) at c + nv d + nv^2 (i + no j)
-        tt.s[1] = nv * nv;
-        tt.s[2] = nv;
-        tt.s[3] = nv * nv * no;
-        permute_add(ex, 1.0, tv(tf, {nv, no, nv, no}), 0.0, tt);
-        ozaki_gemm(ex, false, false, nov, no * no, nv * nv, 1.0, f64_ovvv.d(), nov, TT.d(), nv * nv, 0.0, W.d(), nov,
-                   digits, &f64_ovvv_dig, nullptr);
-        ex.flops += 2.0 * double(nov) * double(no * no) * double(nv * nv);
-        TV w = tv(W.d(), {no, no, nv, no});     // (k, i, b, j) at k + no b + no nv (i + no j)
-        w.s[1] = no * nv;
-        w.s[2] = no;
-        w.s[3] = no * nv * no;
-        permute_add(ex, 1.0, w, 0.0, tv(Y, {no, no, nv, no}));
-    } else {
-        contract(ex, "kbcd,cidj->kibj", 1.0, tv(f64_ovvv.d(), {no, nv, nv, nv}), tv(tf, {nv, no, nv, no}), 0.0,
-                 tv(Y, {no, no, nv, no}));
+    const int64_t oo = no * no, nv2 = nv * nv, rows = no * nmo;
+    LadderY r;
+    r.Y = dalloc(oo * nov, s);
+    r.Q = dalloc(oo * oo, s);
+    if (ex.prec == Prec::MIXED && !ovvv_resident()) {
+        ladder_y(L_vv.d(), tf, r.Y.d());
+        contract(ex, "kcld,cidj->kilj", 1.0, tv(g_ovov_const(), {no, nv, no, nv}), tv(tf, {nv, no, nv, no}), 0.0,
+                 tv(r.Q.d(), {no, no, no, no}));
+        return r;
     }
+    // t as [(c, d), (i, j)], the product [(k, p), (i, j)]
+    DBuf TT = dalloc(oo * nv2, s), W = dalloc(rows * oo, s);
+    {
+        TV dst = tv(TT.d(), {nv, no, nv, no});
+        dst.s[1] = nv2;        // i
+        dst.s[2] = nv;         // d
+        dst.s[3] = nv2 * no;   // j
+        permute_add(ex, 1.0, tv(tf, {nv, no, nv, no}), 0.0, dst);
+    }
+    if (ex.prec == Prec::MIXED) {
+        ovvv_pairs();
+        const int64_t Kq = tc_pad_k(nv2), rows_T = tc_pad_rows_b(oo);
+        DBuf TS(sizeof(__nv_bfloat16) * ex.planes * rows_T * Kq, s);
+        split_rows(ex, TT.d(), nv2, 1, oo, nv2, rows_T, Kq, TS.as<__nv_bfloat16>());
+        tc_gemm_f64_tuned(ex, ybuf.as<__nv_bfloat16>(), tc_pad_rows_a(rows), TS.as<__nv_bfloat16>(), rows_T, Kq, rows, oo,
+                          nv2, 1.0, 0.0, W.d(), rows, 0);
+        ex.flops += 2.0 * double(rows) * double(oo) * double(nv2);
+    } else {
+        f64_integrals();
+        const double fl = 2.0 * double(rows) * double(oo) * double(nv2);
+        if (gemm_takes_digits(ex, rows, oo, nv2, fl) && f64_ovvv_planes(ex.fp64_digits)) {
+            ozaki_gemm(ex, false, false, rows, oo, nv2, 1.0, f64_ovvv.d(), rows, TT.d(), nv2, 0.0, W.d(), rows,
+                       ex.fp64_digits, &f64_ovvv_dig, nullptr);
+            ex.flops += fl;
+        } else {
+            gemm(ex, false, false, rows, oo, nv2, 1.0, f64_ovvv.d(), rows, TT.d(), nv2, 0.0, W.d(), rows, false);
+        }
+    }
+    TV src = tv(W.d(), {no, no, nv, no});   // (k, i, b, j)
+    src.s[1] = rows;
+    src.s[2] = no;
+    src.s[3] = rows * no;
+    permute_add(ex, 1.0, src, 0.0, tv(r.Y.d(), {no, no, nv, no}));
+    src.p += nov;                           // (k, i, l, j)
+    src.n[2] = no;
+    permute_add(ex, 1.0, src, 0.0, tv(r.Q.d(), {no, no, no, no}));
+    return r;
 }
 
 // ---------------------------------------------------------------------------

@@ -61,14 +61,16 @@ struct Context {
     DBuf gov;                  // g_iajb cache (g_ovov_const)
     bool have_gov = false;
     int64_t gov_id = 0;        // bumped whenever gov is formed again
-    DBuf hov;                  // g_lckd - 1/2 g_kcld (h_ovov_const), formed from gov number hov_id
-    int64_t hov_id = -1;
+    // in pair layout (v,o,v,o), formed from gov number gov_pairs_id (g_pairs_const): gex[c,l,d,k] = g_kcld
+    // and hov[c,l,d,k] = g_lckd - 1/2 g_kcld
+    DBuf hov, gex;
+    int64_t gov_pairs_id = -1;
     int64_t l_version = 0;     // bumped whenever the Cholesky vectors change
     // what mbuf holds: 0 nothing, 1 untransformed L_vv pairs (valid for mbuf_version), 2 per call
     int mbuf_kind = 0, mbuf_planes = 0;
     int64_t mbuf_version = -1;
-    // split-bf16 ovvv integrals g_kcbd of the untransformed vectors at [plane][k + no*b][c + nv*d]
-    // (mixed precision; valid for ybuf_version)
+    // split-bf16 integrals g_kcpd of the untransformed vectors at [plane][k + no*p][c + nv*d], p over the
+    // n_v virtual and then the n_o occupied orbitals (mixed precision; valid for ybuf_version)
     DBuf ybuf;
     size_t ybuf_bytes = 0;
     int ybuf_planes = 0;
@@ -131,7 +133,7 @@ struct Context {
     // g_iajb = sum_J L_ia L_jb in FP64, kept until the Cholesky vectors change: the ov block is
     // unchanged by the T1 transformation, so every iteration shares it
     const double *g_ovov_const();
-    const double *h_ovov_const();
+    void g_pairs_const();                    // hov and gex
     double energy();
     void mp2_guess();
     void omega(double *d_omega);
@@ -142,17 +144,23 @@ struct Context {
     // const_t1: take the T1-transformed blocks and the Fock matrix from the context (only when no
     // derivative will be taken and t1_current holds)
     OmegaNodes record_omega(Graph &g, bool const_ovov = true, bool const_t1 = false);
-    void record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, int tf);
+    // Y0_kibj = sum_cd g_kcbd tau_cidj and Q_kilj = sum_cd g_kcld tau_cidj of the untransformed vectors
+    struct LadderY {
+        DBuf Y, Q;
+    };
+    void record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, int tf, std::shared_ptr<LadderY> yq);
     void record_ladder(Graph &g, int om2, int Lvv, int t2);
     void ladder_y(const double *Lvv, const double *tfull, double *Y);
-    // mixed precision: whether the resident ovvv planes fit, their construction, and
-    // Y0_kibj = sum_cd g_kcbd tau_cidj from them
+    // mixed precision: whether the resident ovvv planes fit, and their construction
     bool ovvv_resident();
     void ovvv_pairs();
-    void ladder_y0(const double *tfull, double *Y);
-    // Y with the T1-transformed vv block Ltvv, sum_cd g_kc~bd tau_cidj: in mixed precision
-    // Y0_kibj - sum_l t_bl Q_kilj (Q_kilj = sum_cd g_kcld tau_cidj), else ladder_y(Ltvv)
-    void ladder_y_t1(const double *t1, const double *Ltvv, const double *tfull, double *Y);
+    // whether the current precision evaluates the residual's ladder from untransformed integrals, and Y0
+    // and Q from whatever integrals it keeps, in one product where the planes or blocks are resident
+    bool plain_ladder() { return ex.prec == Prec::MIXED || f64_resident(); }
+    LadderY ladder_y_plain(const double *tfull);
+    // Y with the T1-transformed vv block Ltvv, sum_cd g_kc~bd tau_cidj: Y0_kibj - sum_l t_bl Q_kilj from the
+    // residual's Y0 and Q (yq, may be empty) or resident integrals, else ladder_y(Ltvv)
+    void ladder_y_t1(const double *t1, const double *Ltvv, const double *tfull, const LadderY &yq, double *Y);
     // throws CCSD_GPU_ETIMEOUT (and clears the word) when a tensor-core GEMM of this context
     // reported a bounded wait that ran out
     void check_gemm();
@@ -182,24 +190,25 @@ struct Context {
     TPlanes t_planes(const double *t2, int64_t nvec);
     void ladder_pm_block(const TPlanes &T, int64_t nvec, const __nv_bfloat16 *Pp, int64_t prow, const __nv_bfloat16 *Pm,
                          int64_t mrow, int64_t a0, int64_t a1, double *om2);
-    // Y0_kibj = sum_cd g_kcbd tau_cidj of the untransformed vectors, from whatever integrals the
-    // current precision keeps
-    void ladder_y_plain(const double *tfull, double *Y);
     // om += -A + T4/2 with A_aibj = sum_k t_ak Y0_kibj, T4 = sum_kl t_ak t_bl Q_kilj (om is packed as
     // om + om^T)
-    void ladder_t1_corrections(const double *t1, const double *tf, double *om);
+    void ladder_t1_corrections(const double *t1, const LadderY &yq, double *om);
     // the t2 ladder in FP64 from resident FP64 integrals (f64_resident() must hold)
     bool f64_resident();
     void f64_integrals();
     int f64_ladder_digits();                 // digits of its products on the digit GEMM, 0: DGEMM
     void ladder_f64(const double *t2, double *om2);
-    // digit planes of the resident FP64 integrals for FP64 evaluations on the int8 digit GEMM: the
-    // +/- ladder integrals (B operands) and g_kcbd (A operand of Y), kept per Cholesky set and digit
-    // count while they fit (levels: 2 all three, 1 the ladder pair only, 0 none)
-    int f64_digit_planes(int digits);
+    // digit planes of the resident FP64 integrals for FP64 evaluations on the int8 digit GEMM: the +/- ladder
+    // integrals and g_kcpd (the row operands of their products), each kept per Cholesky set and digit count
+    // while it fits; the ladder's have the first claim on the memory
+    bool f64_ladder_planes(int digits);
+    bool f64_ovvv_planes(int digits);
     OzPlanes f64_gp_dig, f64_gm_dig, f64_ovvv_dig;
-    int64_t f64_dig_version = -1;
-    int f64_dig_digits = 0, f64_dig_level = 0;
+    struct DigitFit {
+        int64_t version = -1;
+        int digits = 0;
+        bool held = false;
+    } f64_ladder_fit, f64_ovvv_fit;
     int davidson(int nstates, int side, const ccsd_gpu_davidson_options *o, double *omega_out, double *vectors_out,
                  int32_t *iters_out, const double *start = nullptr);
     void eta(double *out);

@@ -192,13 +192,30 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         G4 = g.zeros("g_ovov", {no, nv, no, nv});
         g.contract(G4, "Jia,Jjb->iajb", 1.0, Lt_ov, Lt_ov);
     }
+    // its forms in the pair layout of the amplitudes: H = g_lckd - 1/2 g_kcld and the exchanged g_kcld, both
+    // as [c, l, d, k], so that the products with t and u below are matrix products as they lie.  H, g_kcld, t, u
+    // and the exchanged t are symmetric in their two pairs: each product names the pair that it sums first, so
+    // that its operands run along the summed index in memory
+    int H, GX;
+    if (const_ovov) {
+        g_pairs_const();
+        H = g.input("H_cldk", V4, hov.d());
+        GX = g.input("gx_cldk", V4, gex.d());
+    } else {
+        H = g.zeros("H_cldk", V4);
+        GX = g.zeros("gx_cldk", V4);
+        g.permute(GX, "kcld->cldk", 1.0, G4);
+        g.permute(H, "lckd->cldk", 1.0, G4);
+        g.permute(H, "cldk->cldk", -0.5, GX);
+    }
     // omega_ccsd_e2 (omega_ccsd.F90:712-878); Fock parts in FP64
     const int om = g.zeros("omega_aibj", V4), x = g.zeros("x_c2", V4);
     {
         TermTimer tt(ex, "omega ccsd e2");
         const int Xbc = g.zeros("X_bc", {nv, nv}), Ykj = g.zeros("Y_kj", {no, no});
-        g.contract(Xbc, "bkdl,ldkc->bc", -1.0, u, G4);
-        g.contract(Ykj, "kdlc,djcl->kj", 1.0, G4, u);
+        // sum_kdl u_bkdl g_ldkc = 2 sum t_bkdl H_kcld, sum_dlc g_kdlc u_djcl = 2 sum H_lckd t_cldj
+        g.contract(Xbc, ex.prec == Prec::FP64 ? "bkdl,ckdl->bc" : "dlbk,dlck->bc", -2.0, tf, H);
+        g.contract(Ykj, "cldk,cldj->kj", 2.0, H, tf);
         // the Fock blocks join X and Y, so each side is one FP64 product with t (the Fock parts are
         // first-order terms)
         g.permute(Xbc, "bc->bc", 1.0, F_vv);
@@ -206,6 +223,7 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         g.contract(om, "bc,cjai->bjai", 1.0, Xbc, tf, true);
         g.contract(om, "aibk,kj->aibj", -1.0, tf, Ykj, true);
     }
+    auto yq = std::make_shared<LadderY>();
     // om collects the terms that eT symmetrises (symmetric_sum, reordering.F90:416), x the C2 term whose
     // third and exchanged two thirds join them: the doubles residual is pack(z + z^T), z = om + x_aibj/3
     // + 2 x_ajbi/3, with the diagonal halved, formed in one pass at the end.  Terms
@@ -216,7 +234,17 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         g.contract_sym(om, "Jai,Jbj->aibj", 0.5, Lt_vo, true);
         const int X4 = g.zeros("X_klij", {no, no, no, no});
         g.contract(X4, "Jki,Jlj->klij", 1.0, Lt_oo, Lt_oo);
-        g.contract(X4, "kcld,cidj->klij", 1.0, G4, tf);
+        if (const_ovov && plain_ladder()) {
+            // Q_kilj of the ladder's t1 part is this term
+            *yq = ladder_y_plain(g.value(tf));
+            g.contract_given(X4, "kcld,cidj->klij", 1.0, G4, tf, [&]() {
+                TV q = tv(yq->Q.d(), {no, no, no, no});   // [k, i, l, j] read as [k, l, i, j]
+                std::swap(q.s[1], q.s[2]);
+                permute_add(ex, 1.0, q, 1.0, tv(g.node(X4).v, {no, no, no, no}));
+            });
+        } else {
+            g.contract(X4, "kcld,cidj->klij", 1.0, G4, tf);
+        }
         g.contract(om, "akbl,klij->aibj", 0.5, tf, X4);
     }
     // omega_ccsd_c2_d2 (omega_ccsd.F90:586-709) in contraction form
@@ -235,22 +263,21 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
         }
         g.permute(D, "ckaj->ckaj", -1.0, C);
         g.contract(D, "Jai,Jkc->ckai", 2.0, Lt_vo, Lt_ov);
-        g.contract(C, "kcld,djak->claj", -0.5, G4, tf);
-        // the two g_ovov terms of D share u: one contraction with H_lckd = g_lckd - 1/2 g_kcld
-        int H;
-        if (const_ovov) {
-            H = g.input("H_lckd", {no, nv, no, nv}, h_ovov_const());
+        if (ex.prec == Prec::FP64) {
+            // t_djak as [d, k, a, j], shared by both of its products (the tensor-core GEMM gathers it itself)
+            const int tx = g.zeros("tx_dkaj", V4);
+            g.permute(tx, "djak->dkaj", 1.0, tf);
+            g.contract(C, "dkcl,dkaj->claj", -0.5, GX, tx);
+            g.contract(x, "ckai,ckbj->aibj", -1.5, tx, C);
         } else {
-            H = g.zeros("H_lckd", {no, nv, no, nv});
-            g.permute(H, "lckd->lckd", 1.0, G4);
-            g.permute(H, "kcld->lckd", -0.5, G4);
+            g.contract(C, "dkcl,djak->claj", -0.5, GX, tf);
+            g.contract(x, "ciak,ckbj->aibj", -1.5, tf, C);
         }
-        g.contract(D, "lckd,dkaj->claj", 1.0, H, u);
-        g.contract(x, "akci,ckbj->aibj", -1.5, tf, C);
-        g.contract(om, "aick,ckbj->aibj", 0.5, u, D);
+        g.contract(D, "dkcl,dkaj->claj", 1.0, H, u);
+        g.contract(om, "ckai,ckbj->aibj", 0.5, u, D);
     }
     // omega_ccsd_a2 (omega_ccsd.F90:113-480) as custom ops: its t1 part joins om, its t2 part the packed residual
-    record_ladder_t1(g, om, Lt_vv, t1, n.L_vv, tf);
+    record_ladder_t1(g, om, Lt_vv, t1, n.L_vv, tf, yq);
     const int om2 = g.zeros("omega2", {nt2});
     g.sym_pack(om2, om, x, 1.0 / 3.0, 2.0 / 3.0);   // symmetric_sum + scale_diagonal(1/2) + packin
     record_ladder(g, om2, Lt_vv, n.t2);
@@ -284,19 +311,21 @@ void Context::ladder_y(const double *Lvv, const double *tfull, double *Y) {
 // the residual the corrections that turn integrals of the untransformed vectors into T1-transformed
 // ones (nothing when the integrals are formed from transformed vectors); in the derivative passes the
 // t1 derivative through Y.
-void Context::record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, int tf) {
+void Context::record_ladder_t1(Graph &g, int om, int Lvv, int t1, int L_vv_in, int tf, std::shared_ptr<LadderY> yq) {
     auto Ycache = std::make_shared<DBuf>();
-    auto getY = [this, &g, Lvv, t1, tf, Ycache]() -> const double * {
+    auto getY = [this, &g, Lvv, t1, tf, yq, Ycache]() -> const double * {
         if (!*Ycache) {
             *Ycache = dalloc(no * no * nv * no, ex.stream);
-            ladder_y_t1(g.value(t1), g.value(Lvv), g.value(tf), Ycache->d());
+            ladder_y_t1(g.value(t1), g.value(Lvv), g.value(tf), *yq, Ycache->d());
         }
         return Ycache->d();
     };
     CustomOp op;
-    op.forward = [this, &g, om, t1, tf]() {
+    op.forward = [this, &g, om, t1, tf, yq]() {
         TermTimer tt(ex, "omega ccsd a2");
-        if (ex.prec == Prec::MIXED || f64_resident()) ladder_t1_corrections(g.value(t1), g.value(tf), g.node(om).v);
+        if (!plain_ladder()) return;
+        if (!yq->Y) *yq = ladder_y_plain(g.value(tf));
+        ladder_t1_corrections(g.value(t1), *yq, g.node(om).v);
     };
     op.tangent_reads = {t1};
     op.tangent = [this, &g, om, Lvv, t1, getY](int nvec) {
@@ -382,7 +411,7 @@ void Context::omega_eager(double *om_out) {
 }
 
 void Context::prepare_residual_caches() {
-    g_ovov_const();
+    g_pairs_const();
     if (ex.prec == Prec::MIXED) {
         if (ladder_pairs_resident()) ladder_pairs(L_vv.d(), true);
         if (ovvv_resident()) ovvv_pairs();

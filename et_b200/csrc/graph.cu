@@ -229,6 +229,21 @@ void Graph::contract_sym(int out, const char *spec, double alpha, int a, bool fp
     record(std::move(op));
 }
 
+void Graph::contract_given(int out, const char *spec, double alpha, int a, int b,
+                           const std::function<void()> &forward) {
+    GOp op;
+    op.kind = OpKind::Contract;
+    op.out = out;
+    op.a = a;
+    op.b = b;
+    op.alpha = alpha;
+    op.spec = spec;
+    materialize(out);
+    forward();
+    nodes_[a].last_use = nodes_[b].last_use = (int)ops_.size();
+    ops_.push_back(std::move(op));
+}
+
 void Graph::record(GOp op) {
     run_forward(op);
     for (int i : {op.a, op.b})

@@ -69,6 +69,8 @@ class Graph {
     // out += alpha * einsum(spec, a, a), symmetric under exchange of the two factors' indices, where every
     // reader of out takes its symmetric part (sym_pack): the two terms of its derivative count the same
     void contract_sym(int out, const char *spec, double alpha, int a, bool fp64 = false);
+    // the same product when its value is at hand: `forward` adds it to out, the derivative passes contract
+    void contract_given(int out, const char *spec, double alpha, int a, int b, const std::function<void()> &forward);
     // out += alpha * permute(a), spec "ajbi->aibj" (labels name the dims of a / out)
     void permute(int out, const char *spec, double alpha, int a);
     // t (full (v,o,v,o)) += squareup(a packed), u += c1 t_aibj + c2 t_ajbi

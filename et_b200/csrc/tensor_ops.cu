@@ -255,6 +255,11 @@ Route lookup_route(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int
 
 }  // namespace
 
+bool gemm_takes_digits(const Exec &ex, int64_t m, int64_t n, int64_t k, double fl) {
+    return ex.fp64_digits > 0 && fl >= ex.fp64_digits_min_flops &&
+           (ex.fp64_digits_min_flops <= 1 || (m >= 256 && n >= 256 && k >= 512));
+}
+
 namespace {
 
 // The route of a product that lookup_route does not know yet: every candidate timed on these operands
@@ -281,12 +286,6 @@ Route measure_route(Exec &ex, const Route &unknown, bool transA, bool transB, in
     return rt;
 }
 
-// whether an FP64 product goes to the int8 digit GEMM
-bool takes_digits(const Exec &ex, int64_t m, int64_t n, int64_t k, double fl) {
-    return ex.fp64_digits > 0 && fl >= ex.fp64_digits_min_flops &&
-           (ex.fp64_digits_min_flops <= 1 || (m >= 256 && n >= 256 && k >= 512));
-}
-
 void run_gemm(Exec &ex, const Route &rt, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha,
               const double *A, int64_t lda, const double *B, int64_t ldb, double beta, double *C, int64_t ldc) {
     const double fl = 2.0 * double(m) * double(n) * double(k);
@@ -298,7 +297,7 @@ void run_gemm(Exec &ex, const Route &rt, bool transA, bool transB, int64_t m, in
         mixed_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, rt.splits);
         return;
     }
-    if (takes_digits(ex, m, n, k, fl)) {
+    if (gemm_takes_digits(ex, m, n, k, fl)) {
         ozaki_gemm(ex, transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ex.fp64_digits);
         return;
     }
@@ -718,7 +717,7 @@ void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B
         return;
     }
     BatchPlan bp;
-    if (strided && !rt.mixed && !takes_digits(ex, mM, mN, mK, fl) &&
+    if (strided && !rt.mixed && !gemm_takes_digits(ex, mM, mN, mK, fl) &&
         find_batch(A, B, C, info, K, oM, oN, copy_bytes(A, packA, B, packB, C, cmode == 2), &bp)) {
         run_batch(ex, bp, A, B, C, alpha, beta);
         return;
