@@ -5,7 +5,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 
 #include "autotune.cuh"
 #include "mixed_gemm.cuh"
@@ -333,14 +332,43 @@ void gemm_batched_f64(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, 
 
 namespace {
 
+// What a contraction keeps per label and the short lists it sorts them into live on the stack: a small
+// system makes some forty contractions of a few microseconds per residual, and a map and a dozen heap
+// vectors per contraction took as long as their launches.
 struct LabelInfo {
     int64_t n = 1;
     int dA = -1, dB = -1, dC = -1;
+    bool used = false;
 };
+
+struct LabelTable {
+    LabelInfo t[128];
+    LabelInfo &operator[](char c) {
+        LabelInfo &l = t[(unsigned char)c & 127];
+        l.used = true;
+        return l;
+    }
+    const LabelInfo &at(char c) const { return t[(unsigned char)c & 127]; }
+};
+
+template <class T>
+struct Short {   // at most 12 labels or dims (two operands of six)
+    T v[12];
+    int n = 0;
+    void push_back(T x) { v[n++] = x; }
+    T *begin() { return v; }
+    T *end() { return v + n; }
+    const T *begin() const { return v; }
+    const T *end() const { return v + n; }
+    bool empty() const { return n == 0; }
+    T operator[](int i) const { return v[i]; }
+};
+using Labels = Short<char>;
+using Dims = Short<int>;
 
 // Is `v` (dims given by `order1` then `order2`) a column-major matrix [group1][group2]?
 // Returns the leading dimension in *ld.
-bool groupable(const TV &v, const std::vector<int> &g1, const std::vector<int> &g2, int64_t *ld) {
+bool groupable(const TV &v, const Dims &g1, const Dims &g2, int64_t *ld) {
     int64_t expect = 1;
     for (int d : g1) {
         if (v.n[d] == 1) continue;
@@ -363,20 +391,20 @@ bool groupable(const TV &v, const std::vector<int> &g1, const std::vector<int> &
     return true;
 }
 
-std::vector<char> natural_order(const TV &v, const std::vector<char> &labels, const std::map<char, LabelInfo> &info,
+Labels natural_order(const TV &v, const Labels &labels, const LabelTable &info,
                                 int which) {
-    std::vector<char> out = labels;
-    std::stable_sort(out.begin(), out.end(), [&](char x, char y) {
-        const LabelInfo &a = info.at(x), &b = info.at(y);
-        int da = which == 0 ? a.dA : which == 1 ? a.dB : a.dC;
-        int db = which == 0 ? b.dA : which == 1 ? b.dB : b.dC;
-        return v.s[da] < v.s[db];
-    });
+    Labels out = labels;
+    auto stride = [&](char c) {
+        const LabelInfo &l = info.at(c);
+        return v.s[which == 0 ? l.dA : which == 1 ? l.dB : l.dC];
+    };
+    for (int i = 1; i < out.n; i++)   // insertion sort: stable, a handful of labels
+        for (int j = i; j > 0 && stride(out.v[j]) < stride(out.v[j - 1]); j--) std::swap(out.v[j], out.v[j - 1]);
     return out;
 }
 
-std::vector<int> dims_of(const std::vector<char> &labels, const std::map<char, LabelInfo> &info, int which) {
-    std::vector<int> d;
+Dims dims_of(const Labels &labels, const LabelTable &info, int which) {
+    Dims d;
     for (char c : labels) {
         const LabelInfo &li = info.at(c);
         d.push_back(which == 0 ? li.dA : which == 1 ? li.dB : li.dC);
@@ -384,14 +412,14 @@ std::vector<int> dims_of(const std::vector<char> &labels, const std::map<char, L
     return d;
 }
 
-int64_t prod(const std::vector<char> &labels, const std::map<char, LabelInfo> &info) {
+int64_t prod(const Labels &labels, const LabelTable &info) {
     int64_t p = 1;
     for (char c : labels) p *= info.at(c).n;
     return p;
 }
 
 // Contiguous copy of v with dims reordered as [g1 labels][g2 labels].
-TV make_contiguous(Exec &ex, const TV &v, const std::vector<int> &g1, const std::vector<int> &g2, DBuf &buf) {
+TV make_contiguous(Exec &ex, const TV &v, const Dims &g1, const Dims &g2, DBuf &buf) {
     buf = dalloc(v.size(), ex.stream);
     TV dst;
     dst.p = buf.d();
@@ -412,7 +440,7 @@ TV make_contiguous(Exec &ex, const TV &v, const std::vector<int> &g1, const std:
 
 // v as a GEMM operand gather: rows over the dims `rows`, K over the dims `ks` (each in the order
 // given, first fastest; unit dims dropped).  False when a group spans more than four dims.
-bool gather_view(const TV &v, const std::vector<int> &rows, const std::vector<int> &ks, SplitView *out) {
+bool gather_view(const TV &v, const Dims &rows, const Dims &ks, SplitView *out) {
     SplitView g{};
     g.p = v.p;
     for (int d : rows) {
@@ -434,7 +462,7 @@ bool gather_view(const TV &v, const std::vector<int> &rows, const std::vector<in
 }
 
 // C as the output of a GEMM with rows over the dims `rows` and columns over `cols` (first fastest)
-bool out_view(const TV &C, const std::vector<int> &rows, const std::vector<int> &cols, OutView *out) {
+bool out_view(const TV &C, const Dims &rows, const Dims &cols, OutView *out) {
     OutView v{};
     v.p = C.p;
     // neighbouring dims that are one run of memory become one (a matrix then is one by one)
@@ -475,27 +503,27 @@ struct BatchPlan {
     int64_t nz = 1, zA = 0, zB = 0, zC = 0;   // batch count and strides
     int64_t nw = 1, wA = 0, wB = 0, wC = 0;   // loop count and strides
     bool copyA = false, copyB = false;        // an operand still needs its copy (the one without z, w)
-    std::vector<int> a1, a2, b1, b2;          // its dims as (first group, second group)
+    Dims a1, a2, b1, b2;          // its dims as (first group, second group)
 };
 
 // The plan that spares the most copying of those whose launches cost less than that: a copy of 16 MB takes
 // about as long as two launches.  False when none beats `base` bytes.
-bool find_batch(const TV &A, const TV &B, const TV &C, const std::map<char, LabelInfo> &info, const std::vector<char> &K,
-                const std::vector<char> &oM, const std::vector<char> &oN, double base, BatchPlan *best) {
+bool find_batch(const TV &A, const TV &B, const TV &C, const LabelTable &info, const Labels &K,
+                const Labels &oM, const Labels &oN, double base, BatchPlan *best) {
     bool found = false;
     double best_gain = 0.0;
     // a product bound by its flops gains little from the copies it is spared and loses more when the batch
     // falls on a narrower DGEMM tile (2048^3 with a batch of 16: 1.02 ms, 0.55 ms with both copies)
     const double fl = 2.0 * (double)prod(oM, info) * (double)prod(oN, info) * (double)prod(K, info);
     if (fl / 35e12 > 3.0 * base / 4e12) return false;
-    auto without = [](const std::vector<char> &v, char z, char w) {
-        std::vector<char> o;
+    auto without = [](const Labels &v, char z, char w) {
+        Labels o;
         for (char c : v)
             if (c != z && c != w) o.push_back(c);
         return o;
     };
-    std::vector<char> outs = oM;
-    outs.insert(outs.end(), oN.begin(), oN.end());
+    Labels outs = oM;
+    for (char c : oN) outs.push_back(c);
     auto try_plan = [&](char z, char w) {
         BatchPlan p;
         const auto M = without(oM, z, w), N = without(oN, z, w);
@@ -596,20 +624,19 @@ void run_batch(Exec &ex, const BatchPlan &p, const TV &A, const TV &B, const TV 
 
 void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B, double beta, const TV &C) {
     PermTag tag(spec);
-    std::string s(spec);
-    size_t comma = s.find(','), arrow = s.find("->");
-    REQUIRE(comma != std::string::npos && arrow != std::string::npos, CCSD_GPU_EINVAL, "contract: bad spec");
-    std::string la = s.substr(0, comma), lb = s.substr(comma + 1, arrow - comma - 1), lc = s.substr(arrow + 2);
-    REQUIRE((int)la.size() == A.nd && (int)lb.size() == B.nd && (int)lc.size() == C.nd, CCSD_GPU_EINVAL,
+    const char *comma = std::strchr(spec, ','), *arrow = std::strstr(spec, "->");
+    REQUIRE(comma && arrow && comma < arrow, CCSD_GPU_EINVAL, "contract: bad spec");
+    const char *la = spec, *lb = comma + 1, *lc = arrow + 2;
+    REQUIRE(comma - la == A.nd && arrow - lb == B.nd && (int)std::strlen(lc) == C.nd, CCSD_GPU_EINVAL,
             std::string("contract: rank mismatch in ") + spec);
-    std::map<char, LabelInfo> info;
+    LabelTable info;
     for (int d = 0; d < A.nd; d++) {
         info[la[d]].dA = d;
         info[la[d]].n = A.n[d];
     }
     for (int d = 0; d < B.nd; d++) {
         auto &li = info[lb[d]];
-        REQUIRE(li.dA < 0 || li.n == B.n[d], CCSD_GPU_EINVAL, std::string("contract: extent mismatch in ") + spec);
+        if (li.dA >= 0 && li.n != B.n[d]) throw Error(CCSD_GPU_EINVAL, std::string("contract: extent mismatch in ") + spec);
         li.dB = d;
         li.n = B.n[d];
     }
@@ -619,23 +646,24 @@ void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B
         REQUIRE(li.n == C.n[d], CCSD_GPU_EINVAL, std::string("contract: output extent mismatch in ") + spec);
         li.dC = d;
     }
-    std::vector<char> K, M, N;
-    for (auto &kv : info) {
-        const LabelInfo &li = kv.second;
+    Labels K, M, N;
+    for (int c = 0; c < 128; c++) {
+        const LabelInfo &li = info.t[c];
+        if (!li.used) continue;
         int cnt = (li.dA >= 0) + (li.dB >= 0) + (li.dC >= 0);
         REQUIRE(cnt == 2, CCSD_GPU_EINVAL, std::string("contract: label must appear exactly twice in ") + spec);
-        if (li.dA >= 0 && li.dB >= 0) K.push_back(kv.first);
-        else if (li.dA >= 0) M.push_back(kv.first);
-        else N.push_back(kv.first);
+        if (li.dA >= 0 && li.dB >= 0) K.push_back((char)c);
+        else if (li.dA >= 0) M.push_back((char)c);
+        else N.push_back((char)c);
     }
     const int64_t mK = prod(K, info), mM = prod(M, info), mN = prod(N, info);
     if (mM == 0 || mN == 0) return;
 
     // label orders: M/N from C where possible, K from A
-    std::vector<char> oM = natural_order(C, M, info, 2), oN = natural_order(C, N, info, 2);
-    std::vector<char> oK = natural_order(A, K, info, 0);
+    Labels oM = natural_order(C, M, info, 2), oN = natural_order(C, N, info, 2);
+    Labels oK = natural_order(A, K, info, 0);
     {
-        std::vector<char> bK = natural_order(B, K, info, 1);
+        Labels bK = natural_order(B, K, info, 1);
         int64_t ld;
         // prefer B's K order when B is the bigger operand and already groupable with it
         if (B.size() > A.size() && (groupable(B, dims_of(bK, info, 1), dims_of(oN, info, 1), &ld) ||
