@@ -18,7 +18,8 @@
 // accumulated in passes of at most four (4 x 128 TMEM columns = all 512): pass 0 takes d = 0..3
 // (digits 0..3 of both operands), pass 1 takes d = 4..S-1 (all digits).  The epilogue adds
 // 2^(-7(d+2)) acc_d in FP64, scales by alpha 2^(ea_r + eb_c) and accumulates into the FP64 output;
-// one CTA takes all units (K chunk, pass) of a tile in order, so the sum is deterministic.  Every
+// one CTA takes all units (K chunk, pass) of a tile in order, so the sum is deterministic.  That form
+// serves operands of at most 128 rows; all others run on CTA pairs (ozaki_pair_kernel).  Every
 // mbarrier wait is bounded and reports to the caller's error word, as in the split-BF16 GEMM.
 #include <cuda.h>
 
@@ -75,14 +76,14 @@ struct OzMap {
     const int *ea, *eb;  // row exponents of op(A), column exponents of op(B)
     int *err;
     long long wait_cycles;
-    int bm = OBM;        // rows of one tile (256 for a CTA pair)
+    int bm = OBM, bn = OBN;   // tile (256 rows and up to 256 columns for a CTA pair)
     __device__ __forceinline__ void tile(int t, int &m0, int &n0) const {
         const int per_group = group_m * num_nt;
         const int grp = t / per_group, in = t - grp * per_group;
         const int first_m = grp * group_m;
         const int gsz = min(group_m, num_mt - first_m);
         m0 = (first_m + in % gsz) * bm;
-        n0 = (in / gsz) * OBN;
+        n0 = (in / gsz) * bn;
     }
     // diagonals [d0, d1) of pass p and the digits they need
     __device__ __forceinline__ void pass(int p, int &d0, int &d1, int &nd) const {
@@ -97,25 +98,7 @@ struct OzMap {
 // field per 16 bytes, tiles of A_TILE / B_TILE bytes), so issuing an MMA costs a few integer adds.  An
 // int8 MMA of 128 x 128 x 32 lasts ~64 tensor cycles; rebuilding descriptors per MMA had the single
 // issuing thread, not the tensor pipe, set the pace.
-// CTA-pair form of the int8 MMA (cta_group::2, M = 256 over the pair, N = 128): issued by CTA 0,
-// A rows from each CTA's own shared memory, the two 64-row halves of B from the two CTAs
-constexpr uint32_t IDESC_I8_PAIR = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OBN >> 3) << 17) |
-                                   ((uint32_t)(256 >> 4) << 24);
-
-template <bool PAIR>
-__device__ __forceinline__ void mma_i8_any(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-    if constexpr (PAIR) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(IDESC_I8_PAIR), "r"(accumulate));
-    } else {
-        mma_i8(d_tmem, adesc, bdesc, accumulate);
-    }
-}
-
-template <int S, int D0, int D1, bool PAIR, int BT>
+template <int S, int D0, int D1>
 __device__ __forceinline__ void issue_kblock(uint32_t tmem, uint64_t a0, uint64_t b0, bool first_kb) {
 #pragma unroll
     for (int kk = 0; kk < OBK / 32; kk++) {
@@ -125,23 +108,20 @@ __device__ __forceinline__ void issue_kblock(uint32_t tmem, uint64_t a0, uint64_
             for (int t = (d - S + 1 > 0 ? d - S + 1 : 0); t <= (d < S - 1 ? d : S - 1); t++) {
                 const int u = d - t;
                 const bool first = kk == 0 && t == (d - S + 1 > 0 ? d - S + 1 : 0);
-                mma_i8_any<PAIR>(tmem + (uint32_t)((d - D0) * OBN),
-                                 a0 + (uint64_t)(t * (A_TILE >> 4) + kk * 2),
-                                 b0 + (uint64_t)(u * (BT >> 4) + kk * 2), (first_kb && first) ? 0u : 1u);
+                mma_i8(tmem + (uint32_t)((d - D0) * OBN), a0 + (uint64_t)(t * (A_TILE >> 4) + kk * 2),
+                       b0 + (uint64_t)(u * (B_TILE >> 4) + kk * 2), (first_kb && first) ? 0u : 1u);
             }
         }
     }
 }
 
-// BT: bytes of one digit tile of B in shared memory (128 rows, or the 64 of one CTA of a pair);
-// BOFF: offset of the B digit tiles in a stage (after the A digit tiles)
-template <int S, bool PAIR = false, int BT = B_TILE, int BOFF = SLOTS * A_TILE>
+template <int S>
 __device__ __forceinline__ void issue_pass(int p, uint32_t tmem, const uint8_t *st, bool first_kb) {
-    const uint64_t a0 = smem_desc_k<64>(st, 0), b0 = smem_desc_k<64>(st + BOFF, 0);
+    const uint64_t a0 = smem_desc_k<64>(st, 0), b0 = smem_desc_k<64>(st + SLOTS * A_TILE, 0);
     if (p == 0)
-        issue_kblock<S, 0, (S < MAX_DIAG_PER_PASS ? S : MAX_DIAG_PER_PASS), PAIR, BT>(tmem, a0, b0, first_kb);
+        issue_kblock<S, 0, (S < MAX_DIAG_PER_PASS ? S : MAX_DIAG_PER_PASS)>(tmem, a0, b0, first_kb);
     else if constexpr (S > MAX_DIAG_PER_PASS)
-        issue_kblock<S, MAX_DIAG_PER_PASS, S, PAIR, BT>(tmem, a0, b0, first_kb);
+        issue_kblock<S, MAX_DIAG_PER_PASS, S>(tmem, a0, b0, first_kb);
 }
 
 template <int S>
@@ -319,50 +299,145 @@ ozaki_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
 }
 
-// The digit GEMM on a pair of CTAs (a cluster of two): one cta_group::2 MMA of M = 256 (each CTA's
-// 128 rows of A) and N = 128 (64 rows of B staged by each CTA).  A 128 x 128 x 32 int8 MMA reads
-// 8 KB of operands per 64 tensor cycles, all a single SM's shared memory delivers beside the TMA
-// writes; in the pair each SM's shared memory serves its A rows and half of B, 6 KB.  CTA 0 issues
-// the MMAs and waits for both CTAs' loads on its own barriers; its commits arrive on both CTAs.
-constexpr int BP_TILE = (OBN / 2) * OBK;                         // one CTA's half of a B digit tile
+// The digit GEMM on a pair of CTAs (a cluster of two) with 256-wide N tiles: one cta_group::2 MMA of
+// M = 256 (each CTA's 128 rows of A) and N up to 256 (half of B's rows staged by each CTA).
+//
+// What bounds it is shared memory, 128 bytes a cycle: an MMA of N = bn reads 4 KB of A and 32 bn bytes of B in
+// bn / 2 cycles, so a 128-wide tile, its two passes staging ten digit tiles a K block on top, kept the int8
+// pipe 67 % active.  At 256 columns the MMAs need 96 bytes a cycle and the staging 37, but TMEM then holds two
+// accumulators: the diagonals are taken two at a time, each such unit staging the digits up to its higher
+// diagonal (2 + 4 + 6 digit tiles a K block for six digits); tiles of at most 128 columns keep four.  What
+// keeps that rate up at L2's latency is bytes in flight: the ring's slots hold one digit of A and of B, the
+// products of a K block run from its highest digit down, and a slot is freed when its digit has taken part for
+// the last time (freeing a whole K block at once left 96 of the 192 KB idle: 2.1 instead of 2.7 POPS at
+// 4000^3).  Eight epilogue warps drain a unit (the accumulators are not double-buffered), old values a step
+// ahead.
+//
+// The sums keep the order of the single-CTA kernel, diagonals 0..3 and then 4..S-1 per K chunk: the sum of a
+// pass is exact in FP64 (four diagonals span 52 bits), so the units of a pass before its last leave their
+// share in a scratch of the CTA and the last adds it, and only then the scaled sum is rounded into the output.
+// With 6 digits, against the 128-wide pair kernel before it: 10240 x 10240 x 1200 2.65 ms (3.94), 4000^3 1.00 ms
+// (1.20), 4400 x 400 x 40000 1.64 ms (1.63 on single CTAs).
+constexpr int WBN = 256;
+constexpr int WRING = 12 * (A_TILE + (WBN / 2) * OBK);           // bytes of the ring of slots
+constexpr int WSLOTS = 20;                                        // slots at most (16 of a 128-wide tile)
+constexpr int WEPI_WARPS = 8, WTHREADS = 64 + 32 * WEPI_WARPS;
+constexpr int WSMEM = WRING + 1024 + 512 + WEPI_WARPS * (WBN / 2) * 8;
+static_assert(WSMEM <= 232448, "shared memory of the wide digit GEMM");
+constexpr uint32_t WIDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 4) << 24);
 
-// stages of S-digit operands: S digit tiles of A and S half tiles of B per K block; three stages where
-// they fit (up to six digits), which keeps the next two K blocks' loads in flight behind the MMAs
-template <int S>
-struct PairLayout {
-    static constexpr int STAGE = S * (A_TILE + BP_TILE);
-    static constexpr int STAGES = 3 * STAGE + 1024 + 256 <= 232448 ? 3 : 2;
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+__device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+// The digits of a K block in the order their slots are filled (and freed): the highest, 0, the second
+// highest, 1, ...
+__device__ __forceinline__ constexpr int digit_at(int pos, int nd) { return pos & 1 ? pos / 2 : nd - 1 - pos / 2; }
+
+// position in the ring of slots
+struct Ring {
+    int n_slots;
+    int slot = 0;
+    uint32_t phase = 0;   // parity of the slot's present use
+    __device__ __forceinline__ void advance(int n) {
+        slot += n;
+        if (slot >= n_slots) {
+            slot -= n_slots;
+            phase ^= 1;
+        }
+    }
+    __device__ __forceinline__ Ring ahead(int n) const {
+        Ring r = *this;
+        r.advance(n);
+        return r;
+    }
 };
-static_assert(PairLayout<6>::STAGES == 3 && PairLayout<7>::STAGES == 2, "pair stages");
 
-template <int S>
-__global__ void __launch_bounds__(OTHREADS, 1)
+// Waits for the slots of one K block (from ring position r) and issues its products of the NDIAG diagonals
+// ND - NDIAG .. ND - 1 (accumulator d - (ND - NDIAG), each `width` columns), from the products of the highest
+// digit down: step k pairs digit ND - 1 - k with the lower ones, so digit ND - 1 - k is free after step k and
+// digit j after step j + NDIAG - 1.  False when a wait ran out.
+template <int ND, int NDIAG>
+__device__ __forceinline__ bool issue_unit(uint32_t tmem, uint32_t width, uint64_t desc0, int slot_bytes, uint64_t *full, uint64_t *empty,
+                                           const Ring &r, uint32_t idesc, bool first_kb, long long limit) {
+    constexpr int D1 = ND - 1, D0 = ND - NDIAG, STEPS = D1 - (D0 + 1) / 2 + 1;
+    uint64_t da[ND];
+    bool ok = true;
+#pragma unroll
+    for (int step = 0; step < STEPS; step++) {
+        const int hi = D1 - step;
+#pragma unroll
+        for (int pos = 2 * step; pos < 2 * step + 2; pos++) {
+            if (pos < ND) {
+                const Ring p = r.ahead(pos);
+                ok = ok && mbar_wait(&full[p.slot], p.phase, limit);
+                da[digit_at(pos, ND)] = desc0 + (uint64_t)(p.slot * (slot_bytes >> 4));
+            }
+        }
+        if (!ok) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int d = D1; d >= D0; d--) {
+            const int lo = d - hi;
+            if (lo < 0 || lo > hi) continue;
+            const uint32_t acc = tmem + (uint32_t)(d - D0) * width;
+#pragma unroll
+            for (int kk = 0; kk < OBK / 32; kk++) {
+                // the first product of the unit into this accumulator overwrites it
+                const uint32_t add = first_kb && kk == 0 && lo == 0 ? 0u : 1u;
+                mma_i8_pair(acc, da[hi] + (uint64_t)(kk * 2), da[lo] + (uint64_t)((A_TILE >> 4) + kk * 2), idesc, add);
+                if (lo < hi)
+                    mma_i8_pair(acc, da[lo] + (uint64_t)(kk * 2), da[hi] + (uint64_t)((A_TILE >> 4) + kk * 2), idesc, 1u);
+            }
+        }
+        // positions 2 step (digit ND - 1 - step) and 2 (step - NDIAG + 1) + 1 (digit step - NDIAG + 1)
+        if (2 * step < ND) mma_commit_pair(&empty[r.ahead(2 * step).slot]);
+        const int low = 2 * (step - NDIAG + 1) + 1;
+        if (low > 0 && low < ND) mma_commit_pair(&empty[r.ahead(low).slot]);
+    }
+    // what the last step leaves
+#pragma unroll
+    for (int pos = 0; pos < ND; pos++) {
+        const bool freed = pos % 2 == 0 ? pos / 2 < STEPS : pos / 2 + NDIAG - 1 < STEPS;
+        if (!freed) mma_commit_pair(&empty[r.ahead(pos).slot]);
+    }
+    return true;
+}
+
+// Units of an S-digit product: `wide` tiles (more than 128 columns) take the diagonals two at a time, others
+// four at a time; unit u stages the digits up to its highest diagonal.
+__device__ __forceinline__ int unit_digits(int u, int digits, bool wide) { return min((wide ? 2 : 4) * (u + 1), digits); }
+
+__global__ void __launch_bounds__(WTHREADS, 1)
 ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OzMap map,
-                  int num_tiles) {
-    using PL = PairLayout<S>;
-    constexpr int NST = PL::STAGES, STAGE = PL::STAGE, BOFF = S * A_TILE;
+                  int num_tiles, double *__restrict__ scratch) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + NST * STAGE);
-    uint64_t *empty = full + NST;
-    uint64_t *acc_full = empty + NST;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + WRING);
+    uint64_t *empty = full + WSLOTS;
+    uint64_t *acc_full = empty + WSLOTS;
     uint64_t *acc_empty = acc_full + 1;   // used on CTA 0
     uint64_t *done = acc_empty + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    double *col_scales = reinterpret_cast<double *>(smem + WRING + 512);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const bool lead = rank == 0;
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NST; s++) {
+        for (int s = 0; s < WSLOTS; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         mbar_init(acc_full, 1);
-        mbar_init(acc_empty, 2 * (OEPI / 32));   // one arrival per epilogue warp of each CTA
+        mbar_init(acc_empty, 2 * WEPI_WARPS);   // one arrival per epilogue warp of each CTA
         mbar_init(done, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -378,66 +453,83 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     cluster_sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    const bool wide = map.bn > WBN / 2;
+    const int half = map.bn / 2, per = wide ? 2 : 4, units = (map.digits + per - 1) / per;
+    const int slot_bytes = A_TILE + half * OBK, n_slots = min(WSLOTS, WRING / slot_bytes);   // a slot: one digit of both
 
     if (warp == 0) {
         if (lane == 0) {
+            // producer of this CTA: for every (tile, chunk, unit) the digits of each K block, a slot each
+            const uint32_t bytes = 2u * (uint32_t)(A_TILE + half * OBK);
+            Ring r{n_slots};
             int g = 0;
-            int issued[NST] = {};
             for (int t = pair; t < num_tiles && !*abort_flag; t += npairs) {
                 int m0, n0;
                 map.tile(t, m0, n0);
+                const int ma = m0 + OBM * (int)rank, nb = n0 + half * (int)rank;
                 for (int c = 0; c < map.nchunks && !*abort_flag; c++) {
                     const int kb0 = c * map.kc, kb1 = min(map.nk_all, kb0 + map.kc);
-                    for (int p = 0; p < map.npass && !*abort_flag; p++) {
-                        int d0, d1, nd;
-                        map.pass(p, d0, d1, nd);
-                        for (int kb = kb0; kb < kb1; kb++, g++) {
-                            const int s = g % NST;
-                            if (!mbar_wait(&empty[s], ((g / NST) & 1) ^ 1, map.wait_cycles) || *abort_flag) {
-                                record_error(map.err, ERR_PRODUCER);
-                                *abort_flag = 1;
-                                break;
-                            }
-                            issued[s]++;
-                            uint8_t *st = smem + s * STAGE;
-                            if (lead) mbar_expect_tx(&full[s], 2u * (uint32_t)nd * (A_TILE + BP_TILE));
-                            for (int q = 0; q < nd; q++) {
-                                tma_load_3d_pair(&tmA, &full[s], st + q * A_TILE, kb * OBK, m0 + OBM * (int)rank, q);
-                                tma_load_3d_pair(&tmB, &full[s], st + BOFF + q * BP_TILE, kb * OBK,
-                                                 n0 + (OBN / 2) * (int)rank, q);
+                    for (int u = 0; u < units && !*abort_flag; u++) {
+                        const int nd = unit_digits(u, map.digits, wide);
+                        for (int kb = kb0; kb < kb1 && !*abort_flag; kb++) {
+                            for (int pos = 0; pos < nd; pos++) {
+                                if (!mbar_wait(&empty[r.slot], r.phase ^ 1, map.wait_cycles)) {
+                                    record_error(map.err, ERR_PRODUCER);
+                                    *abort_flag = 1;
+                                    break;
+                                }
+                                uint8_t *st = smem + r.slot * slot_bytes;
+                                const int q = digit_at(pos, nd);
+                                if (lead) mbar_expect_tx(&full[r.slot], bytes);
+                                tma_load_3d_pair(&tmA, &full[r.slot], st, kb * OBK, ma, q);
+                                tma_load_3d_pair(&tmB, &full[r.slot], st + A_TILE, kb * OBK, nb, q);
+                                r.advance(1);
+                                g++;
                             }
                         }
                     }
                 }
             }
+            // CTA 0 waits for the last load of each slot (both CTAs' bytes land on its barrier); CTA 1 keeps its
+            // shared memory until the final cluster barrier, which CTA 0 reaches after this
             if (lead)
-                for (int s = 0; s < NST; s++)
-                    if (issued[s] && !mbar_wait(&full[s], (issued[s] - 1) & 1, map.wait_cycles))
-                        record_error(map.err, ERR_DRAIN);
+                for (int s = 0; s < n_slots && s < g; s++)
+                    if (!mbar_wait(&full[s], ((g - 1 - s) / n_slots) & 1, map.wait_cycles)) record_error(map.err, ERR_DRAIN);
         }
     } else if (warp == 1) {
         if (lane == 0 && lead) {
-            int g = 0, uc = 0;
+            const uint32_t idesc = WIDESC | ((uint32_t)(map.bn >> 3) << 17);
+            const uint64_t desc0 = smem_desc_k<64>(smem, 0);
+            Ring r{n_slots};
+            int uc = 0;
             for (int t = pair; t < num_tiles && !*abort_flag; t += npairs) {
                 for (int c = 0; c < map.nchunks && !*abort_flag; c++) {
                     const int kb0 = c * map.kc, kb1 = min(map.nk_all, kb0 + map.kc);
-                    for (int p = 0; p < map.npass && !*abort_flag; p++, uc++) {
+                    for (int u = 0; u < units && !*abort_flag; u++, uc++) {
+                        const int nd = unit_digits(u, map.digits, wide), diags = nd - per * u;
                         if (!mbar_wait(acc_empty, (uc & 1) ^ 1, map.wait_cycles)) {
                             record_error(map.err, ERR_MMA_ACC);
                             *abort_flag = 1;
                             break;
                         }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        for (int kb = kb0; kb < kb1; kb++, g++) {
-                            const int s = g % NST;
-                            if (!mbar_wait(&full[s], (g / NST) & 1, map.wait_cycles) || *abort_flag) {
+                        for (int kb = kb0; kb < kb1; kb++) {
+                            const bool first = kb == kb0;
+                            bool ok = false;
+#define OZ_UNIT(ND, NDIAG)                                                                                                  case 8 * ND + NDIAG:                                                                                                       ok = issue_unit<ND, NDIAG>(tmem, wide ? WBN : WBN / 2, desc0, slot_bytes, full, empty, r, idesc, first, map.wait_cycles);          break;
+                            switch (8 * nd + diags) {
+                                // two at a time: 2, 4, 6 digits, or the last diagonal of 3, 5, 7
+                                OZ_UNIT(2, 2) OZ_UNIT(4, 2) OZ_UNIT(6, 2) OZ_UNIT(3, 1) OZ_UNIT(5, 1) OZ_UNIT(7, 1)
+                                // four at a time: up to four digits, then the rest of 6 or 7
+                                OZ_UNIT(3, 3) OZ_UNIT(4, 4) OZ_UNIT(7, 3)
+                            }
+#undef OZ_UNIT
+                            if (!ok || *abort_flag) {
                                 record_error(map.err, ERR_MMA_FULL);
                                 *abort_flag = 1;
                                 break;
                             }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            issue_pass<S, true, BP_TILE, BOFF>(p, tmem, smem + s * STAGE, kb == kb0);
-                            mma_commit_pair(&empty[s]);
+                            r.advance(nd);
                         }
                         mma_commit_pair(acc_full);
                     }
@@ -446,19 +538,28 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             mma_commit_pair(done);
         }
     } else {
-        // epilogue: this CTA's 128 rows; warp w drains TMEM lanes 32 (w % 4) .. +31
-        const int quarter = warp & 3;
+        // epilogue: this CTA's 128 rows; warp w drains TMEM lanes 32 (w % 4) .. +31, the first four warps the
+        // lower half of the columns
+        const int quarter = warp & 3, e = warp - 2;
+        double *scale = col_scales + e * (WBN / 2);
+        const int cbeg = e < 4 ? 0 : (map.bn / 32) * 16, cend = e < 4 ? (map.bn / 32) * 16 : map.bn;
+        // this thread's column of the CTA's scratch, 128 rows a column
+        double *part = scratch + (size_t)blockIdx.x * OBM * WBN + quarter * 32 + lane;
         int uc = 0;
         bool aborted = false;
         for (int t = pair; t < num_tiles && !aborted; t += npairs) {
             int m0, n0;
             map.tile(t, m0, n0);
             const int row = m0 + OBM * (int)rank + quarter * 32 + lane;
-            const double row_scale = row < map.M ? map.alpha * exp2((double)map.ea[row]) : 0.0;
+            const bool live = row < map.M;
+            const double row_scale = live ? map.alpha * exp2((double)map.ea[row]) : 0.0;
+            __syncwarp();
+            for (int i = lane; i < cend - cbeg; i += 32)
+                scale[i] = n0 + cbeg + i < map.N ? exp2((double)map.eb[n0 + cbeg + i]) : 0.0;
+            __syncwarp();
+            double *out = map.C + (long long)n0 * map.ldc + row;
             for (int c = 0; c < map.nchunks && !aborted; c++) {
-                for (int p = 0; p < map.npass; p++, uc++) {
-                    int d0, d1, nd;
-                    map.pass(p, d0, d1, nd);
+                for (int u = 0; u < units; u++, uc++) {
                     bool ok = !*abort_flag && mbar_wait(acc_full, uc & 1, map.wait_cycles);
                     __syncwarp();
                     if (!ok || *abort_flag) {
@@ -468,37 +569,58 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const bool first = (c == 0 && p == 0);
+                    const int d_lo = per * u, diags = unit_digits(u, map.digits, wide) - d_lo;
+                    // of a pass of four diagonals, the first unit and the last
+                    const bool opens = d_lo % MAX_DIAG_PER_PASS == 0;
+                    const bool closes = !wide || u == units - 1 || u == 1;
+                    const bool first = c == 0 && d_lo < MAX_DIAG_PER_PASS;      // beta applies to the first pass
+                    const bool read_c = closes && live && (!first || map.beta != 0.0);
+                    const uint32_t width = wide ? WBN : WBN / 2;
+                    const double w0 = exp2(-7.0 * (double)(d_lo + 2));
                     const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16);
+                    double ca[8], cb[8], pa[8], pb[8];   // output and scratch values of this step and the next
+                    auto fetch = [&](int cc, double (&o)[8], double (&p)[8]) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            o[j] = read_c && cc < cend && n0 + cc + j < map.N ? __ldcg(out + (long long)(cc + j) * map.ldc) : 0.0;
+                            p[j] = !opens && cc < cend ? __ldcg(part + (size_t)(cc + j) * OBM) : 0.0;
+                        }
+                    };
+                    auto emit = [&](int cc, const double (&o)[8], const double (&p)[8]) {
+                        uint32_t acc[MAX_DIAG_PER_PASS][8];
+#pragma unroll
+                        for (int h = 0; h < MAX_DIAG_PER_PASS; h++)   // diags is the same for every lane
+                            if (h < diags) tmem_ld8u_async(base + h * width + (uint32_t)cc, acc[h]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        double v[8], w = w0;
+#pragma unroll
+                        for (int j = 0; j < 8; j++) v[j] = p[j];
+#pragma unroll
+                        for (int h = 0; h < MAX_DIAG_PER_PASS; h++) {
+                            if (h < diags) {
+                                tmem_loaded8u(acc[h]);
+#pragma unroll
+                                for (int j = 0; j < 8; j++) v[j] += w * (double)(int)acc[h][j];
+                                w *= 1.0 / 128.0;
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            if (!closes) {
+                                part[(size_t)(cc + j) * OBM] = v[j];
+                            } else if (live && n0 + cc + j < map.N) {
+                                const double x = row_scale * scale[cc - cbeg + j] * v[j];
+                                out[(long long)(cc + j) * map.ldc] = first ? x + map.beta * o[j] : x + o[j];
+                            }
+                        }
+                    };
+                    fetch(cbeg, ca, pa);
 #pragma unroll 1
-                    for (int cc = 0; cc < OBN; cc += 16) {
-                        double v[16];
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = 0.0;
-                        for (int d = d0; d < d1; d++) {
-                            uint32_t r[16];
-                            tmem_ld16u(base + (uint32_t)((d - d0) * OBN + cc), r);
-                            const double w = exp2(-7.0 * (double)(d + 2));
-#pragma unroll
-                            for (int j = 0; j < 16; j++) v[j] += w * (double)(int)r[j];
-                        }
-                        if (row < map.M) {
-                            double *out = map.C + (long long)(n0 + cc) * map.ldc + row;
-                            double old[16];
-#pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                const bool in = n0 + cc + j < map.N;
-                                old[j] = (in && (!first || map.beta != 0.0)) ? __ldcg(out + (long long)j * map.ldc) : 0.0;
-                            }
-#pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                const int col = n0 + cc + j;
-                                if (col < map.N) {
-                                    const double x = row_scale * exp2((double)map.eb[col]) * v[j];
-                                    out[(long long)j * map.ldc] = first ? x + map.beta * old[j] : x + old[j];
-                                }
-                            }
-                        }
+                    for (int cc = cbeg; cc < cend; cc += 16) {
+                        fetch(cc + 8, cb, pb);
+                        emit(cc, ca, pa);
+                        fetch(cc + 16, ca, pa);
+                        emit(cc + 8, cb, pb);
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
@@ -722,6 +844,28 @@ void slab_digits(Exec &ex, const double *src, int64_t sr, int64_t sk, int64_t R,
     CU_CHECK(cudaGetLastError());
 }
 
+// N tile of the pair kernel: of the equal cuts of n into multiples of 32 from 64 to 256 columns the one whose
+// waves over the pairs cost least.  Per K block an SM's tensor core takes bn / 2 cycles per MMA, and its shared
+// memory moves 128 bytes a cycle: per MMA 4 KB of A and 32 bn of B, and once the digit tiles staged.  The
+// second is the larger below 224 columns, which is why narrow tiles need the better last wave to win.
+int pair_n_tile(int64_t mt, int64_t n, int digits, int64_t pairs) {
+    auto cost = [&](int bn) {
+        const int per = bn > WBN / 2 ? 2 : 4;
+        int tiles = 0;   // digit tiles staged per K block
+        for (int nd = per; nd < digits + per; nd += per) tiles += std::min(nd, digits);
+        const int64_t units = mt * ((n + bn - 1) / bn);
+        const double mmas = digits * (digits + 1) / 2 * (OBK / 32);
+        const double smem = (mmas * (OBM * 32 + bn * 32) + tiles * double(A_TILE + bn / 2 * OBK)) / 128.0;
+        return double((units + pairs - 1) / pairs) * std::max(mmas * bn / 2.0, smem);
+    };
+    int best = WBN;
+    for (int64_t nt = (n + WBN - 1) / WBN; nt <= (n + 63) / 64; nt++) {
+        const int bn = (int)std::min<int64_t>(WBN, round_up((n + nt - 1) / nt, (int64_t)32));
+        if (cost(bn) < 0.999 * cost(best)) best = bn;
+    }
+    return best;
+}
+
 }  // namespace
 
 void ozaki_prepare(Exec &ex, bool trans, int64_t rows, int64_t k, const double *X, int64_t ldx, int digits,
@@ -763,52 +907,19 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     // op(A)(r, kk): A[r + lda kk] (N) or A[kk + lda r] (T); op(B)(kk, c) rows c: B[kk + ldb c] (N) or B[c + ldb kk] (T)
     const int64_t a_sr = transA ? lda : 1, a_sk = transA ? 1 : lda;
     const int64_t b_sr = transB ? 1 : ldb, b_sk = transB ? ldb : 1;
-    // scratch: exponents of both operands and the digit planes of one K slab
-    const size_t exp_bytes = round_up(sizeof(int) * (size_t)(Mp + Np), 256);
-    // the digit planes of K slabs of whole 16384-wide chunks, at most ~4 GB of them at a time (a
-    // 21 GB operand would otherwise need 18 GB of planes at once); each slab's launch adds its chunks
-    // to C in the order one launch over all K would, so the result does not depend on the slabs
-    const int64_t per_chunk = (int64_t)digits * std::max<int64_t>(OBM, (pa ? 0 : Mp) + (pb ? 0 : Np)) * OK_CHUNK;
-    int64_t budget = 4ll << 30;
-    if (const char *mb = std::getenv("CCSD_GPU_DIGIT_SLAB_MB")) budget = std::max<int64_t>(1, std::atoll(mb)) << 20;
-    const int64_t chunks_per_slab = std::max<int64_t>(1, budget / per_chunk);
-    const int64_t kslab = std::min<int64_t>(round_up(k, OBK), chunks_per_slab * OK_CHUNK);
-    const size_t a_bytes = pa ? 0 : round_up((size_t)digits * Mp * kslab, (size_t)1024);
-    const size_t b_bytes = pb ? 0 : (size_t)digits * Np * kslab;
-    const size_t need = exp_bytes + a_bytes + b_bytes;
-    DBuf local;
-    DBuf *arena = ex.digit_arena ? ex.digit_arena : &local;
-    if (arena->bytes() < need) {
-        arena->release();
-        arena->alloc(need, ex.stream);
-    }
-    uint8_t *base = arena->as<uint8_t>();
-    int *ea = reinterpret_cast<int *>(base), *eb = ea + Mp;
-    int8_t *da = reinterpret_cast<int8_t *>(base + exp_bytes), *db = da + a_bytes;
-    // a prepared operand brings its exponents and the digit planes of all of K (no conversion here)
-    if (pa) ea = pa->buf.as<int>();
-    else row_exponents(ex, A, a_sr, a_sk, m, k, Mp, ea);
-    if (pb) eb = pb->buf.as<int>();
-    else row_exponents(ex, B, b_sr, b_sk, n, k, Np, eb);
-    auto kernel = digits == 7 ? ozaki_gemm_kernel<7> : digits == 6 ? ozaki_gemm_kernel<6>
-                : digits == 5 ? ozaki_gemm_kernel<5> : digits == 4 ? ozaki_gemm_kernel<4>
-                : digits == 3 ? ozaki_gemm_kernel<3> : ozaki_gemm_kernel<2>;
-    auto pkernel = digits == 7 ? ozaki_pair_kernel<7> : digits == 6 ? ozaki_pair_kernel<6>
-                 : digits == 5 ? ozaki_pair_kernel<5> : digits == 4 ? ozaki_pair_kernel<4>
-                 : digits == 3 ? ozaki_pair_kernel<3> : ozaki_pair_kernel<2>;
-    // CTA pairs where 256-row pair tiles pad op(A) no further than 128-row tiles do (10240^3 with 6
-    // digits: 18.47 against 18.72 ms; a 528-row operand would run a third of its pair rows empty);
+    // CTA pairs for every op(A) of more than one 128-row tile: a 256 x 256 pair tile stages half the bytes per
+    // product that four 128 x 128 tiles do, so that even a pair tile half empty costs no more than they.
     // CCSD_GPU_PAIR_DIGITS=0 keeps single CTAs
     static const bool pairs_on = [] {
         const char *e = std::getenv("CCSD_GPU_PAIR_DIGITS");
         return !(e && e[0] == '0');
     }();
-    const bool pair = pairs_on && m >= 2 * OBM && round_up(m, (int64_t)(2 * OBM)) == Mp;
+    const bool pair = pairs_on && m > OBM;
+    auto kernel = digits == 7 ? ozaki_gemm_kernel<7> : digits == 6 ? ozaki_gemm_kernel<6>
+                : digits == 5 ? ozaki_gemm_kernel<5> : digits == 4 ? ozaki_gemm_kernel<4>
+                : digits == 3 ? ozaki_gemm_kernel<3> : ozaki_gemm_kernel<2>;
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OSMEM));
-    const int psmem = digits == 7 ? PairLayout<7>::SMEM : digits == 6 ? PairLayout<6>::SMEM
-                    : digits == 5 ? PairLayout<5>::SMEM : digits == 4 ? PairLayout<4>::SMEM
-                    : digits == 3 ? PairLayout<3>::SMEM : PairLayout<2>::SMEM;
-    CU_CHECK(cudaFuncSetAttribute(pkernel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
+    CU_CHECK(cudaFuncSetAttribute(ozaki_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WSMEM));
     const int nsm = num_sms();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -816,8 +927,8 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(OTHREADS);
-    cfg.dynamicSmemBytes = psmem;
+    cfg.blockDim = dim3(WTHREADS);
+    cfg.dynamicSmemBytes = WSMEM;
     cfg.stream = ex.stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -830,11 +941,43 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
         if (mp == 0) {
             cfg.gridDim = dim3((unsigned)(2 * (nsm / 2)));
             int n = 0;
-            CU_CHECK(cudaOccupancyMaxActiveClusters(&n, pkernel, &cfg));
+            CU_CHECK(cudaOccupancyMaxActiveClusters(&n, ozaki_pair_kernel, &cfg));
             mp = std::max(1, n);
         }
         max_pairs = mp;
     }
+    // scratch: exponents of both operands and the digit planes of one K slab
+    const size_t exp_bytes = round_up(sizeof(int) * (size_t)(Mp + Np), 256);
+    // the digit planes of K slabs of whole 16384-wide chunks, at most ~4 GB of them at a time (a
+    // 21 GB operand would otherwise need 18 GB of planes at once); each slab's launch adds its chunks
+    // to C in the order one launch over all K would, so the result does not depend on the slabs
+    const int64_t per_chunk = (int64_t)digits * std::max<int64_t>(OBM, (pa ? 0 : Mp) + (pb ? 0 : Np)) * OK_CHUNK;
+    int64_t budget = 4ll << 30;
+    if (const char *mb = std::getenv("CCSD_GPU_DIGIT_SLAB_MB")) budget = std::max<int64_t>(1, std::atoll(mb)) << 20;
+    const int64_t chunks_per_slab = std::max<int64_t>(1, budget / per_chunk);
+    const int64_t kslab = std::min<int64_t>(round_up(k, OBK), chunks_per_slab * OK_CHUNK);
+    const size_t a_bytes = pa ? 0 : round_up((size_t)digits * Mp * kslab, (size_t)1024);
+    const size_t b_bytes = pb ? 0 : (size_t)digits * Np * kslab;
+    // the pair kernel's partial sums, a 128 x 256 block per CTA
+    const size_t digit_bytes = round_up(a_bytes + b_bytes, (size_t)256);
+    const size_t need = exp_bytes + digit_bytes + (pair ? sizeof(double) * OBM * WBN * (size_t)(2 * max_pairs) : 0);
+    DBuf local;
+    DBuf *arena = ex.digit_arena ? ex.digit_arena : &local;
+    if (arena->bytes() < need) {
+        arena->release();
+        arena->alloc(need, ex.stream);
+    }
+    uint8_t *base = arena->as<uint8_t>();
+    int *ea = reinterpret_cast<int *>(base), *eb = ea + Mp;
+    int8_t *da = reinterpret_cast<int8_t *>(base + exp_bytes), *db = da + a_bytes;
+    double *scratch = reinterpret_cast<double *>(base + exp_bytes + digit_bytes);
+    // a prepared operand brings its exponents and the digit planes of all of K (no conversion here)
+    if (pa) ea = pa->buf.as<int>();
+    else row_exponents(ex, A, a_sr, a_sk, m, k, Mp, ea);
+    if (pb) eb = pb->buf.as<int>();
+    else row_exponents(ex, B, b_sr, b_sk, n, k, Np, eb);
+    const int64_t num_mt = pair ? round_up(m, (int64_t)(2 * OBM)) / (2 * OBM) : Mp / OBM;
+    const int bn = pair ? pair_n_tile(num_mt, n, digits, max_pairs) : OBN;
     for (int64_t k0 = 0; k0 < k; k0 += kslab) {
         const int64_t kk = std::min(kslab, k - k0), Kp = round_up(kk, OBK);
         if (!pa) slab_digits(ex, A + k0 * a_sk, a_sr, a_sk, m, kk, Mp, Kp, digits, ea, da);
@@ -844,12 +987,13 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
         CUtensorMap ta = pa ? make_i8_map(pa->digits_base() + k0, Mp, Kp, pa->Rp * pa->Kp, digits, OBM, pa->Kp)
                             : make_i8_map(da, Mp, Kp, Mp * Kp, digits);
         CUtensorMap tb = pb ? make_i8_map(pb->digits_base() + k0, Np, Kp, pb->Rp * pb->Kp, digits,
-                                          pair ? OBN / 2 : OBN, pb->Kp)
-                            : make_i8_map(db, Np, Kp, Np * Kp, digits, pair ? OBN / 2 : OBN);
+                                          pair ? bn / 2 : OBN, pb->Kp)
+                            : make_i8_map(db, Np, Kp, Np * Kp, digits, pair ? bn / 2 : OBN);
         OzMap map{};
         map.bm = pair ? 2 * OBM : OBM;
-        map.num_mt = (int)(pair ? round_up(Mp, (int64_t)(2 * OBM)) / (2 * OBM) : Mp / OBM);
-        map.num_nt = (int)(Np / OBN);
+        map.bn = bn;
+        map.num_mt = (int)num_mt;
+        map.num_nt = (int)((n + bn - 1) / bn);
         // raster groups of 2048 rows: their A digit panels (2048 x K x digits bytes) stay in L2 while
         // the group's N tiles stream past
         map.group_m = std::min(map.num_mt, pair ? 8 : 16);
@@ -878,7 +1022,7 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
         }
         if (pair) {
             cfg.gridDim = dim3((unsigned)(2 * grid));
-            CU_CHECK(cudaLaunchKernelEx(&cfg, pkernel, ta, tb, map, num_tiles));
+            CU_CHECK(cudaLaunchKernelEx(&cfg, ozaki_pair_kernel, ta, tb, map, num_tiles, scratch));
         } else {
             kernel<<<grid, OTHREADS, OSMEM, ex.stream>>>(ta, tb, map, num_tiles);
             CU_CHECK(cudaGetLastError());
