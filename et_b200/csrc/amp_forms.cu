@@ -170,9 +170,9 @@ __device__ __forceinline__ void put_planes(double x, int np, int64_t plane, __nv
 // (c, i), t_cjdi along c in row (d, i), turned in shared memory; both forms are stored along d.  Bound by
 // HBM: n_t2 read, the forms written; each thread of the element-wise version found its four indices by two
 // square roots and read two elements whose neighbours lay a packed row apart.  bf16 planes at o=32, v=320
-// 0.54 ms (1.2 TB/s).
+// 0.34 ms (1.9 TB/s), 0.54 without MIN_BLOCKS.
 template <bool PLANES>
-__global__ void __launch_bounds__(TILE * ROWS)
+__global__ void __launch_bounds__(TILE * ROWS, MIN_BLOCKS)
 tpm_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec, TpmOut o) {
     __shared__ double s[TILE][TILE + 1];   // t_cjdi of (c0 + x, d0 + r) at [r][x]
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -215,8 +215,9 @@ tpm_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec
 // An occupied pair i >= j and a 32 x 32 tile of (a, b), a >= b: w+- are read along b, Omega_aibj is added
 // to along b in its packed row (a, i), Omega_ajbi along a in row (b, i) through shared memory.  Bound by
 // HBM: w+- read, n_t2 read and written.  The element-wise version ran along ij, so that neighbouring threads
-// updated packed rows far apart: 1.37 ms at o=32, v=320; so 0.54 (2.3 TB/s).
-__global__ void __launch_bounds__(TILE * ROWS)
+// updated packed rows far apart: 1.37 ms at o=32, v=320; so 0.34 (3.7 TB/s), 0.54
+// without MIN_BLOCKS.
+__global__ void __launch_bounds__(TILE * ROWS, MIN_BLOCKS)
 add_omega_pm_kernel(double *__restrict__ om2, const double *__restrict__ wp, const double *__restrict__ wm, int no, int nv,
                     int64_t nvec, int a0, int a1, int64_t ldwp, int64_t ldwm) {
     __shared__ double s[TILE][TILE + 1];   // the Omega_ajbi share of (a, b) at [a][b]
