@@ -15,55 +15,6 @@
 
 namespace ccsd {
 
-namespace {
-
-#define GRID_STRIDE(i, total) \
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (total); i += (int64_t)gridDim.x * blockDim.x)
-
-inline int grid_for(int64_t total, int block) {
-    int64_t g = (total + block - 1) / block;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(g, 148 * 64));
-}
-
-// [t1 | t2] columns <-> separate (nt1 x n) and (nt2 x n) arrays, with the doubles diagonal scaled
-__global__ void split_amp_kernel(const double *__restrict__ x, int64_t nt1, int64_t nov, int64_t nvec, double diag,
-                                 double *__restrict__ x1, double *__restrict__ x2) {
-    const int64_t nt2 = nov * (nov + 1) / 2, namp = nt1 + nt2;
-    GRID_STRIDE(idx, namp * nvec) {
-        int64_t n = idx / namp, k = idx - n * namp;
-        double v = x[idx];
-        if (k < nt1) x1[n * nt1 + k] = v;
-        else {
-            int64_t p = k - nt1;
-            int64_t M = (int64_t)((sqrt(8.0 * (double)p + 1.0) - 1.0) * 0.5);
-            while (M * (M + 1) / 2 > p) M--;
-            while ((M + 1) * (M + 2) / 2 <= p) M++;
-            if (p - M * (M + 1) / 2 == M) v *= diag;
-            x2[n * nt2 + p] = v;
-        }
-    }
-}
-
-__global__ void join_amp_kernel(const double *__restrict__ x1, const double *__restrict__ x2, int64_t nt1, int64_t nov,
-                                int64_t nvec, double diag, double *__restrict__ x) {
-    const int64_t nt2 = nov * (nov + 1) / 2, namp = nt1 + nt2;
-    GRID_STRIDE(idx, namp * nvec) {
-        int64_t n = idx / namp, k = idx - n * namp;
-        if (k < nt1) x[idx] = x1[n * nt1 + k];
-        else {
-            int64_t p = k - nt1;
-            int64_t M = (int64_t)((sqrt(8.0 * (double)p + 1.0) - 1.0) * 0.5);
-            while (M * (M + 1) / 2 > p) M--;
-            while ((M + 1) * (M + 2) / 2 <= p) M++;
-            double v = x2[n * nt2 + p];
-            if (p - M * (M + 1) / 2 == M) v *= diag;
-            x[idx] = v;
-        }
-    }
-}
-
-}  // namespace
-
 // ---------------------------------------------------------------------------
 // Omega on the graph
 // ---------------------------------------------------------------------------
@@ -181,7 +132,7 @@ OmegaNodes Context::record_omega(Graph &g, bool const_ovov, bool const_t1) {
     {
         // omega_doubles_c1 (:207-258)
         TermTimer tt(ex, "omega doubles c1");
-        g.contract(om1, "aibj,jb->ai", 1.0, u, F_ov, true);
+        g.contract(om1, "bjai,jb->ai", 1.0, u, F_ov, true);
     }
 
     // g_ldkc, shared below (FP64 cache unless the adjoint into L_ov is wanted)
@@ -554,14 +505,9 @@ void Context::jacobian(int64_t nvec, const double *c, double *rho) {
     std::unique_ptr<Graph> local;
     OmegaNodes n;
     Graph &g = transform_graph(local, n);
-    DBuf s1 = dalloc(nt1 * nvec, ex.stream), s2 = dalloc(nt2 * nvec, ex.stream);
-    split_amp_kernel<<<grid_for(namp * nvec, 256), 256, 0, ex.stream>>>(c, nt1, nov, nvec, 2.0, s1.d(), s2.d());
-    ex.launches++;
-    DBuf r1 = dalloc(nt1 * nvec, ex.stream), r2 = dalloc(nt2 * nvec, ex.stream);
-    g.jvp({n.t1, n.t2}, {s1.d(), s2.d()}, (int)nvec, {n.om1, n.om2}, {r1.d(), r2.d()});
-    join_amp_kernel<<<grid_for(namp * nvec, 256), 256, 0, ex.stream>>>(r1.d(), r2.d(), nt1, nov, nvec, 1.0, rho);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
+    // the diagonal factor D = 2 goes on the copy of c that the tangents start from
+    g.jvp({n.t1, n.t2}, {{c, namp}, {c + nt1, namp}}, (int)nvec, {n.om1, n.om2}, {{rho, namp}, {rho + nt1, namp}},
+          [&] { scale_doubles_diag(ex, g.tangent(n.t2, (int)nvec), nov, nvec, nt2, 2.0); });
     g.clear_derivatives();
     CU_CHECK(cudaStreamSynchronize(ex.stream));
     check_gemm();
@@ -575,14 +521,8 @@ void Context::jacobian_transpose(int64_t nvec, const double *b, double *sigma) {
     std::unique_ptr<Graph> local;
     OmegaNodes n;
     Graph &g = transform_graph(local, n);
-    DBuf s1 = dalloc(nt1 * nvec, ex.stream), s2 = dalloc(nt2 * nvec, ex.stream);
-    split_amp_kernel<<<grid_for(namp * nvec, 256), 256, 0, ex.stream>>>(b, nt1, nov, nvec, 1.0, s1.d(), s2.d());
-    ex.launches++;
-    DBuf r1 = dalloc(nt1 * nvec, ex.stream), r2 = dalloc(nt2 * nvec, ex.stream);
-    g.vjp({n.om1, n.om2}, {s1.d(), s2.d()}, (int)nvec, {n.t1, n.t2}, {r1.d(), r2.d()});
-    join_amp_kernel<<<grid_for(namp * nvec, 256), 256, 0, ex.stream>>>(r1.d(), r2.d(), nt1, nov, nvec, 2.0, sigma);
-    ex.launches++;
-    CU_CHECK(cudaGetLastError());
+    g.vjp({n.om1, n.om2}, {{b, namp}, {b + nt1, namp}}, (int)nvec, {n.t1, n.t2}, {{sigma, namp}, {sigma + nt1, namp}});
+    scale_doubles_diag(ex, sigma + nt1, nov, nvec, namp, 2.0);
     g.clear_derivatives();
     CU_CHECK(cudaStreamSynchronize(ex.stream));
     check_gemm();
@@ -594,13 +534,13 @@ void Context::adjoint(const double *b, double *dt, double *dL, double *dh) {
     REQUIRE(have_t, CCSD_GPU_ESTATE, "amplitudes not set");
     Graph g(ex);
     OmegaNodes n = record_omega(g, dL == nullptr);
-    DBuf s1 = dalloc(nt1, ex.stream), s2 = dalloc(nt2, ex.stream);
-    split_amp_kernel<<<grid_for(namp, 256), 256, 0, ex.stream>>>(b, nt1, nov, 1, 1.0, s1.d(), s2.d());
-    ex.launches++;
     std::vector<int> ins = {n.t1, n.t2};
     std::vector<DBuf> outs;
-    outs.push_back(dalloc(nt1, ex.stream));
-    outs.push_back(dalloc(nt2, ex.stream));
+    DBuf dt_own;
+    if (!dt) {
+        dt_own = dalloc(namp, ex.stream);
+        dt = dt_own.d();
+    }
     const bool wantL = dL != nullptr, wanth = dh != nullptr;
     if (wantL)
         for (int node : {n.L_oo, n.L_ov, n.L_vo, n.L_vv}) {
@@ -612,14 +552,10 @@ void Context::adjoint(const double *b, double *dt, double *dL, double *dh) {
             ins.push_back(node);
             outs.push_back(dalloc(g.node(node).size, ex.stream));
         }
-    std::vector<double *> res;
-    for (auto &o : outs) res.push_back(o.d());
-    g.vjp({n.om1, n.om2}, {s1.d(), s2.d()}, 1, ins, res);
-    if (dt) {
-        join_amp_kernel<<<grid_for(namp, 256), 256, 0, ex.stream>>>(outs[0].d(), outs[1].d(), nt1, nov, 1, 1.0, dt);
-        ex.launches++;
-    }
-    size_t k = 2;
+    std::vector<Graph::Out> res = {{dt, namp}, {dt + nt1, namp}};
+    for (auto &o : outs) res.push_back({o.d(), 0});
+    g.vjp({n.om1, n.om2}, {{b, namp}, {b + nt1, namp}}, 1, ins, res);
+    size_t k = 0;
     auto scatter = [&](double *full, int64_t ld, int64_t p0, int64_t q0, int64_t np, int64_t nq, const double *blk,
                        int64_t inner) {
         // full[(inner) x (p0+p) x (q0+q)] <- blk[inner x p x q]

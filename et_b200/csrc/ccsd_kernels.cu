@@ -300,9 +300,10 @@ __global__ void qn_precondition_kernel(double *__restrict__ v, const double *__r
     }
 }
 
-__global__ void scale_doubles_diag_kernel(double *__restrict__ x, int64_t nov, int64_t nt1, double f) {
-    GRID_STRIDE(M, nov) {
-        x[nt1 + M * (M + 1) / 2 + M] *= f;
+__global__ void scale_doubles_diag_kernel(double *__restrict__ x, int64_t nov, int64_t nvec, int64_t ld, double f) {
+    GRID_STRIDE(idx, nov * nvec) {
+        const int64_t n = idx / nov, M = idx - n * nov;
+        x[n * ld + M * (M + 1) / 2 + M] *= f;
     }
 }
 
@@ -466,8 +467,8 @@ void qn_precondition(Exec &ex, double *v, const double *epsdiff, int64_t n, int6
     CU_CHECK(cudaGetLastError());
 }
 
-void scale_doubles_diag(Exec &ex, double *x, int64_t nov, int64_t nt1, double f) {
-    scale_doubles_diag_kernel<<<grid_for(nov, 256), 256, 0, ex.stream>>>(x, nov, nt1, f);
+void scale_doubles_diag(Exec &ex, double *x, int64_t nov, int64_t nvec, int64_t ld, double f) {
+    scale_doubles_diag_kernel<<<grid_for(nov * nvec, 256), 256, 0, ex.stream>>>(x, nov, nvec, ld, f);
     ex.launches++;
     CU_CHECK(cudaGetLastError());
 }

@@ -36,7 +36,8 @@ void trace_oo(Exec &ex, const double *L_oo, int64_t nJ, int64_t no, double *X);
 void qn_update(Exec &ex, double *omega, const double *epsdiff, double *t, int64_t n, int64_t nt1);
 // v <- the quasi-Newton image of the residual v (-v / eps, doubles diagonal x2), t untouched
 void qn_precondition(Exec &ex, double *v, const double *epsdiff, int64_t n, int64_t nt1);
-void scale_doubles_diag(Exec &ex, double *x, int64_t nov, int64_t nt1, double f);
+// the diagonal of nvec packed doubles vectors (stride ld) times f
+void scale_doubles_diag(Exec &ex, double *x, int64_t nov, int64_t nvec, int64_t ld, double f);
 void diis_solve(Exec &ex, double *Gslot, int maxdim, const double *dots, int new_slot, const DiisOrder &order,
                 double *w, int *status);
 void extrapolate(Exec &ex, const double *const *recs, const double *w, int nrec, int64_t n, double *x);

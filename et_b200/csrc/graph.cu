@@ -327,16 +327,36 @@ void Graph::clear_derivatives() {
     }
 }
 
-void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *> &seeds, int nvec,
-                const std::vector<int> &outputs, const std::vector<double *> &results) {
+void Graph::copy_columns(double *dst, int64_t ldd, const double *src, int64_t lds, int64_t size, int nvec) {
+    if (size == 0) return;
+    const size_t eb = sizeof(double);
+    if (nvec == 1 || (ldd == size && lds == size))
+        CU_CHECK(cudaMemcpyAsync(dst, src, eb * size * nvec, cudaMemcpyDeviceToDevice, ex_.stream));
+    else if (eb * (size_t)std::max(ldd, lds) < ((size_t)1 << 31))   // the pitch of a 2-D copy is limited
+        CU_CHECK(cudaMemcpy2DAsync(dst, eb * ldd, src, eb * lds, eb * size, nvec, cudaMemcpyDeviceToDevice, ex_.stream));
+    else
+        for (int k = 0; k < nvec; k++) copy_columns(dst + k * ldd, ldd, src + k * lds, lds, size, 1);
+}
+
+void Graph::store_result(int i, int nvec, bool adj, const Out &out) {
+    const GNode &n = nodes_[i];
+    const DBuf &buf = adj ? n.adj : n.tan;
+    if (n.active && buf && !(adj ? n.adj_zero : n.tan_zero))
+        copy_columns(out.p, out.ld, buf.d(), n.size, n.size, nvec);
+    else
+        for (int k = 0; k < nvec; k++) fill(ex_, out.p + k * out.ld, n.size, 0.0);
+}
+
+void Graph::jvp(const std::vector<int> &inputs, const std::vector<In> &seeds, int nvec, const std::vector<int> &outputs,
+                const std::vector<Out> &results, const std::function<void()> &seeded) {
     clear_derivatives();
     mark_active(inputs);
     for (size_t k = 0; k < inputs.size(); k++) {
         double *t = derivative(inputs[k], nvec, false);
         nodes_[inputs[k]].tan_zero = false;
-        CU_CHECK(cudaMemcpyAsync(t, seeds[k], sizeof(double) * nodes_[inputs[k]].size * nvec,
-                                 cudaMemcpyDeviceToDevice, ex_.stream));
+        copy_columns(t, nodes_[inputs[k]].size, seeds[k].p, seeds[k].ld, nodes_[inputs[k]].size, nvec);
     }
+    seeded();
     // the tangents that the outputs depend on: an op feeding only others is skipped
     std::vector<char> needed(nodes_.size(), 0);
     for (int i : outputs) needed[i] = 1;
@@ -413,24 +433,17 @@ void Graph::jvp(const std::vector<int> &inputs, const std::vector<const double *
         }
         CU_CHECK(cudaGetLastError());
     }
-    for (size_t k = 0; k < outputs.size(); k++) {
-        const GNode &n = nodes_[outputs[k]];
-        if (n.active && n.tan && !n.tan_zero)
-            CU_CHECK(cudaMemcpyAsync(results[k], n.tan.d(), sizeof(double) * n.size * nvec, cudaMemcpyDeviceToDevice,
-                                     ex_.stream));
-        else
-            fill(ex_, results[k], n.size * nvec, 0.0);
-    }
+    for (size_t k = 0; k < outputs.size(); k++) store_result(outputs[k], nvec, false, results[k]);
 }
 
-void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double *> &seeds, int nvec,
-                const std::vector<int> &inputs, const std::vector<double *> &results) {
+void Graph::vjp(const std::vector<int> &outputs, const std::vector<In> &seeds, int nvec, const std::vector<int> &inputs,
+                const std::vector<Out> &results) {
     clear_derivatives();
     mark_active(inputs);
     for (size_t k = 0; k < outputs.size(); k++) {
         double beta;
         const TV a = twrite(outputs[k], nvec, true, &beta);
-        axpby(ex_, nodes_[outputs[k]].size * nvec, 1.0, seeds[k], beta, a.p);
+        copy_columns(a.p, nodes_[outputs[k]].size, seeds[k].p, seeds[k].ld, nodes_[outputs[k]].size, nvec);
     }
     double beta = 1.0;
     for (int oi = (int)ops_.size() - 1; oi >= 0; --oi) {
@@ -504,14 +517,7 @@ void Graph::vjp(const std::vector<int> &outputs, const std::vector<const double 
         }
         CU_CHECK(cudaGetLastError());
     }
-    for (size_t k = 0; k < inputs.size(); k++) {
-        const GNode &n = nodes_[inputs[k]];
-        if (n.adj && !n.adj_zero)
-            CU_CHECK(cudaMemcpyAsync(results[k], n.adj.d(), sizeof(double) * n.size * nvec, cudaMemcpyDeviceToDevice,
-                                     ex_.stream));
-        else
-            fill(ex_, results[k], n.size * nvec, 0.0);
-    }
+    for (size_t k = 0; k < inputs.size(); k++) store_result(inputs[k], nvec, true, results[k]);
 }
 
 }  // namespace ccsd
