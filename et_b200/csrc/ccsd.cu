@@ -305,10 +305,10 @@ void Context::g_pairs_const() {
 double Context::energy() {
     Prec keep = ex.prec;
     ex.prec = Prec::FP64;
-    const double *gov_p = g_ovov_const();
+    g_pairs_const();
     {
         TermTimer tt(ex, "Calculate energy");
-        energy_reduce(ex, t.d(), t.d() + nt1, gov_p, no, nv, e_hf, scal.d());
+        energy_reduce(ex, t.d(), t.d() + nt1, hov.d(), nov, e_hf, scal.d());
     }
     ex.prec = keep;
     double e;
@@ -861,24 +861,32 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
         return r;
     }
     // t as [(c, d), (i, j)], the product [(k, p), (i, j)]
-    DBuf TT = dalloc(oo * nv2, s), W = dalloc(rows * oo, s);
-    {
-        TV dst = tv(TT.d(), {nv, no, nv, no});
-        dst.s[1] = nv2;        // i
-        dst.s[2] = nv;         // d
-        dst.s[3] = nv2 * no;   // j
-        permute_add(ex, 1.0, tv(tf, {nv, no, nv, no}), 0.0, dst);
-    }
+    DBuf W = dalloc(rows * oo, s);
     if (ex.prec == Prec::MIXED) {
         ovvv_pairs();
         const int64_t Kq = tc_pad_k(nv2), rows_T = tc_pad_rows_b(oo);
         DBuf TS(sizeof(__nv_bfloat16) * ex.planes * rows_T * Kq, s);
-        split_rows(ex, TT.d(), nv2, 1, oo, nv2, rows_T, Kq, TS.as<__nv_bfloat16>());
+        SplitView v{};
+        v.p = tf;
+        v.nr = v.nk = 2;
+        v.rn[0] = v.rn[1] = no;   // i, j
+        v.rs[0] = nv;
+        v.rs[1] = nov * nv;
+        v.kn[0] = v.kn[1] = nv;   // c, d
+        v.ks[0] = 1;
+        v.ks[1] = nov;
+        split_tensor(ex, v, oo, nv2, rows_T, Kq, TS.as<__nv_bfloat16>());
         tc_gemm_f64_tuned(ex, ybuf.as<__nv_bfloat16>(), tc_pad_rows_a(rows), TS.as<__nv_bfloat16>(), rows_T, Kq, rows, oo,
                           nv2, 1.0, 0.0, W.d(), rows, 0);
         ex.flops += 2.0 * double(rows) * double(oo) * double(nv2);
     } else {
         f64_integrals();
+        DBuf TT = dalloc(oo * nv2, s);
+        TV dst = tv(TT.d(), {nv, no, nv, no});
+        dst.s[1] = nv2;        // i
+        dst.s[2] = nv;         // d
+        dst.s[3] = nv2 * no;   // j
+        permute_add(ex, 1.0, tv(tf, {nv, no, nv, no}), 0.0, dst);
         const double fl = 2.0 * double(rows) * double(oo) * double(nv2);
         if (gemm_takes_digits(ex, rows, oo, nv2, fl) && f64_ovvv_planes(ex.fp64_digits)) {
             ozaki_gemm(ex, false, false, rows, oo, nv2, 1.0, f64_ovvv.d(), rows, TT.d(), nv2, 0.0, W.d(), rows,

@@ -28,8 +28,9 @@ void density_energy_part(Exec &ex, double *D, const double *t1, int64_t no, int6
 void construct_eta(Exec &ex, const double *F, const double *g_ovov, int64_t no, int64_t nv, double *eta);
 void multiplier_guess(Exec &ex, const double *t, int64_t no, int64_t nv, double *out);
 
-void energy_reduce(Exec &ex, const double *t1, const double *t2, const double *g_ovov, int64_t no, int64_t nv,
-                   double add, double *d_out);
+// *d_out = add + E_corr from packed amplitudes and H[a,i,b,j] = g_iajb - 1/2 g_ibja (calculate_energy_ccsd)
+void energy_reduce(Exec &ex, const double *t1, const double *t2, const double *H, int64_t nov, double add,
+                   double *d_out);
 void orbital_differences(Exec &ex, const double *eps, int64_t no, int64_t nv, double *out);
 void mp2_amplitudes(Exec &ex, const double *g_vovo, const double *epsdiff, int64_t nov, double *t2);
 void trace_oo(Exec &ex, const double *L_oo, int64_t nJ, int64_t no, double *X);

@@ -1385,6 +1385,10 @@ void split_rows(Exec &ex, const double *src, int64_t sr, int64_t sk, int64_t R, 
     split(ex, src, sr, sk, R, K, Rp, Kp, check_planes(ex.planes), out);
 }
 
+void split_tensor(Exec &ex, const SplitView &src, int64_t R, int64_t K, int64_t Rp, int64_t Kp, __nv_bfloat16 *out) {
+    split_view(ex, src, R, K, Rp, Kp, check_planes(ex.planes), out);
+}
+
 void tc_gemm_f64(Exec &ex, const __nv_bfloat16 *A, int64_t Mp, const __nv_bfloat16 *B, int64_t Np, int64_t Kp,
                  int64_t m, int64_t n, int64_t k_true, double alpha, double beta, double *C, int64_t ldc,
                  int splits) {

@@ -76,6 +76,8 @@ int64_t tc_pad_k(int64_t k);
 void split_rows(Exec &ex, const double *src, int64_t sr, int64_t sk, int64_t R, int64_t K, int64_t Rp, int64_t Kp,
                 __nv_bfloat16 *out);
 
+// the same from a tensor's own layout
+void split_tensor(Exec &ex, const SplitView &src, int64_t R, int64_t K, int64_t Rp, int64_t Kp, __nv_bfloat16 *out);
 // Tensor-core GEMM on pre-split operands A [2][Mp][Kp], B [2][Np][Kp]:
 // C (m x n, col-major, FP64) = alpha A B^T + beta C.  splits > 1 divides K into that many
 // deterministic partial products summed afterwards; 0 chooses the count from the tile waves.
