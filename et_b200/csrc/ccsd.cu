@@ -364,33 +364,53 @@ void Context::ladder(const double *Lvv, const double *t2, double *om2, int64_t n
         dst.s[2] = nJ;        // c
         permute_add(ex, 1.0, src, 0.0, dst);
     }
+    // the g+- of all pairs at once where they take no more than 3 GB: G is then formed block by block but
+    // contracted in one product per sign
+    const bool all_pairs = ladder_batch <= 0 && 8.0 * (double(nvp) * nvp + double(nvm) * nvm) <= 3.0e9;
     // batch length over a: keep G + g+- + w+- within the budget
     int64_t nA = ladder_batch;
-    if (nA <= 0) {
+    if (all_pairs) {
+        nA = pair_block(3.0e9);
+    } else if (nA <= 0) {
         const double budget = 6.0e9;   // bytes
         double per_a = 8.0 * (double)nv * nv * nv + 16.0 * (double)nvp * nv + 16.0 * (double)np * nv;
         nA = std::max<int64_t>(1, std::min<int64_t>(nv, (int64_t)(budget / per_a)));
     }
-    int64_t maxab = 0;
-    for (int64_t a0 = 0; a0 < nv; a0 += nA) {
+    auto pairs_p = [](int64_t a) { return a * (a + 1) / 2; };
+    auto pairs_m = [](int64_t a) { return a * (a - 1) / 2; };
+    int64_t maxab = all_pairs ? nvp : 0;
+    for (int64_t a0 = 0; a0 < nv && !all_pairs; a0 += nA) {
         int64_t a1 = std::min(nv, a0 + nA);
-        maxab = std::max(maxab, a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2);
+        maxab = std::max(maxab, pairs_p(a1) - pairs_p(a0));
     }
     DBuf G = dalloc(nv * nA * nv * nv, s);
     DBuf gp = dalloc(nvp * maxab, s), gm = dalloc(std::max<int64_t>(nvm * maxab, 1), s);
     DBuf wp = dalloc(np * maxab, s), wm = dalloc(std::max<int64_t>(nm * maxab, 1), s);
+    // the pairs a in [a0, a1) from their g+-
+    auto contract_pairs = [&](int64_t a0, int64_t a1) {
+        const int64_t nabp = pairs_p(a1) - pairs_p(a0), nabm = pairs_m(a1) - pairs_m(a0);
+        gemm(ex, true, false, nabp, np, nvp, 0.5, gp.d(), nvp, tp.d(), nvp, 0.0, wp.d(), nabp);
+        if (nom > 0 && nabm > 0) gemm(ex, true, false, nabm, nm, nvm, 0.5, gm.d(), nvm, tm.d(), nvm, 0.0, wm.d(), nabm);
+        add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, nvec, a0, a1, nabp, nabm);
+    };
     for (int64_t a0 = 0; a0 < nv; a0 += nA) {
         int64_t a1 = std::min(nv, a0 + nA);
         int64_t M = nv * (a1 - a0), N = nv * a1;
         // G[(c,a),(d,b)] = sum_J L_ac L_bd   (eri_t1%get('vvvv') / get_packed('vv')), once for all vectors
         gemm(ex, true, false, M, N, nJ, 1.0, LT.d() + nJ * nv * a0, nJ, LT.d(), nJ, 0.0, G.d(), M);
-        form_gpm(ex, G.d(), M, gp.d(), gm.d(), nv, a0, a1);
-        int64_t nabp = a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2;
-        int64_t nabm = a1 * (a1 - 1) / 2 - a0 * (a0 - 1) / 2;
-        gemm(ex, true, false, nabp, np, nvp, 0.5, gp.d(), nvp, tp.d(), nvp, 0.0, wp.d(), nabp);
-        if (nom > 0 && nabm > 0) gemm(ex, true, false, nabm, nm, nvm, 0.5, gm.d(), nvm, tm.d(), nvm, 0.0, wm.d(), nabm);
-        add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, nvec, a0, a1, nabp, nabm);
+        const int64_t col_p = all_pairs ? pairs_p(a0) : 0, col_m = all_pairs ? pairs_m(a0) : 0;
+        form_gpm(ex, G.d(), M, gp.d() + nvp * col_p, gm.d() + nvm * col_m, nv, a0, a1);
+        if (!all_pairs) contract_pairs(a0, a1);
     }
+    if (all_pairs) contract_pairs(0, nv);
+}
+
+// Length of the blocks of a whose integrals g_acbd, b < a1, are formed in one product of at most `bytes`: only
+// b <= a is used, so one block over all of a forms twice what is needed and six blocks 1.17 times; shorter
+// blocks than 8 make thin products, and below n_v = 48 the launches cost more than the half saved.
+int64_t Context::pair_block(double bytes) const {
+    const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(nv, (int64_t)(bytes / (8.0 * nv * nv * nv))));
+    return nv < 48 ? fit : std::min<int64_t>(fit, std::max<int64_t>(8, (nv + 5) / 6));
 }
 
 void Context::set_precision(int32_t precision) {
@@ -495,8 +515,7 @@ void Context::ladder_pairs(const double *Lvv, bool untransformed) {
     __nv_bfloat16 *Pp = mbuf.as<__nv_bfloat16>(), *Pm = Pp + np * ps.plane_p();
     DBuf LT = lvv_jca(Lvv);
     // blocks of a whose G fits in about 2 GB
-    const int64_t nA = ladder_batch > 0 ? ladder_batch
-                                        : std::max<int64_t>(1, std::min<int64_t>(nv, (int64_t)(2.0e9 / (8.0 * nv * nv * nv))));
+    const int64_t nA = ladder_batch > 0 ? ladder_batch : pair_block(2.0e9);
     DBuf G = dalloc(nv * std::min(nA, nv) * nv * nv, s);
     for (int64_t a0 = 0; a0 < nv; a0 += nA)
         form_pair_planes(LT.d(), a0, std::min(nv, a0 + nA), G.d(), Pp, ps.rows_p, 0, Pm, ps.rows_m, 0);
@@ -752,7 +771,7 @@ void Context::f64_integrals() {
         dst.s[1] = nJ * nv;
         dst.s[2] = nJ;
         permute_add(ex, 1.0, tv(L_vv.d(), {nJ, nv, nv}), 0.0, dst);
-        const int64_t nA = std::max<int64_t>(1, std::min<int64_t>(nv, (int64_t)(4.0e9 / (8.0 * nv * nv * nv))));
+        const int64_t nA = pair_block(4.0e9);
         DBuf G = dalloc(nv * nA * nv * nv, s);
         for (int64_t a0 = 0; a0 < nv; a0 += nA) {
             const int64_t a1 = std::min(nv, a0 + nA), M = nv * (a1 - a0), N = nv * a1;

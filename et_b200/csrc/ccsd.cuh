@@ -177,6 +177,7 @@ struct Context {
     // n_t2); the integrals are formed once per call
     void ladder(const double *Lvv, const double *t2, double *om2, int64_t nvec = 1);
     void ladder_tc(const double *Lvv, const double *t2, double *om2, int64_t nvec, bool untransformed);
+    int64_t pair_block(double bytes) const;
     DBuf lvv_jca(const double *Lvv);
     void form_pair_planes(const double *LT, int64_t a0, int64_t a1, double *G, __nv_bfloat16 *Pp, int64_t rows_p,
                           int64_t rowp0, __nv_bfloat16 *Pm, int64_t rows_m, int64_t rowm0);
