@@ -732,7 +732,7 @@ void Context::ladder_t1_corrections(const double *t1, const LadderY &yq, double 
 
 // FP64 integrals of the untransformed vectors, resident while they fit in half of the free memory
 // (50 GB at o = 32, v = 320): the +/- ladder integrals of all pairs (eT's packing, formed block by
-// block exactly as the per-call ladder forms them) and g_kcbd.
+// block exactly as the per-call ladder forms them) and g_kcpd.
 bool Context::f64_resident() {
     if (!f64_resident_on) return false;
     if (f64_version == l_version) return true;

@@ -80,7 +80,7 @@ struct Context {
     int ybuf_fit_planes = 0;
     // FP64 residual with resident integrals of the untransformed vectors (when they fit): eT's +/-
     // ladder integrals g+ [v(v+1)/2 x v(v+1)/2] and g- [v(v-1)/2 x v(v-1)/2] for all pairs, and the
-    // ovvv block g_kcbd as [k, b, c, d]; valid for f64_version
+    // integrals g_kcpd as [k, p, c, d], p over the virtual and then the occupied orbitals; valid for f64_version
     DBuf f64_gp, f64_gm, f64_ovvv;
     int64_t f64_version = -1;
     int f64_fit = -1;               // residency decision for f64_fit_version

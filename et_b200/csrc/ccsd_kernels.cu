@@ -154,7 +154,7 @@ __global__ void multiplier_guess_kernel(const double *__restrict__ t, int64_t no
 // E_corr partial sums: sum_{ai,bj} (t_aibj + t_ai t_bj)(2 g_iajb - g_ibja) = 2 sum T H with H = g_iajb - g_ibja/2
 // in the pair layout of the amplitudes.  Both are symmetric in their pairs, so a packed row M of t2 meets the
 // first M + 1 elements of column M of H, both contiguous: t2 and half of H are read once, in rows M and
-// nov - 1 - M by turns so that the blocks' shares are equal.  Bound by HBM: 0.05 ms for o=24 v=192 (170 MB);
+// nov - 1 - M by turns so that the blocks' shares are equal.  Bound by HBM: 0.04 ms for o=24 v=192 (170 MB);
 // the sums over o x o sub-blocks of g_iajb, whose reads were o elements long, took 0.22 ms.
 __global__ void __launch_bounds__(256) energy_rows_kernel(const double *__restrict__ t1, const double *__restrict__ t2,
                                                           const double *__restrict__ H, int64_t nov,

@@ -24,90 +24,122 @@ struct PermArgs {
     int64_t so[MAXD];
 };
 
+// Index arithmetic in I: 32-bit divisions wherever the count of rows, tiles or elements allows, a third of the
+// 64-bit chain's time, which is what bounds these kernels on small tensors.
+template <class I>
+__device__ __forceinline__ void locate(const PermArgs &a, int first, I r, int64_t &oi, int64_t &oo) {
+#pragma unroll
+    for (int d = 0; d < MAXD; d++) {
+        if (d >= first && d < a.nd) {
+            const I n = (I)a.n[d], q = r / n, i = r - q * n;
+            r = q;
+            oi += (int64_t)i * a.si[d];
+            oo += (int64_t)i * a.so[d];
+        }
+    }
+}
+
 // One output element per thread; dims are ordered by output stride (dim 0 fastest).
+template <class I>
 __global__ void permute_simple_kernel(PermArgs a, int64_t total, double alpha, const double *__restrict__ in,
                                       double beta, double *__restrict__ out) {
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        int64_t r = idx, oi = 0, oo = 0;
-#pragma unroll
-        for (int d = 0; d < MAXD; d++) {
-            if (d < a.nd) {
-                int64_t q = r / a.n[d];
-                int64_t i = r - q * a.n[d];
-                r = q;
-                oi += i * a.si[d];
-                oo += i * a.so[d];
-            }
-        }
+        int64_t oi = 0, oo = 0;
+        locate<I>(a, 0, (I)idx, oi, oo);
         double v = alpha * in[oi];
         if (beta != 0.0) v += beta * out[oo];
         out[oo] = v;
     }
 }
 
-// Rows of the output-fastest dim (dim 0, at least 16 long): a warp takes one row, so the int64
-// div/mod chain that locates a row in the other dims runs once per row instead of once per element,
+// Rows of the output-fastest dim (dim 0, at least 16 long): a warp takes a row or a segment of a long one, so the division chain that locates it in the other dims runs once per row instead of once per element,
 // and both sides stream along dim 0 (this kernel serves permutations whose input-fastest dim is dim
-// 0 as well, or whose other dims are too short for the tiled transpose).
-__global__ void permute_rows_kernel(PermArgs a, int64_t nrows, double alpha, const double *__restrict__ in,
-                                    double beta, double *__restrict__ out) {
+// 0 as well, or whose other dims are too short for the tiled transpose).  Bound by HBM or, for rows of a few
+// hundred, by loads in flight: four per lane.
+template <class I>
+__global__ void __launch_bounds__(256) permute_rows_kernel(PermArgs a, int64_t nwork, int nseg, int seg, double alpha,
+                                                           const double *__restrict__ in, double beta,
+                                                           double *__restrict__ out) {
     const int64_t n0 = a.n[0], si0 = a.si[0], so0 = a.so[0];
-    for (int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; row < nrows;
-         row += (int64_t)gridDim.x * blockDim.y) {
-        int64_t r = row, oi = 0, oo = 0;
-#pragma unroll
-        for (int d = 1; d < MAXD; d++) {
-            if (d < a.nd) {
-                const int64_t q = r / a.n[d];
-                const int64_t i = r - q * a.n[d];
-                r = q;
-                oi += i * a.si[d];
-                oo += i * a.so[d];
-            }
+    for (int64_t w = (int64_t)blockIdx.x * 8 + threadIdx.y; w < nwork; w += (int64_t)gridDim.x * 8) {
+        I row = (I)w;
+        int64_t lo = 0, oi = 0, oo = 0;
+        if (nseg > 1) {
+            const I q = row / (I)nseg;
+            lo = (int64_t)(row - q * (I)nseg) * seg;
+            row = q;
         }
+        locate<I>(a, 1, row, oi, oo);
+        const int64_t end = nseg > 1 ? min(n0, lo + seg) : n0;
         const double *src = in + oi;
         double *dst = out + oo;
-        if (beta == 0.0) {
-            for (int64_t i0 = threadIdx.x; i0 < n0; i0 += 32) dst[i0 * so0] = alpha * src[i0 * si0];
-        } else {
-            for (int64_t i0 = threadIdx.x; i0 < n0; i0 += 32) dst[i0 * so0] = alpha * src[i0 * si0] + beta * dst[i0 * so0];
+        for (int64_t i0 = lo + threadIdx.x; i0 < end; i0 += 128) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int64_t i = i0 + 32 * k;
+                v[k] = i < end ? alpha * src[i * si0] : 0.0;
+            }
+            if (beta != 0.0) {
+                double old[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int64_t i = i0 + 32 * k;
+                    old[k] = i < end ? dst[i * so0] : 0.0;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) v[k] += beta * old[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int64_t i = i0 + 32 * k;
+                if (i < end) dst[i * so0] = v[k];
+            }
         }
     }
 }
 
 // 32x32 tile over (p = input-fastest dim, q = output-fastest dim); the remaining dims
 // are flattened into the z loop.  Dims 2.. of `a` are the batch dims.
-__global__ void permute_tiled_kernel(PermArgs a, int64_t nbatch, double alpha, const double *__restrict__ in,
-                                     double beta, double *__restrict__ out) {
+template <class I>
+__global__ void __launch_bounds__(256) permute_tiled_kernel(PermArgs a, int64_t nbatch, double alpha,
+                                                            const double *__restrict__ in, double beta,
+                                                            double *__restrict__ out) {
     __shared__ double tile[32][33];
     const int64_t np = a.n[0], nq = a.n[1];
-    const int64_t p0 = (int64_t)blockIdx.x * 32, q0 = (int64_t)blockIdx.y * 32;
+    const int64_t p0 = (int64_t)blockIdx.x * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
     for (int64_t b = blockIdx.z; b < nbatch; b += gridDim.z) {
-        int64_t r = b, bi = 0, bo = 0;
-        for (int d = 2; d < a.nd; d++) {
-            int64_t q = r / a.n[d];
-            int64_t i = r - q * a.n[d];
-            r = q;
-            bi += i * a.si[d];
-            bo += i * a.so[d];
-        }
-        for (int k = ty; k < 32; k += 8) {
-            int64_t p = p0 + tx, q = q0 + k;
-            if (p < np && q < nq) tile[k][tx] = in[bi + p * a.si[0] + q * a.si[1]];
-        }
-        __syncthreads();
-        for (int k = ty; k < 32; k += 8) {
-            int64_t q = q0 + tx, p = p0 + k;
-            if (p < np && q < nq) {
-                int64_t o = bo + p * a.so[0] + q * a.so[1];
-                double v = alpha * tile[tx][k];
-                if (beta != 0.0) v += beta * out[o];
-                out[o] = v;
+        int64_t bi = 0, bo = 0;
+        locate<I>(a, 2, (I)b, bi, bo);
+        for (int64_t q0 = (int64_t)blockIdx.y * 32; q0 < nq; q0 += (int64_t)gridDim.y * 32) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int64_t p = p0 + tx, q = q0 + ty + 8 * k;
+                v[k] = p < np && q < nq ? in[bi + p * a.si[0] + q * a.si[1]] : 0.0;
             }
+#pragma unroll
+            for (int k = 0; k < 4; k++) tile[ty + 8 * k][tx] = v[k];
+            __syncthreads();
+            const int64_t q = q0 + tx;
+            double *dst = out + bo + q * a.so[1];
+            if (beta != 0.0) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int64_t p = p0 + ty + 8 * k;
+                    v[k] = p < np && q < nq ? beta * dst[p * a.so[0]] : 0.0;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int64_t p = p0 + ty + 8 * k;
+                const double x = alpha * tile[tx][ty + 8 * k];
+                if (p < np && q < nq) dst[p * a.so[0]] = beta != 0.0 ? x + v[k] : x;
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 
@@ -162,45 +194,53 @@ void permute_add(Exec &ex, double alpha, const TV &in, double beta, const TV &ou
     if (total == 0) return;
     PermArgs a{};
     if (dims.empty()) dims.push_back(0);
-    // order by output stride
+    // order by output stride, neighbours that are one run on both sides taken as one dim (the long runs that
+    // leaves fill the tiles below: 1.6 GB of six [a,j,b,k] with j of 24 moved in front of a 1.39 ms in tiles
+    // of 32 x 24, 0.85 ms so)
     std::sort(dims.begin(), dims.end(), [&](int x, int y) { return out.s[x] < out.s[y]; });
-    int q = dims[0];                                       // output-fastest
-    int p = *std::min_element(dims.begin(), dims.end(), [&](int x, int y) { return in.s[x] < in.s[y]; });
-    if (p != q && in.n[p] >= 8 && in.n[q] >= 8) {
-        a.nd = (int)dims.size();
-        a.n[0] = in.n[p];
-        a.si[0] = in.s[p];
-        a.so[0] = out.s[p];
-        a.n[1] = in.n[q];
-        a.si[1] = in.s[q];
-        a.so[1] = out.s[q];
-        int k = 2;
-        int64_t nb = 1;
-        for (int d : dims)
-            if (d != p && d != q) {
-                a.n[k] = in.n[d];
-                a.si[k] = in.s[d];
-                a.so[k] = out.s[d];
-                nb *= in.n[d];
-                k++;
-            }
-        dim3 grid((unsigned)((a.n[0] + 31) / 32), (unsigned)((a.n[1] + 31) / 32),
-                  (unsigned)std::min<int64_t>(nb, 65535));
-        permute_tiled_kernel<<<grid, dim3(32, 8), 0, ex.stream>>>(a, nb, alpha, in.p, beta, out.p);
+    for (int d : dims) {
+        const int k = a.nd;
+        if (k > 0 && in.s[d] == a.si[k - 1] * a.n[k - 1] && out.s[d] == a.so[k - 1] * a.n[k - 1]) {
+            a.n[k - 1] *= in.n[d];
+            continue;
+        }
+        a.n[k] = in.n[d];
+        a.si[k] = in.s[d];
+        a.so[k] = out.s[d];
+        a.nd++;
+    }
+    int p = 0;   // the input-fastest dim; the output-fastest is 0
+    for (int d = 1; d < a.nd; d++)
+        if (a.si[d] < a.si[p]) p = d;
+    const bool small = total < (1ll << 31);
+    if (p != 0 && a.n[p] >= 8 && a.n[0] >= 8) {
+        // (p, 0, the others)
+        const int64_t n = a.n[p], si = a.si[p], so = a.so[p];
+        for (int d = p; d > 0; d--) {
+            a.n[d] = a.n[d - 1];
+            a.si[d] = a.si[d - 1];
+            a.so[d] = a.so[d - 1];
+        }
+        a.n[0] = n;
+        a.si[0] = si;
+        a.so[0] = so;
+        const int64_t nb = total / (a.n[0] * a.n[1]);
+        const dim3 grid((unsigned)((a.n[0] + 31) / 32), (unsigned)std::min<int64_t>((a.n[1] + 31) / 32, 65535),
+                        (unsigned)std::min<int64_t>(nb, 65535));
+        auto kernel = nb < (1ll << 31) ? permute_tiled_kernel<uint32_t> : permute_tiled_kernel<int64_t>;
+        kernel<<<grid, dim3(32, 8), 0, ex.stream>>>(a, nb, alpha, in.p, beta, out.p);
+    } else if (a.n[0] >= 16) {
+        // segments of 128 to 1024, short enough for 48 warps an SM
+        const int64_t per_warp = (total / (148 * 48) + 127) / 128 * 128;
+        const int seg = (int)std::min<int64_t>(1024, std::max<int64_t>(128, per_warp));
+        const int nseg = (int)((a.n[0] + seg - 1) / seg);
+        const int64_t nwork = total / a.n[0] * nseg;
+        const int blocks = (int)std::min<int64_t>((nwork + 7) / 8, 148 * 64);
+        auto kernel = nwork < (1ll << 31) ? permute_rows_kernel<uint32_t> : permute_rows_kernel<int64_t>;
+        kernel<<<blocks, dim3(32, 8), 0, ex.stream>>>(a, nwork, nseg, seg, alpha, in.p, beta, out.p);
     } else {
-        a.nd = (int)dims.size();
-        for (size_t k = 0; k < dims.size(); k++) {
-            a.n[k] = in.n[dims[k]];
-            a.si[k] = in.s[dims[k]];
-            a.so[k] = out.s[dims[k]];
-        }
-        if (a.n[0] >= 16) {
-            const int64_t nrows = total / a.n[0];
-            const int blocks = (int)std::min<int64_t>((nrows + 7) / 8, 148 * 64);
-            permute_rows_kernel<<<blocks, dim3(32, 8), 0, ex.stream>>>(a, nrows, alpha, in.p, beta, out.p);
-        } else {
-            permute_simple_kernel<<<grid_for(total, 256), 256, 0, ex.stream>>>(a, total, alpha, in.p, beta, out.p);
-        }
+        auto kernel = small ? permute_simple_kernel<uint32_t> : permute_simple_kernel<int64_t>;
+        kernel<<<grid_for(total, 256), 256, 0, ex.stream>>>(a, total, alpha, in.p, beta, out.p);
     }
     ex.launches++;
     CU_CHECK(cudaGetLastError());
