@@ -527,6 +527,108 @@ bool out_view(const TV &C, const Dims &rows, const Dims &cols, OutView *out) {
     return true;
 }
 
+// A small product of strided tensors in one launch: C = alpha sum_k A B + beta C for any order of the indices.
+// Such a product is bound by its launches: with cuBLAS an operand's copy, the product, the sum of its K
+// slices and the output's scatter are up to five of some 3 us each.  The offsets of the K positions in A and B
+// stand in shared memory; G threads sum one element, 1 for a short K (the warp then runs along the output), else
+// 32 or 256 along K.  An H2O iteration in cc-pVDZ (n_o = 5, n_v = 19) 542 us without, 461 with it; at
+// n_o = 9, n_v = 71 few products are this small and nothing changes.
+struct SmallDims {
+    int nd;
+    int n[4];
+    long long s0[4], s1[4];   // strides in the two tensors that have these dims
+    __device__ __forceinline__ void locate(int x, long long &o0, long long &o1) const {
+        o0 = o1 = 0;
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            if (d < nd) {
+                const int q = x / n[d], i = x - q * n[d];
+                x = q;
+                o0 += i * s0[d];
+                o1 += i * s1[d];
+            }
+        }
+    }
+};
+
+struct SmallProduct {
+    SmallDims m, n, k;   // in (A, C), (B, C) and (A, B)
+    int M, N, K;
+    const double *A, *B;
+    double *C;
+    double alpha, beta;
+};
+
+constexpr int SMALL_K = 1024;            // K positions per table
+// The line: products of up to 2^18 flops alone leave the H2O iteration at 493 us instead of 456; up to 2^23
+// would give it 447 but the residual at n_o = 9, n_v = 71 1054 us instead of 987, cuBLAS being faster there.
+constexpr double SMALL_FLOPS = 1 << 20;
+
+template <int G>
+__global__ void __launch_bounds__(256) small_product_kernel(SmallProduct p) {
+    __shared__ long long ka[SMALL_K], kb[SMALL_K];
+    __shared__ double part[8];
+    const int lane = threadIdx.x % G, o = blockIdx.x * (256 / G) + threadIdx.x / G;
+    const bool live = o < p.M * p.N;
+    long long oa = 0, ob = 0, ocm = 0, ocn = 0;
+    if (live) {
+        p.m.locate(o % p.M, oa, ocm);
+        p.n.locate(o / p.M, ob, ocn);
+    }
+    const double *A = p.A + oa, *B = p.B + ob;
+    double acc = 0.0;
+    for (int k0 = 0; k0 < p.K; k0 += SMALL_K) {
+        const int nk = min(SMALL_K, p.K - k0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < nk; i += 256) p.k.locate(k0 + i, ka[i], kb[i]);
+        __syncthreads();
+        if (live) {
+#pragma unroll 4
+            for (int i = lane; i < nk; i += G) acc += A[ka[i]] * B[kb[i]];
+        }
+    }
+    if (G > 1)
+        for (int h = 16; h > 0; h >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, h);
+    if (G > 32) {
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < 8; w++) acc += part[w];
+    }
+    if (live && lane == 0) {
+        double *c = p.C + ocm + ocn;
+        *c = p.beta != 0.0 ? p.alpha * acc + p.beta * *c : p.alpha * acc;
+    }
+}
+
+// the dims of labels v with their strides in x (dims d0) and y (dims d1), runs in both taken as one
+bool small_dims(const TV &x, const Dims &d0, const TV &y, const Dims &d1, SmallDims *out) {
+    SmallDims v{};
+    for (int i = 0; i < d0.n; i++) {
+        const int64_t n = x.n[d0[i]], s0 = x.s[d0[i]], s1 = y.s[d1[i]];
+        if (n == 1) continue;
+        if (v.nd > 0 && s0 == v.s0[v.nd - 1] * v.n[v.nd - 1] && s1 == v.s1[v.nd - 1] * v.n[v.nd - 1]) {
+            v.n[v.nd - 1] *= (int)n;
+            continue;
+        }
+        if (v.nd == 4) return false;
+        v.n[v.nd] = (int)n;
+        v.s0[v.nd] = s0;
+        v.s1[v.nd++] = s1;
+    }
+    *out = v;
+    return true;
+}
+
+void run_small(Exec &ex, const SmallProduct &p) {
+    const int outs = p.M * p.N;
+    if (p.K <= 64) small_product_kernel<1><<<(outs + 255) / 256, 256, 0, ex.stream>>>(p);
+    else if (p.K < 1024 || outs > 1024) small_product_kernel<32><<<(outs + 7) / 8, 256, 0, ex.stream>>>(p);
+    else small_product_kernel<256><<<outs, 256, 0, ex.stream>>>(p);
+    ex.launches++;
+    CU_CHECK(cudaGetLastError());
+}
+
 // bytes that the reordering copies of a product move (each read and written once; an output that is
 // scattered also reads its old values)
 double copy_bytes(const TV &A, bool packA, const TV &B, bool packB, const TV &C, bool scatter) {
@@ -771,6 +873,29 @@ void contract(Exec &ex, const char *spec, double alpha, const TV &A, const TV &B
         copies();
         rt = swap ? measure_route(ex, rt, !tB, !tA, mN, mM, mK, alpha, Bu.p, ldb, Au.p, lda, fl, true)
                         : measure_route(ex, rt, tA, tB, mM, mN, mK, alpha, Au.p, lda, Bu.p, ldb, fl, true);
+    }
+    // a small product that cuBLAS needs several launches for: copies, or K slices and their sum (rows: the group
+    // of C's unit stride)
+    SmallProduct sp{};
+    if ((strided || (mK >= 512 && mM * mN <= 1024)) && !rt.mixed && fl <= SMALL_FLOPS && mK > 0 && !gemm_takes_digits(ex, mM, mN, mK, fl)) {
+        const bool flip = !cM.empty() && !cN.empty() && C.s[cN[0]] < C.s[cM[0]];
+        if (flip ? small_dims(B, bN, C, cN, &sp.m) && small_dims(A, aM, C, cM, &sp.n) && small_dims(B, bK, A, aK, &sp.k)
+                 : small_dims(A, aM, C, cM, &sp.m) && small_dims(B, bN, C, cN, &sp.n) && small_dims(A, aK, B, bK, &sp.k)) {
+            sp.M = (int)(flip ? mN : mM);
+            sp.N = (int)(flip ? mM : mN);
+            sp.K = (int)mK;
+            sp.A = flip ? B.p : A.p;
+            sp.B = flip ? A.p : B.p;
+            sp.C = C.p;
+            sp.alpha = alpha;
+            sp.beta = beta;
+            ex.flops += fl;
+            if (trace_level() >= 2)
+                std::fprintf(stderr, "ccsd_gpu gemm [%s] fp64 small m %lld n %lld k %lld\n", spec, (long long)mM,
+                             (long long)mN, (long long)mK);
+            run_small(ex, sp);
+            return;
+        }
     }
     SplitView va, vb;
     OutView vc;
