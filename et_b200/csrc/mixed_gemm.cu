@@ -942,7 +942,7 @@ void launch_mode(Exec &ex, const __nv_bfloat16 *A, int64_t a_rows, int64_t a_pla
     }
 }
 
-// the two-plane GEMM on CTA pairs: tiles of 256 x 256, persistent over the pairs that can be resident
+// the two-plane GEMM on CTA pairs: tiles of 256 rows and up to 256 columns, persistent over the pairs that can be resident
 template <class Epi>
 void launch_pair(Exec &ex, const __nv_bfloat16 *A, int64_t a_rows, int64_t a_plane, int64_t m_out,
                  const __nv_bfloat16 *B, int64_t b_rows, int64_t b_plane, int64_t n_out, int64_t Kp, const Epi &epi,
@@ -1304,7 +1304,7 @@ std::vector<int> tc_split_candidates(int64_t m, int64_t n, int64_t k, int planes
         // counts whose units fill about j waves of the persistent grid
         for (int j = 1; j <= 4; j++) add(j * nsm / tiles, 4);
     }
-    // the same K splits on CTA pairs (256 x 256 tiles) for products with a full pair tile of rows
+    // the same K splits on CTA pairs (256-row tiles) for products with a full pair tile of rows
     if (planes == 2 && m >= 2 * BM) {
         const size_t single = out.size();
         for (size_t i = 0; i < single; i++) out.push_back(PAIR_ROUTE + out[i]);

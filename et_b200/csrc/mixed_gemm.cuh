@@ -52,7 +52,7 @@ void mixed_gemm_views(Exec &ex, const SplitView &A, const SplitView &B, int64_t 
                       double beta, const OutView &C, int splits = -1);
 
 // Routes (the `splits` argument of the GEMMs below and of mixed_gemm): s in 1..99 runs the
-// single-CTA kernel with s K splits, PAIR_ROUTE + s the CTA-pair kernel (cta_group::2, 256 x 256
+// single-CTA kernel with s K splits, PAIR_ROUTE + s the CTA-pair kernel (cta_group::2, 256-row
 // tiles) with s K splits; 0 or less takes the fixed rule's count.
 constexpr int PAIR_ROUTE = 100;
 
