@@ -156,6 +156,7 @@ struct TpmOut {
     __nv_bfloat16 *bp, *bm;        // or bf16 planes
     int64_t ldp, ldm, plane_p, plane_m;
     int np;
+    int64_t rows_p, rows_m;        // rows of a plane; those beyond the vectors' pairs are cleared
 };
 
 __device__ __forceinline__ void put_planes(double x, int np, int64_t plane, __nv_bfloat16 *out) {
@@ -170,7 +171,25 @@ __device__ __forceinline__ void put_planes(double x, int np, int64_t plane, __nv
 // (c, i), t_cjdi along c in row (d, i), turned in shared memory; both forms are stored along d.  Bound by
 // HBM: n_t2 read, the forms written; each thread of the element-wise version found its four indices by two
 // square roots and read two elements whose neighbours lay a packed row apart.  bf16 planes at o=32, v=320
-// 0.34 ms (1.9 TB/s), 0.54 without MIN_BLOCKS.
+// 0.34 ms (1.9 TB/s; 0.38 with the padding), 0.54 without MIN_BLOCKS.
+// The padding of one form's planes: K positions beyond the k pairs cd and rows beyond the used ones (ld is a
+// multiple of 8), shared out over the whole grid.  As up to four 2-D memsets before the kernel a residual at o=13,
+// v=107 took 1.081 ms, so 1.067; from o=16, v=128 on it makes no difference.
+__device__ __forceinline__ void clear_pads(__nv_bfloat16 *t, int np, int64_t rows, int64_t used, int64_t ld, int64_t k) {
+    const int64_t id = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * (TILE * ROWS) + threadIdx.y * TILE + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * gridDim.y * (TILE * ROWS);
+    const int pad = (int)(ld - k);
+    for (int64_t x = id; x < (int64_t)np * used * pad; x += step) {
+        const int64_t row = x / pad, q = row / used;   // plane q
+        t[(q * rows + row - q * used) * ld + k + (x - row * pad)] = __float2bfloat16(0.0f);
+    }
+    const int64_t tail = (rows - used) * ld / 8;
+    for (int64_t x = id; x < np * tail; x += step) {
+        const int64_t q = x / tail;
+        reinterpret_cast<uint4 *>(t + (q * rows + used) * ld)[x - q * tail] = make_uint4(0, 0, 0, 0);
+    }
+}
+
 template <bool PLANES>
 __global__ void __launch_bounds__(TILE * ROWS, MIN_BLOCKS)
 tpm_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec, TpmOut o) {
@@ -178,6 +197,10 @@ tpm_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int64_t nov = (int64_t)no * nv, nt2 = nov * (nov + 1) / 2;
     const int64_t nop = (int64_t)no * (no + 1) / 2, nom = (int64_t)no * (no - 1) / 2;
+    if (PLANES) {
+        clear_pads(o.bp, o.np, o.rows_p, nvec * nop, o.ldp, (int64_t)nv * (nv + 1) / 2);
+        clear_pads(o.bm, o.np, o.rows_m, nvec * nom, o.ldm, (int64_t)nv * (nv - 1) / 2);
+    }
     int ct, dt, i, j;
     untri32(blockIdx.x, ct, dt);
     const int c0 = TILE * ct, d0 = TILE * dt;
@@ -316,7 +339,7 @@ void sym_pack(Exec &ex, const double *F, const double *X, int64_t no, int64_t nv
 
 void build_tpm(Exec &ex, const double *t2, int64_t no, int64_t nv, int64_t nvec, double *tp, int64_t ldp, double *tm,
                int64_t ldm) {
-    const TpmOut o{tp, tm, nullptr, nullptr, ldp, ldm, 0, 0, 0};
+    const TpmOut o{tp, tm, nullptr, nullptr, ldp, ldm, 0, 0, 0, 0, 0};
     tpm_forms_kernel<false><<<pair_grid(no, nv, nvec), dim3(TILE, ROWS), 0, ex.stream>>>(t2, (int)no, (int)nv, nvec, o);
     ex.launches++;
     CU_CHECK(cudaGetLastError());
@@ -324,15 +347,7 @@ void build_tpm(Exec &ex, const double *t2, int64_t no, int64_t nv, int64_t nvec,
 
 void build_tpm_planes(Exec &ex, const double *t2, int64_t no, int64_t nv, int64_t nvec, int np, __nv_bfloat16 *tp,
                       int64_t rows_p, int64_t ldp, __nv_bfloat16 *tm, int64_t rows_m, int64_t ldm) {
-    const TpmOut o{nullptr, nullptr, tp, tm, ldp, ldm, rows_p * ldp, rows_m * ldm, np};
-    const size_t eb = sizeof(__nv_bfloat16);
-    auto clear = [&](__nv_bfloat16 *t, int64_t rows, int64_t used, int64_t ld, int64_t k) {
-        if (ld > k) CU_CHECK(cudaMemset2DAsync(t + k, ld * eb, 0, (ld - k) * eb, (size_t)np * rows, ex.stream));
-        if (rows > used)
-            CU_CHECK(cudaMemset2DAsync(t + used * ld, rows * ld * eb, 0, (rows - used) * ld * eb, np, ex.stream));
-    };
-    clear(tp, rows_p, nvec * (no * (no + 1) / 2), ldp, nv * (nv + 1) / 2);
-    clear(tm, rows_m, nvec * (no * (no - 1) / 2), ldm, nv * (nv - 1) / 2);
+    const TpmOut o{nullptr, nullptr, tp, tm, ldp, ldm, rows_p * ldp, rows_m * ldm, np, rows_p, rows_m};
     tpm_forms_kernel<true><<<pair_grid(no, nv, nvec), dim3(TILE, ROWS), 0, ex.stream>>>(t2, (int)no, (int)nv, nvec, o);
     ex.launches++;
     CU_CHECK(cudaGetLastError());
