@@ -630,9 +630,10 @@ void Context::ladder_tc_streamed(const double *Lvv, const double *t2, double *om
 
 // Mixed precision keeps the ovvv and ovov integrals of the untransformed Cholesky vectors resident as split
 // bf16, ybuf[plane][k + no*p][c + nv*d] = g_kcpd with p over the virtual and then the occupied orbitals
-// (o (o + v) v^2 elements per plane: 4.6 GB for both planes at o = 32, v = 320), formed once per Cholesky set
-// by one tensor-core GEMM whose epilogue writes the planes.  The ladder's Y0 and the Q of its corrections
-// and of omega_ccsd_b2 then cost one GEMM of o^2 x o (o + v) x v^2 per call.
+// (o (o + v) v^2 elements per plane: 4.6 GB for both planes at o = 32, v = 320), formed once per Cholesky set:
+// the virtual rows by one tensor-core GEMM whose epilogue writes the planes, the occupied rows as the planes of
+// the FP64 g_kcld.  The ladder's Y0 and the Q of its corrections and of omega_ccsd_b2 then cost one GEMM of
+// o^2 x o (o + v) x v^2 per call.
 bool Context::ovvv_resident() {
     const size_t need = sizeof(__nv_bfloat16) * (size_t)ex.planes * (size_t)tc_pad_rows_a(no * nmo) * tc_pad_k(nv * nv);
     if (ybuf_bytes >= need) return true;
@@ -662,19 +663,16 @@ void Context::ovvv_pairs() {
         permute_add(ex, 1.0, tv(L_ov.d(), {nJ, no, nv}), 0.0, dst);
         split_rows(ex, LO.d(), nJ, 1, nov, nJ, o_rows, Jp, LOS.as<__nv_bfloat16>());
     }
-    // rows d + nv*p of L_vv and then of L_ov: L[J, p, d] copied to (J, d, p)
-    const int64_t v_rows = tc_pad_rows_b(nv * nmo);
+    // L_vv split rows d + nv*b: L_vv[J, b, d] copied to (J, d, b)
+    const int64_t v_rows = tc_pad_rows_b(nv2);
     DBuf LVS(sizeof(__nv_bfloat16) * np * v_rows * Jp, s);
     {
-        DBuf LV = dalloc(nJ * nv * nmo, s);
+        DBuf LV = dalloc(nJ * nv2, s);
         TV dst = tv(LV.d(), {nJ, nv, nv});   // [J, b, d] at J + nJ*(d + nv*b)
         dst.s[1] = nJ * nv;
         dst.s[2] = nJ;
         permute_add(ex, 1.0, tv(L_vv.d(), {nJ, nv, nv}), 0.0, dst);
-        dst.p += nJ * nv2;
-        dst.n[1] = no;                       // [J, l, d] behind it
-        permute_add(ex, 1.0, tv(L_ov.d(), {nJ, no, nv}), 0.0, dst);
-        split_rows(ex, LV.d(), nJ, 1, nv * nmo, nJ, v_rows, Jp, LVS.as<__nv_bfloat16>());
+        split_rows(ex, LV.d(), nJ, 1, nv2, nJ, v_rows, Jp, LVS.as<__nv_bfloat16>());
     }
     const int64_t yrows = tc_pad_rows_a(no * nmo);
     const size_t need = sizeof(__nv_bfloat16) * (size_t)np * (size_t)yrows * Kq;
@@ -687,6 +685,22 @@ void Context::ovvv_pairs() {
     }
     tc_gemm_ovvv(ex, LOS.as<__nv_bfloat16>(), o_rows, LVS.as<__nv_bfloat16>(), v_rows, Jp, no, nv,
                  ybuf.as<__nv_bfloat16>(), yrows, Kq, nJ);
+    // the occupied rows k + no*(nv + l) from the FP64 g_kcld: a product of split vectors would cost their bits
+    const int64_t oo = no * no, occ_rows = tc_pad_rows_a(oo);
+    DBuf OS(sizeof(__nv_bfloat16) * np * occ_rows * Kq, s);
+    SplitView g{};
+    g.p = g_ovov_const();
+    g.nr = g.nk = 2;
+    g.rn[0] = g.rn[1] = no;   // k, l
+    g.rs[0] = 1;
+    g.rs[1] = nov;
+    g.kn[0] = g.kn[1] = nv;   // c, d
+    g.ks[0] = no;
+    g.ks[1] = nov * no;
+    split_tensor(ex, g, oo, nv2, occ_rows, Kq, OS.as<__nv_bfloat16>());
+    for (int p = 0; p < np; p++)
+        CU_CHECK(cudaMemcpyAsync(ybuf.as<__nv_bfloat16>() + (p * yrows + nov) * Kq, OS.as<__nv_bfloat16>() + p * occ_rows * Kq,
+                                 sizeof(__nv_bfloat16) * oo * Kq, cudaMemcpyDeviceToDevice, s));
     ybuf_version = l_version;
     ybuf_planes = np;
     cache_epoch++;

@@ -154,10 +154,9 @@ __device__ __forceinline__ void store_split_planes(__nv_bfloat16 *out, size_t pl
     if (np == 3) out[2 * plane + idx] = __float2bfloat16(r - __bfloat162float(mid));
 }
 
-// Integrals g_kcpd of the untransformed Cholesky vectors for the ladder's Y and Q intermediates: row
-// (c, k) = c + nv*k of L_ov, column (d, p) = d + nv*p of L_vv (virtual p) and then L_ov (occupied p);
-// written as np bf16 planes at row k + no*p, K position c + nv*d (the 32 lanes of a warp
-// take consecutive c and store to consecutive addresses).
+// Integrals g_kcbd of the untransformed Cholesky vectors for the ladder's Y intermediate: row
+// (c, k) = c + nv*k of L_ov, column (d, b) = d + nv*b of L_vv; written as np bf16 planes at row k + no*b,
+// K position c + nv*d (the 32 lanes of a warp take consecutive c and store to consecutive addresses).
 struct EpiOvvv {
     static constexpr bool kChunked = false;
     static constexpr bool kTable = false;
@@ -1416,7 +1415,7 @@ void tc_gemm_f64(Exec &ex, const __nv_bfloat16 *A, int64_t Mp, const __nv_bfloat
 void tc_gemm_ovvv(Exec &ex, const __nv_bfloat16 *Lov, int64_t ov_rows, const __nv_bfloat16 *Lvv, int64_t vv_rows,
                   int64_t Kp, int64_t no, int64_t nv, __nv_bfloat16 *out, int64_t out_rows_pad, int64_t out_ld,
                   int64_t k_true) {
-    REQUIRE(out_rows_pad >= no * (no + nv) && out_ld >= nv * nv && ov_rows >= no * nv && vv_rows >= nv * (no + nv),
+    REQUIRE(out_rows_pad >= no * nv && out_ld >= nv * nv && ov_rows >= no * nv && vv_rows >= nv * nv,
             CCSD_GPU_EINVAL, "tc_gemm_ovvv: bad padding");
     EpiOvvv epi{};
     epi.out = out;
@@ -1425,7 +1424,7 @@ void tc_gemm_ovvv(Exec &ex, const __nv_bfloat16 *Lov, int64_t ov_rows, const __n
     epi.no = (int)no;
     epi.nv = (int)nv;
     epi.M = (int)(no * nv);
-    epi.N = (int)(nv * (no + nv));
+    epi.N = (int)(nv * nv);
     epi.np = check_planes(ex.planes);
     launch_tc(ex, epi.np, Lov, ov_rows, ov_rows * Kp, epi.M, Lvv, vv_rows, vv_rows * Kp, epi.N, Kp, epi,
               double(epi.M) * double(epi.N) * double(k_true));

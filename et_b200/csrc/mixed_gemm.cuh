@@ -85,10 +85,9 @@ void tc_gemm_f64(Exec &ex, const __nv_bfloat16 *A, int64_t Mp, const __nv_bfloat
                  int64_t m, int64_t n, int64_t k_true, double alpha, double beta, double *C, int64_t ldc,
                  int splits = 1);
 
-// integrals g_kcpd = sum_J L_kc L_pd of the untransformed Cholesky vectors as split bf16, p over the virtual
-// and then the occupied orbitals: Lov holds split rows c + nv*k (K = N_J padded to Kp), Lvv split rows
-// d + nv*p; the result goes to out[plane][k + no*p][c + nv*d] (row stride out_ld, plane stride
-// out_rows_pad * out_ld).
+// integrals g_kcbd = sum_J L_kc L_bd of the untransformed Cholesky vectors as split bf16:
+// Lov holds split rows c + nv*k (K = N_J padded to Kp), Lvv split rows d + nv*b; the result goes
+// to out[plane][k + no*b][c + nv*d] (row stride out_ld, plane stride out_rows_pad * out_ld).
 void tc_gemm_ovvv(Exec &ex, const __nv_bfloat16 *Lov, int64_t ov_rows, const __nv_bfloat16 *Lvv, int64_t vv_rows,
                   int64_t Kp, int64_t no, int64_t nv, __nv_bfloat16 *out, int64_t out_rows_pad, int64_t out_ld,
                   int64_t k_true);
