@@ -883,16 +883,25 @@ void Context::ladder_f64(const double *t2, double *om2) {
 
 Context::LadderY Context::ladder_y_plain(const double *tf) {
     cudaStream_t s = ex.stream;
-    const int64_t oo = no * no, nv2 = nv * nv, rows = no * nmo;
+    const int64_t oo = no * no, nv2 = nv * nv;
     LadderY r;
     r.Y = dalloc(oo * nov, s);
     r.Q = dalloc(oo * oo, s);
-    if (ex.prec == Prec::MIXED && !ovvv_resident()) {
-        ladder_y(L_vv.d(), tf, r.Y.d());
+    // Q by itself, in the arithmetic that the dispatch gives a product of its size
+    auto own_q = [&]() {
         contract(ex, "kcld,cidj->kilj", 1.0, tv(g_ovov_const(), {no, nv, no, nv}), tv(tf, {nv, no, nv, no}), 0.0,
                  tv(r.Q.d(), {no, no, no, no}));
+    };
+    if (ex.prec == Prec::MIXED && !ovvv_resident()) {
+        ladder_y(L_vv.d(), tf, r.Y.d());
+        own_q();
         return r;
     }
+    // Mixed precision: Q joins Y0's product only where the dispatch may run a product of its size on the tensor
+    // cores; smaller ones are FP64.  Where routes are timed both arithmetics are open to it, and joined costs
+    // least: a residual at o=13, v=107 1.07 ms, 1.13 with Q on the route that was fastest for it alone (DGEMM)
+    const bool joined = ex.prec != Prec::MIXED || gemm_may_take_tensor_cores(ex, oo, oo, nv2);
+    const int64_t rows = joined ? no * nmo : nov;
     // t as [(c, d), (i, j)], the product [(k, p), (i, j)]
     DBuf W = dalloc(rows * oo, s);
     if (ex.prec == Prec::MIXED) {
@@ -909,7 +918,7 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
         v.ks[0] = 1;
         v.ks[1] = nov;
         split_tensor(ex, v, oo, nv2, rows_T, Kq, TS.as<__nv_bfloat16>());
-        tc_gemm_f64_tuned(ex, ybuf.as<__nv_bfloat16>(), tc_pad_rows_a(rows), TS.as<__nv_bfloat16>(), rows_T, Kq, rows, oo,
+        tc_gemm_f64_tuned(ex, ybuf.as<__nv_bfloat16>(), tc_pad_rows_a(no * nmo), TS.as<__nv_bfloat16>(), rows_T, Kq, rows, oo,
                           nv2, 1.0, 0.0, W.d(), rows, 0);
         ex.flops += 2.0 * double(rows) * double(oo) * double(nv2);
     } else {
@@ -934,9 +943,13 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
     src.s[2] = no;
     src.s[3] = rows * no;
     permute_add(ex, 1.0, src, 0.0, tv(r.Y.d(), {no, no, nv, no}));
-    src.p += nov;                           // (k, i, l, j)
-    src.n[2] = no;
-    permute_add(ex, 1.0, src, 0.0, tv(r.Q.d(), {no, no, no, no}));
+    if (joined) {
+        src.p += nov;                       // (k, i, l, j)
+        src.n[2] = no;
+        permute_add(ex, 1.0, src, 0.0, tv(r.Q.d(), {no, no, no, no}));
+    } else {
+        own_q();
+    }
     return r;
 }
 

@@ -269,13 +269,15 @@ Route fixed_route(const Exec &ex, int64_t m, int64_t n, int64_t k, double fl, bo
     return r;
 }
 
+// products big enough to be worth timing on the tensor cores
+bool worth_timing(int64_t m, int64_t n, int64_t k, double fl) { return k >= 16 && fl >= 5e7 && m >= 16 && n >= 16; }
+
 Route lookup_route(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double fl, bool allow_mixed) {
     Route r;
     const bool tc_ok = allow_mixed && ex.prec == Prec::MIXED && k >= 16;
     if (tc_ok && ex.autotune) {
-        // measured route (0 = DGEMM, s >= 1 = tensor cores with s K-splits) for products big enough
-        // to be worth timing
-        if (fl < 5e7 || m < 16 || n < 16) {
+        // measured route (0 = DGEMM, s >= 1 = tensor cores with s K-splits)
+        if (!worth_timing(m, n, k, fl)) {
             r.splits = 0;
             return r;
         }
@@ -345,6 +347,12 @@ void run_gemm(Exec &ex, const Route &rt, bool transA, bool transB, int64_t m, in
 }
 
 }  // namespace
+
+bool gemm_may_take_tensor_cores(const Exec &ex, int64_t m, int64_t n, int64_t k) {
+    const double fl = 2.0 * double(m) * double(n) * double(k);
+    if (ex.prec == Prec::MIXED && ex.autotune) return worth_timing(m, n, k, fl);
+    return fixed_route(ex, m, n, k, fl, true).mixed;
+}
 
 void gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha, const double *A,
           int64_t lda, const double *B, int64_t ldb, double beta, double *C, int64_t ldc, bool allow_mixed) {

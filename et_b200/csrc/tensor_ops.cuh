@@ -21,6 +21,9 @@ void gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_t k, d
           const double *A, int64_t lda, const double *B, int64_t ldb, double beta, double *C,
           int64_t ldc, bool allow_mixed = true);
 
+// whether the dispatch lets a product of this size onto the tensor cores at all (with measured routes: times them
+// there against DGEMM)
+bool gemm_may_take_tensor_cores(const Exec &ex, int64_t m, int64_t n, int64_t k);
 // whether an FP64 product of fl flops goes to the int8 digit GEMM
 bool gemm_takes_digits(const Exec &ex, int64_t m, int64_t n, int64_t k, double fl);
 // C_z = alpha op(A_z) op(B_z) + beta C_z for z < batch, operand z at base + z * stride (FP64

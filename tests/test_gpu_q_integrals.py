@@ -39,3 +39,16 @@ def test_integrals_split_from_fp64(n_o, n_v):
     out = _omega((L, h, eps), t, n_o, n_v, 2, precision=MIXED, mixed_min_flops=1)
     # integers below 2^16 are exact in two planes, their sums below 2^24 exact in FP32
     assert np.linalg.norm(out - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n_o,n_v", [(2, 9), (8, 64)])
+def test_small_products_stay_fp64(n_o, n_v):
+    """Products below mixed_min_flops stay FP64, Q and X_klij among them."""
+    from et_b200 import FP64, MIXED
+    rng, L, h, eps, t = _system(n_o, n_v, 7, n_v)
+    L[:, :n_o, n_o:] = rng.standard_normal((7, n_o, n_v))
+    t = rng.standard_normal(t.size)
+    t[:n_o * n_v] *= 0.1
+    ref = _omega((L, h, eps), t, n_o, n_v, 7, precision=FP64)
+    out = _omega((L, h, eps), t, n_o, n_v, 7, precision=MIXED, mixed_min_flops=10 ** 15)
+    assert np.linalg.norm(out - ref) <= 1e-12 * np.linalg.norm(ref)
