@@ -831,16 +831,17 @@ bool Context::f64_ladder_planes(int digits) {
     return f.held;
 }
 
-bool Context::f64_ovvv_planes(int digits) {
+bool Context::f64_ovvv_planes(int digits, int64_t rows) {
     DigitFit &f = f64_ovvv_fit;
-    if (f.version == f64_version && f.digits == digits) return f.held;
+    if (f.version == f64_version && f.digits == digits && f.rows == rows) return f.held;
     f64_ovvv_dig.buf.release();
     const bool ladder = f64_ladder_digits() > 0;
     if (ladder) f64_ladder_planes(digits);   // first claim
     size_t free_b = 0, total_b = 0;
     CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    f.held = (!ladder || f64_ladder_fit.held) && digit_bytes(digits, no * nmo, nv * nv) <= 0.6 * (double)free_b;
-    if (f.held) ozaki_prepare(ex, false, no * nmo, nv * nv, f64_ovvv.d(), no * nmo, digits, f64_ovvv_dig);
+    f.held = (!ladder || f64_ladder_fit.held) && digit_bytes(digits, rows, nv * nv) <= 0.6 * (double)free_b;
+    if (f.held) ozaki_prepare(ex, false, rows, nv * nv, f64_ovvv.d(), no * nmo, digits, f64_ovvv_dig);
+    f.rows = rows;
     f.version = f64_version;
     f.digits = digits;
     cache_epoch++;
@@ -881,6 +882,16 @@ void Context::ladder_f64(const double *t2, double *om2) {
     add_omega_pm(ex, om2, wp.d(), wm.d(), no, nv, 1, 0, nv, nvp, nvm);
 }
 
+namespace {
+// the digit count of FP64 products within a scope
+struct DigitScope {
+    Exec &ex;
+    const int keep;
+    DigitScope(Exec &e, int digits) : ex(e), keep(e.fp64_digits) { ex.fp64_digits = digits; }
+    ~DigitScope() { ex.fp64_digits = keep; }
+};
+}  // namespace
+
 Context::LadderY Context::ladder_y_plain(const double *tf) {
     cudaStream_t s = ex.stream;
     const int64_t oo = no * no, nv2 = nv * nv;
@@ -897,11 +908,15 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
         own_q();
         return r;
     }
-    // Mixed precision: Q joins Y0's product only where the dispatch may run a product of its size on the tensor
-    // cores; smaller ones are FP64.  Where routes are timed both arithmetics are open to it, and joined costs
-    // least: a residual at o=13, v=107 1.07 ms, 1.13 with Q on the route that was fastest for it alone (DGEMM)
-    const bool joined = ex.prec != Prec::MIXED || gemm_may_take_tensor_cores(ex, oo, oo, nv2);
-    const int64_t rows = joined ? no * nmo : nov;
+    // Each of the two in the arithmetic that the dispatch gives a product of its size.  Mixed precision: Q joins
+    // Y0's product only where the tensor cores are open to it; smaller ones are FP64.  Where routes are timed both
+    // arithmetics are open, and joined costs least: a residual at o=13, v=107 1.07 ms, 1.13 with Q on the route
+    // that was fastest for it alone (DGEMM).  FP64: joined where both or neither go to the digit GEMM
+    const double fl_y = 2.0 * double(nov) * double(oo) * double(nv2), fl_q = 2.0 * double(oo) * double(oo) * double(nv2);
+    const bool y_digits = ex.prec == Prec::FP64 && gemm_takes_digits(ex, nov, oo, nv2, fl_y);
+    const bool q_digits = ex.prec == Prec::FP64 && gemm_takes_digits(ex, oo, oo, nv2, fl_q);
+    const bool joined = ex.prec == Prec::MIXED ? gemm_may_take_tensor_cores(ex, oo, oo, nv2) : y_digits == q_digits;
+    const int64_t rows = joined || ex.prec == Prec::FP64 ? no * nmo : nov;
     // t as [(c, d), (i, j)], the product [(k, p), (i, j)]
     DBuf W = dalloc(rows * oo, s);
     if (ex.prec == Prec::MIXED) {
@@ -929,13 +944,23 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
         dst.s[2] = nv;         // d
         dst.s[3] = nv2 * no;   // j
         permute_add(ex, 1.0, tv(tf, {nv, no, nv, no}), 0.0, dst);
-        const double fl = 2.0 * double(rows) * double(oo) * double(nv2);
-        if (gemm_takes_digits(ex, rows, oo, nv2, fl) && f64_ovvv_planes(ex.fp64_digits)) {
-            ozaki_gemm(ex, false, false, rows, oo, nv2, 1.0, f64_ovvv.d(), rows, TT.d(), nv2, 0.0, W.d(), rows,
-                       ex.fp64_digits, &f64_ovvv_dig, nullptr);
-            ex.flops += fl;
+        auto product = [&](int64_t r0, int64_t m, bool digits) {
+            const double *g = f64_ovvv.d() + r0;
+            double *w = W.d() + r0;
+            if (digits && r0 == 0 && f64_ovvv_planes(ex.fp64_digits, m)) {
+                ozaki_gemm(ex, false, false, m, oo, nv2, 1.0, g, rows, TT.d(), nv2, 0.0, w, rows, ex.fp64_digits,
+                           &f64_ovvv_dig, nullptr);
+                ex.flops += 2.0 * double(m) * double(oo) * double(nv2);
+                return;
+            }
+            DigitScope line(ex, digits ? ex.fp64_digits : 0);   // joined, Y0 and Q may pass a line that neither does
+            gemm(ex, false, false, m, oo, nv2, 1.0, g, rows, TT.d(), nv2, 0.0, w, rows, false);
+        };
+        if (joined) {
+            product(0, rows, y_digits);
         } else {
-            gemm(ex, false, false, rows, oo, nv2, 1.0, f64_ovvv.d(), rows, TT.d(), nv2, 0.0, W.d(), rows, false);
+            product(0, nov, y_digits);
+            product(nov, oo, q_digits);
         }
     }
     TV src = tv(W.d(), {no, no, nv, no});   // (k, i, b, j)
@@ -943,7 +968,7 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
     src.s[2] = no;
     src.s[3] = rows * no;
     permute_add(ex, 1.0, src, 0.0, tv(r.Y.d(), {no, no, nv, no}));
-    if (joined) {
+    if (rows > nov) {
         src.p += nov;                       // (k, i, l, j)
         src.n[2] = no;
         permute_add(ex, 1.0, src, 0.0, tv(r.Q.d(), {no, no, no, no}));

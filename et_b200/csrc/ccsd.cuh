@@ -203,11 +203,12 @@ struct Context {
     // integrals and g_kcpd (the row operands of their products), each kept per Cholesky set and digit count
     // while it fits; the ladder's have the first claim on the memory
     bool f64_ladder_planes(int digits);
-    bool f64_ovvv_planes(int digits);
+    bool f64_ovvv_planes(int digits, int64_t rows);   // of the first `rows` rows of f64_ovvv
     OzPlanes f64_gp_dig, f64_gm_dig, f64_ovvv_dig;
     struct DigitFit {
         int64_t version = -1;
         int digits = 0;
+        int64_t rows = 0;
         bool held = false;
     } f64_ladder_fit, f64_ovvv_fit;
     int davidson(int nstates, int side, const ccsd_gpu_davidson_options *o, double *omega_out, double *vectors_out,

@@ -52,3 +52,21 @@ def test_small_products_stay_fp64(n_o, n_v):
     ref = _omega((L, h, eps), t, n_o, n_v, 7, precision=FP64)
     out = _omega((L, h, eps), t, n_o, n_v, 7, precision=MIXED, mixed_min_flops=10 ** 15)
     assert np.linalg.norm(out - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+def test_small_products_stay_on_dgemm():
+    """Products below the line of set_fp64_digits stay on DGEMM, Q and X_klij among them.  A virtual pair of two
+    odd orbitals has integrals of 2^-40, one of two even orbitals integrals of 1, and only the former meet
+    amplitudes: in the rows of every other product a row's integrals have one size, in those of Q (k, l) both
+    occur and four digits keep the larger only."""
+    n_o, n_v = 16, 48
+    rng, L, h, eps, t = _system(n_o, n_v, 2, 5)
+    odd = np.arange(n_v) % 2 == 1
+    a = rng.integers(0, 2, (n_o, n_v)) * 2.0 - 1.0
+    L[0, :n_o, n_o:], L[1, :n_o, n_o:] = np.where(odd, 0.0, a), np.where(odd, 2.0 ** -20 * a, 0.0)
+    M, m = np.tril_indices(n_o * n_v)
+    t[n_o * n_v:] *= odd[M % n_v] & odd[m % n_v]
+    # the line lies between Q (3.0e8 flops) and the products over n_o n_v (9.1e8)
+    out = _omega((L, h, eps), t, n_o, n_v, 2, digits=4, min_flops=5e8)
+    ref = _omega((L, h, eps), t, n_o, n_v, 2)
+    assert np.linalg.norm(out - ref) <= 1e-12 * np.linalg.norm(ref)
