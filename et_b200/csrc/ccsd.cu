@@ -255,8 +255,15 @@ DBuf Context::g_ovov() {
     return g;
 }
 
+// Guard of everything kept per Cholesky set: formed inside a capture, its buffer would belong to the graph while
+// the host takes it for filled.  prepare_residual_caches forms it before.
+void Context::not_captured() {
+    REQUIRE(!ex.capturing, CCSD_GPU_ESTATE, "integrals kept per Cholesky set would be formed inside a graph capture");
+}
+
 const double *Context::g_ovov_const() {
     if (!have_gov) {
+        not_captured();
         const Prec keep = ex.prec;
         ex.prec = Prec::FP64;
         gov = g_ovov();
@@ -277,6 +284,7 @@ const double *Context::g_ovov_const() {
 void Context::g_pairs_const() {
     const double *g = g_ovov_const();
     if (hov && gov_pairs_id == gov_id) return;
+    not_captured();
     if (!hov) {
         hov = dalloc(nov * nov, ex.stream);
         gex = dalloc(nov * nov, ex.stream);
@@ -500,6 +508,7 @@ void Context::ladder_pairs(const double *Lvv, bool untransformed) {
     if (!untransformed && pairs_reuse_id >= 0 && mbuf_kind == 2 && mbuf_reuse == pairs_reuse_id &&
         mbuf_src == Lvv && mbuf_version == l_version && mbuf_planes == np)
         return;
+    not_captured();
     cudaStream_t s = ex.stream;
     const PairShape ps = pair_shape(nv);
     const size_t bytes = sizeof(__nv_bfloat16) * np * (ps.plane_p() + ps.plane_m());
@@ -650,6 +659,7 @@ bool Context::ovvv_resident() {
 void Context::ovvv_pairs() {
     const int np = ex.planes;
     if (ybuf_version == l_version && ybuf_planes == np) return;
+    not_captured();
     cudaStream_t s = ex.stream;
     const int64_t nv2 = nv * nv, Jp = tc_pad_k(nJ), Kq = tc_pad_k(nv2);
     // L_ov split rows c + nv*k: L_ov[J, k, c] sits at J + nJ*(k + no*c); copy to (J, c, k) first
@@ -766,6 +776,7 @@ bool Context::f64_resident() {
 
 void Context::f64_integrals() {
     if (f64_version == l_version) return;
+    not_captured();
     cudaStream_t s = ex.stream;
     const Prec keep = ex.prec;
     ex.prec = Prec::FP64;
@@ -816,6 +827,7 @@ double digit_bytes(int digits, int64_t rows, int64_t k) {
 bool Context::f64_ladder_planes(int digits) {
     DigitFit &f = f64_ladder_fit;
     if (f.version == f64_version && f.digits == digits) return f.held;
+    not_captured();
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
     for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig}) p->buf.release();
     size_t free_b = 0, total_b = 0;
@@ -834,6 +846,7 @@ bool Context::f64_ladder_planes(int digits) {
 bool Context::f64_ovvv_planes(int digits, int64_t rows) {
     DigitFit &f = f64_ovvv_fit;
     if (f.version == f64_version && f.digits == digits && f.rows == rows) return f.held;
+    not_captured();
     f64_ovvv_dig.buf.release();
     const bool ladder = f64_ladder_digits() > 0;
     if (ladder) f64_ladder_planes(digits);   // first claim
@@ -892,6 +905,18 @@ struct DigitScope {
 };
 }  // namespace
 
+// Each of the two in the arithmetic that the dispatch gives a product of its size.  Mixed precision: Q joins Y0's
+// product only where the tensor cores are open to it; smaller ones are FP64.  Where routes are timed both
+// arithmetics are open, and joined costs least: a residual at o=13, v=107 1.07 ms, 1.13 with Q on the route that
+// was fastest for it alone (DGEMM).  FP64: joined where both or neither go to the digit GEMM.
+Context::YqRoute Context::yq_route() const {
+    const int64_t oo = no * no, nv2 = nv * nv;
+    if (ex.prec == Prec::MIXED) return {gemm_may_take_tensor_cores(ex, oo, oo, nv2), false, false};
+    const double fl_y = 2.0 * double(nov) * double(oo) * double(nv2), fl_q = 2.0 * double(oo) * double(oo) * double(nv2);
+    const bool y = gemm_takes_digits(ex, nov, oo, nv2, fl_y), q = gemm_takes_digits(ex, oo, oo, nv2, fl_q);
+    return {y == q, y, q};
+}
+
 Context::LadderY Context::ladder_y_plain(const double *tf) {
     cudaStream_t s = ex.stream;
     const int64_t oo = no * no, nv2 = nv * nv;
@@ -908,14 +933,7 @@ Context::LadderY Context::ladder_y_plain(const double *tf) {
         own_q();
         return r;
     }
-    // Each of the two in the arithmetic that the dispatch gives a product of its size.  Mixed precision: Q joins
-    // Y0's product only where the tensor cores are open to it; smaller ones are FP64.  Where routes are timed both
-    // arithmetics are open, and joined costs least: a residual at o=13, v=107 1.07 ms, 1.13 with Q on the route
-    // that was fastest for it alone (DGEMM).  FP64: joined where both or neither go to the digit GEMM
-    const double fl_y = 2.0 * double(nov) * double(oo) * double(nv2), fl_q = 2.0 * double(oo) * double(oo) * double(nv2);
-    const bool y_digits = ex.prec == Prec::FP64 && gemm_takes_digits(ex, nov, oo, nv2, fl_y);
-    const bool q_digits = ex.prec == Prec::FP64 && gemm_takes_digits(ex, oo, oo, nv2, fl_q);
-    const bool joined = ex.prec == Prec::MIXED ? gemm_may_take_tensor_cores(ex, oo, oo, nv2) : y_digits == q_digits;
+    const auto [joined, y_digits, q_digits] = yq_route();
     const int64_t rows = joined || ex.prec == Prec::FP64 ? no * nmo : nov;
     // t as [(c, d), (i, j)], the product [(k, p), (i, j)]
     DBuf W = dalloc(rows * oo, s);

@@ -101,13 +101,24 @@ struct Context {
     int64_t mbuf_reuse = -1;            // the prepared id they were formed for
 
     // The residual evaluation captured as a CUDA graph, one per precision.  The first evaluation in
-    // a precision runs eagerly (it builds the caches and times the GEMM routes); later ones replay
-    // a graph captured for the same Cholesky set, caches and GEMM settings, which writes om_stage.
+    // a precision, or with other digits, runs eagerly (it builds the caches, times the GEMM routes and sizes
+    // the digit arena); later ones replay a graph captured for the same Cholesky set, caches and GEMM settings,
+    // which writes om_stage.
     struct ResidualGraph {
         cudaGraphExec_t exec = nullptr;
         bool warm = false;
-        int64_t l_version = -1, cache_epoch = -1, k_chunk = 0;
-        int planes = 0;
+        // what the captured kernels and pointers depend on
+        struct Key {
+            int64_t l_version = -1, cache_epoch = -1, k_chunk = 0;
+            int planes = 0, digits = 0;
+            double digits_min_flops = 0.0;
+            const void *arena = nullptr;
+            bool operator==(const Key &o) const {
+                return l_version == o.l_version && cache_epoch == o.cache_epoch && k_chunk == o.k_chunk &&
+                       planes == o.planes && same_digits(o) && arena == o.arena;
+            }
+            bool same_digits(const Key &o) const { return digits == o.digits && digits_min_flops == o.digits_min_flops; }
+        } key;
         int64_t launches = 0;
         double flops = 0.0;
         void reset() {
@@ -154,9 +165,16 @@ struct Context {
     // mixed precision: whether the resident ovvv planes fit, and their construction
     bool ovvv_resident();
     void ovvv_pairs();
+    void not_captured();                     // throws while a residual graph is being captured
+    ResidualGraph::Key graph_key() const;
     // whether the current precision evaluates the residual's ladder from untransformed integrals, and Y0
     // and Q from whatever integrals it keeps, in one product where the planes or blocks are resident
     bool plain_ladder() { return ex.prec == Prec::MIXED || f64_resident(); }
+    // how ladder_y_plain evaluates the two: in one product or each by itself, FP64 ones on digits or DGEMM
+    struct YqRoute {
+        bool joined, y_digits, q_digits;
+    };
+    YqRoute yq_route() const;
     LadderY ladder_y_plain(const double *tfull);
     // Y with the T1-transformed vv block Ltvv, sum_cd g_kc~bd tau_cidj: Y0_kibj - sum_l t_bl Q_kilj from the
     // residual's Y0 and Q (yq, may be empty) or resident integrals, else ladder_y(Ltvv)

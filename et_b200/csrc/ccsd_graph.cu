@@ -368,7 +368,16 @@ void Context::prepare_residual_caches() {
         if (ovvv_resident()) ovvv_pairs();
     } else if (f64_resident()) {
         f64_integrals();
+        const int digits = f64_ladder_digits();
+        if (digits) f64_ladder_planes(digits);
+        const YqRoute yq = yq_route();
+        if (yq.y_digits) f64_ovvv_planes(ex.fp64_digits, yq.joined ? no * nmo : nov);
     }
+}
+
+Context::ResidualGraph::Key Context::graph_key() const {
+    return {l_version, cache_epoch, ex.k_chunk, ex.planes, ex.fp64_digits, ex.fp64_digits_min_flops,
+            digit_arena.as<void>()};
 }
 
 // Records the residual on ex.stream into G.  A capture that fails (a call that cannot be captured)
@@ -381,11 +390,13 @@ void Context::capture_residual(ResidualGraph &G, double *om_out) {
     cudaGraph_t graph = nullptr;
     std::string why;
     CU_CHECK(cudaStreamBeginCapture(ex.stream, cudaStreamCaptureModeThreadLocal));
+    ex.capturing = true;
     try {
         omega_eager(om_out);
     } catch (const std::exception &e) {
         why = e.what();
     }
+    ex.capturing = false;
     cudaError_t rc = cudaStreamEndCapture(ex.stream, &graph);
     if (why.empty() && rc == cudaSuccess && graph) {
         rc = cudaGraphInstantiate(&G.exec, graph, 0);
@@ -403,10 +414,7 @@ void Context::capture_residual(ResidualGraph &G, double *om_out) {
     G.launches = ex.launches - launches0;
     ex.flops = flops0;
     ex.launches = launches0;
-    G.l_version = l_version;
-    G.cache_epoch = cache_epoch;
-    G.planes = ex.planes;
-    G.k_chunk = ex.k_chunk;
+    G.key = graph_key();
 }
 
 void Context::omega(double *om_out) {
@@ -421,15 +429,15 @@ void Context::omega(double *om_out) {
     } else {
         prepare_residual_caches();
         ResidualGraph &G = rgraph[ex.prec == Prec::MIXED ? 1 : 0];
-        if (!G.warm) {
+        if (!G.warm || !G.key.same_digits(graph_key())) {
             omega_eager(om_out);
+            G.reset();
+            G.key = graph_key();
             G.warm = true;
         } else {
             // the graph writes a buffer of its own, so callers may pass any output
             if (!om_stage) om_stage = dalloc(namp, ex.stream);
-            const bool match = G.exec && G.l_version == l_version && G.cache_epoch == cache_epoch &&
-                               G.planes == ex.planes && G.k_chunk == ex.k_chunk;
-            if (!match) capture_residual(G, om_stage.d());
+            if (!(G.exec && G.key == graph_key())) capture_residual(G, om_stage.d());
             if (G.exec) {
                 CU_CHECK(cudaGraphLaunch(G.exec, ex.stream));
                 CU_CHECK(cudaMemcpyAsync(om_out, om_stage.d(), sizeof(double) * namp, cudaMemcpyDeviceToDevice,

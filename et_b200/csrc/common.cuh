@@ -177,6 +177,8 @@ struct Exec {
     double fp64_digits_min_flops = 1e10;
     // digits of the first-order (FP64) terms inside a mixed-precision residual (0: cuBLAS DGEMM)
     int mixed_fp64_digits = 6;
+    // the stream is being captured into a residual graph: what outlives the evaluation is neither formed nor grown
+    bool capturing = false;
     // grow-only scratch of the digit GEMM (digit planes and exponents), owned by the context: the
     // multi-GB planes are neither allocated nor freed per product
     DBuf *digit_arena = nullptr;

@@ -962,7 +962,8 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     const size_t digit_bytes = round_up(a_bytes + b_bytes, (size_t)256);
     const size_t need = exp_bytes + digit_bytes + (pair ? sizeof(double) * OBM * WBN * (size_t)(2 * max_pairs) : 0);
     DBuf local;
-    DBuf *arena = ex.digit_arena ? ex.digit_arena : &local;
+    // a buffer grown inside a capture would belong to the graph: there a small arena is left alone
+    DBuf *arena = ex.digit_arena && !(ex.capturing && ex.digit_arena->bytes() < need) ? ex.digit_arena : &local;
     if (arena->bytes() < need) {
         arena->release();
         arena->alloc(need, ex.stream);

@@ -82,3 +82,29 @@ def test_solver_with_graphs_matches_eager_solver(prec_name):
     assert np.array_equal(g.get_amplitudes(), e.get_amplitudes())
     g.close()
     e.close()
+
+
+def test_digits_may_change_between_replays():
+    """Digits set after a capture, other digits, new Cholesky vectors and a digit product that outgrows the arena
+    between replays: each evaluation equals the eager one."""
+    from et_b200 import FP64
+    s, g, e = _pair(FP64, dims=(17, 40, 60))
+    rng = np.random.default_rng(2)
+    t, c = 0.02 * rng.standard_normal(g.n_amp), rng.standard_normal((g.n_amp, 3))
+    steps = [None, (6, 1e8), (4, 1.0), (4, 1e8), s.L_mo * 1.01, (0, 0.0), (7, 1.0)]
+    for step in steps:
+        for x in (g, e):
+            if isinstance(step, tuple):
+                x.set_fp64_digits(*step)
+            elif step is not None:
+                x.set_cholesky_mo(step)
+            x.set_amplitudes(t)
+        for k in range(4):
+            replays = g.graph_stats()[0]
+            assert np.array_equal(g.construct_omega(), e.construct_omega()), (step, k)
+            # the first evaluation with other digits is eager
+            assert g.graph_stats()[0] - replays == (0 if k == 0 and not isinstance(step, np.ndarray) else 1)
+            if k == 2:
+                assert np.array_equal(g.jacobian_transformation(c), e.jacobian_transformation(c))
+    g.close()
+    e.close()
