@@ -591,7 +591,7 @@ void Context::ladder_tc(const double *Lvv, const double *t2, double *om2, int64_
 // The same ladder with bounded memory: the g+- planes of a block of consecutive a are formed into
 // one buffer and contracted right away (omega_ccsd_a2's (a, b) batching on the tensor cores,
 // omega_ccsd.F90:236-458).  Every output element is the dot product it is in the resident form (the
-// same planes, one K split, the same K chunks), so the result equals the resident ladder's bit for bit.
+// same planes, K splits and K chunks), so the result equals the resident ladder's bit for bit.
 void Context::ladder_tc_streamed(const double *Lvv, const double *t2, double *om2, int64_t nvec) {
     cudaStream_t s = ex.stream;
     const int np = ex.planes;
@@ -599,8 +599,13 @@ void Context::ladder_tc_streamed(const double *Lvv, const double *t2, double *om
     const int64_t ldp = nvec * (no * (no + 1) / 2), ldm = std::max<int64_t>(nvec * (no * (no - 1) / 2), 1);
     DBuf LT = lvv_jca(Lvv);
     const TPlanes T = t_planes(t2, nvec);
-    // blocks: consecutive a whose G, planes and W fit the budget (or a quarter of the free memory),
-    // at least one a each
+    // blocks: consecutive a whose G, planes, W and the partial products of a W in K splits (one sign at a time)
+    // fit the budget (or a quarter of the free memory), at least one a each
+    const auto partials = [&](int64_t nvx, int64_t n, int64_t kx) {
+        const int splits = tc_tall_route(nvx, n, kx, np) % PAIR_ROUTE;
+        return splits > 1 ? splits * double(n) : 0.0;
+    };
+    const double part_p = partials(ps.nvp, ldp, ps.kp), part_m = partials(ps.nvm, ldm, ps.km);
     int64_t budget = ladder_pair_budget;
     if (budget <= 0) {
         size_t free_b = 0, total_b = 0;
@@ -611,7 +616,7 @@ void Context::ladder_tc_streamed(const double *Lvv, const double *t2, double *om
         const int64_t nabp = a1 * (a1 + 1) / 2 - a0 * (a0 + 1) / 2, nabm = a1 * (a1 - 1) / 2 - a0 * (a0 - 1) / 2;
         return 8.0 * double(nv * (a1 - a0)) * double(nv * a1) +
                2.0 * np * (double(tc_pad_rows_b(nabp)) * ps.kp + double(tc_pad_rows_b(std::max<int64_t>(nabm, 1))) * ps.km) +
-               8.0 * (double(ldp) * nabp + double(ldm) * nabm);
+               8.0 * (double(ldp) * nabp + double(ldm) * nabm + std::max(part_p * nabp, part_m * nabm));
     };
     std::vector<std::pair<int64_t, int64_t>> blocks;
     int64_t g_max = 0, prow_max = 0, mrow_max = 0;

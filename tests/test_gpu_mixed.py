@@ -215,12 +215,13 @@ def test_mixed_singles_jacobian_with_t1_matches_fp64(dims):
                 assert err <= 1e-3 * ladder_t1, (err, ladder_t1)
 
 
-@pytest.mark.parametrize("dims", [(5, 19, 33), (6, 40, 90)])
+@pytest.mark.parametrize("dims", [(5, 19, 33), (6, 40, 90), (7, 64, 50), (11, 61, 40)])
 def test_streamed_ladder_equals_resident(dims):
     """A pair-integral budget below the resident size forms the split-bf16 ladder integrals block by
-    block in every call (eT's (a, b) batching).  With one K split (the fixed GEMM rule) every output
-    element is the same dot product, so Omega, A c and A^T b equal the resident form's bit for bit,
-    for one a per block (budget 1 byte) and for blocks of several a."""
+    block in every call (eT's (a, b) batching).  The K splits depend on the whole ladder only, so every
+    output element is the same dot product and Omega, A c and A^T b equal the resident form's bit for
+    bit, for one a per block (budget 1 byte) and for blocks of several a; from n_v = 46 on the ladder
+    has K blocks enough for several splits."""
     from et_b200 import CCSD, MIXED
     n_o, n_v, n_J = dims
     s = make_system(n_o, n_v, n_J, seed=23)
@@ -237,6 +238,41 @@ def test_streamed_ladder_equals_resident(dims):
     for budget in list(res)[1:]:
         for x, y in zip(res[0], res[budget]):
             assert np.array_equal(x, y), budget
+
+
+def test_streamed_ladder_keeps_to_its_budget():
+    """No fewer blocks than keep each one's G, planes, W and partial products within the budget (n_o = 24,
+    n_v = 48: two K splits of the 300 and 276 columns).  A block is three tensor-core products: G and one per
+    sign, the block of a = 0 alone two."""
+    from et_b200 import CCSD, MIXED
+    n_o, n_v, n_J, budget = 24, 48, 30, 6 << 20
+    s = make_system(n_o, n_v, n_J, seed=7)
+    gemms = {}
+    for b in (1, budget):
+        with CCSD(n_o, n_v, n_J, precision=MIXED, mixed_min_flops=1, ladder_pair_budget=b) as g:
+            g.set_system(s.L_mo, s.h_mo, s.eps)
+            g.set_initial_amplitudes_guess()
+            g.construct_omega()
+            g.set_profiling(True)
+            g.construct_omega()
+            gemms[b] = g.gemm_profile()[0]
+    blocks = n_v + (gemms[budget] - gemms[1] - 1) // 3
+
+    def pairs(a0, a1, sign):
+        return (a1 * (a1 + sign) - a0 * (a0 + sign)) // 2
+
+    def size(a0, a1):
+        n = 8 * n_v * (a1 - a0) * n_v * a1
+        for sign in (1, -1):   # two planes of whole tiles of 256 rows and 64 K positions
+            n += 4 * (-(-pairs(a0, a1, sign) // 256) * 256) * (-(-pairs(0, n_v, sign) // 64) * 64)
+        w = [8 * pairs(0, n_o, sign) * pairs(a0, a1, sign) for sign in (1, -1)]
+        return n + sum(w) + 2 * max(w)
+
+    least, a0 = 0, 0
+    while a0 < n_v:
+        a0 = max([a0 + 1] + [a1 for a1 in range(a0 + 1, n_v + 1) if size(a0, a1) <= budget])
+        least += 1
+    assert blocks >= least
 
 
 def test_gathered_operands_equal_reordered_copies():
