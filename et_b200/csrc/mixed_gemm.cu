@@ -700,7 +700,7 @@ struct RowSplit {
 
 // np planes of x (each the bf16 rounding of what the planes before it leave, the differences in FP64)
 __device__ __forceinline__ __nv_bfloat16 take_plane(double &x) {
-    const __nv_bfloat16 h = __float2bfloat16((float)x);
+    const __nv_bfloat16 h = __double2bfloat16(x);   // by way of FP32 a value next to a tie would be rounded twice
     x -= (double)__bfloat162float(h);
     return h;
 }
