@@ -837,7 +837,10 @@ bool Context::f64_ladder_planes(int digits) {
     for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig}) p->buf.release();
     size_t free_b = 0, total_b = 0;
     CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    f.held = digit_bytes(digits, nvp, nvp) + (nvm > 0 ? digit_bytes(digits, nvm, nvm) : 0.0) <= 0.6 * (double)free_b;
+    const double need = digit_bytes(digits, nvp, nvp) + (nvm > 0 ? digit_bytes(digits, nvm, nvm) : 0.0);
+    f.room = 0.6 * (double)free_b;
+    f.held = need <= f.room;
+    if (f.held) f.room -= need;
     if (f.held) {
         ozaki_prepare(ex, true, nvp, nvp, f64_gp.d(), nvp, digits, f64_gp_dig);
         if (nvm > 0) ozaki_prepare(ex, true, nvm, nvm, f64_gm.d(), nvm, digits, f64_gm_dig);
@@ -857,7 +860,9 @@ bool Context::f64_ovvv_planes(int digits, int64_t rows) {
     if (ladder) f64_ladder_planes(digits);   // first claim
     size_t free_b = 0, total_b = 0;
     CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    f.held = (!ladder || f64_ladder_fit.held) && digit_bytes(digits, rows, nv * nv) <= 0.6 * (double)free_b;
+    f.room = 0.6 * (double)free_b;
+    if (ladder) f.room = f64_ladder_fit.held ? std::min(f.room, f64_ladder_fit.room) : 0.0;
+    f.held = digit_bytes(digits, rows, nv * nv) <= f.room;
     if (f.held) ozaki_prepare(ex, false, rows, nv * nv, f64_ovvv.d(), no * nmo, digits, f64_ovvv_dig);
     f.rows = rows;
     f.version = f64_version;

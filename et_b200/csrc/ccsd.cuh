@@ -219,7 +219,7 @@ struct Context {
     void ladder_f64(const double *t2, double *om2);
     // digit planes of the resident FP64 integrals for FP64 evaluations on the int8 digit GEMM: the +/- ladder
     // integrals and g_kcpd (the row operands of their products), each kept per Cholesky set and digit count
-    // while it fits; the ladder's have the first claim on the memory
+    // while they fit: together in 0.6 of the memory that is free before the first, the ladder's first
     bool f64_ladder_planes(int digits);
     bool f64_ovvv_planes(int digits, int64_t rows);   // of the first `rows` rows of f64_ovvv
     OzPlanes f64_gp_dig, f64_gm_dig, f64_ovvv_dig;
@@ -227,6 +227,7 @@ struct Context {
         int64_t version = -1;
         int digits = 0;
         int64_t rows = 0;
+        double room = 0.0;   // bytes of the bound that are left
         bool held = false;
     } f64_ladder_fit, f64_ovvv_fit;
     int davidson(int nstates, int side, const ccsd_gpu_davidson_options *o, double *omega_out, double *vectors_out,

@@ -368,10 +368,10 @@ void Context::prepare_residual_caches() {
         if (ovvv_resident()) ovvv_pairs();
     } else if (f64_resident()) {
         f64_integrals();
-        const int digits = f64_ladder_digits();
-        if (digits) f64_ladder_planes(digits);
         const YqRoute yq = yq_route();
         if (yq.y_digits) f64_ovvv_planes(ex.fp64_digits, yq.joined ? no * nmo : nov);
+        const int digits = f64_ladder_digits();
+        if (digits) f64_ladder_planes(digits);
     }
 }
 

@@ -68,3 +68,31 @@ def test_resident_fp64_integrals_follow_new_cholesky_vectors():
         g.set_amplitudes(amp)
         om = g.construct_omega()
     assert np.abs(om - ref.omega()).max() <= 1e-12 * max(1.0, np.abs(ref.omega()).max())
+
+
+def test_digit_planes_share_one_bound():
+    """The ladder's digit planes (305 MB) and those of g_kcpd (185 MB) stay only where both fit in 0.6 of the free
+    memory: with 650 MB free g_kcpd is converted in every residual, with the whole device free in none."""
+    import torch
+    from et_b200 import CCSD, FP64
+    n_o, n_v, n_J = 24, 100, 30
+    s = make_system(n_o, n_v, n_J, seed=9)
+    launches, out = [], []
+    for free in (650e6, None):
+        with CCSD(n_o, n_v, n_J, precision=FP64) as g:
+            g.set_system(s.L_mo, s.h_mo, s.eps)
+            g.set_initial_amplitudes_guess()
+            g.construct_omega()
+            rest = None
+            if free:
+                torch.cuda.empty_cache()
+                rest = torch.empty(int(torch.cuda.mem_get_info()[0] - free), dtype=torch.uint8, device="cuda")
+            g.set_fp64_digits(6, 1e8)
+            g.construct_omega()
+            n = g.stats()[0]
+            out.append(g.construct_omega())
+            launches.append(g.stats()[0] - n)
+            del rest
+            torch.cuda.empty_cache()
+    assert np.array_equal(*out)
+    assert launches[0] > launches[1]
