@@ -516,12 +516,16 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                         for (int kb = kb0; kb < kb1; kb++) {
                             const bool first = kb == kb0;
                             bool ok = false;
-#define OZ_UNIT(ND, NDIAG)                                                                                                  case 8 * ND + NDIAG:                                                                                                       ok = issue_unit<ND, NDIAG>(tmem, wide ? WBN : WBN / 2, desc0, slot_bytes, full, empty, r, idesc, first, map.wait_cycles);          break;
+#define OZ_UNIT(ND, NDIAG)                                                                                        \
+    case 8 * ND + NDIAG:                                                                                          \
+        ok = issue_unit<ND, NDIAG>(tmem, wide ? WBN : WBN / 2, desc0, slot_bytes, full, empty, r, idesc, first,   \
+                                   map.wait_cycles);                                                              \
+        break;
                             switch (8 * nd + diags) {
-                                // two at a time: 2, 4, 6 digits, or the last diagonal of 3, 5, 7
-                                OZ_UNIT(2, 2) OZ_UNIT(4, 2) OZ_UNIT(6, 2) OZ_UNIT(3, 1) OZ_UNIT(5, 1) OZ_UNIT(7, 1)
-                                // four at a time: up to four digits, then the rest of 6 or 7
-                                OZ_UNIT(3, 3) OZ_UNIT(4, 4) OZ_UNIT(7, 3)
+                                // two at a time: 2, 4, 6 digits, or the last diagonal of 5, 7
+                                OZ_UNIT(2, 2) OZ_UNIT(4, 2) OZ_UNIT(6, 2) OZ_UNIT(5, 1) OZ_UNIT(7, 1)
+                                // four at a time: four digits, then the rest of 6 or 7
+                                OZ_UNIT(4, 4) OZ_UNIT(7, 3)
                             }
 #undef OZ_UNIT
                             if (!ok || *abort_flag) {
@@ -871,7 +875,7 @@ int pair_n_tile(int64_t mt, int64_t n, int digits, int64_t pairs) {
 void ozaki_prepare(Exec &ex, bool trans, int64_t rows, int64_t k, const double *X, int64_t ldx, int digits,
                    OzPlanes &out) {
     REQUIRE(rows > 0 && k > 0 && rows < (1ll << 31) && k < (1ll << 31), CCSD_GPU_EINVAL, "ozaki_prepare: bad size");
-    REQUIRE(digits >= 2 && digits <= SLOTS, CCSD_GPU_EINVAL, "ozaki_prepare: 2 to 7 digits");
+    REQUIRE(digits >= 4 && digits <= SLOTS, CCSD_GPU_EINVAL, "ozaki_prepare: 4 to 7 digits");
     // rows of op(X): X[r + ldx kk] (N) or X[kk + ldx r] (T), padded to 128 (either operand's tiles)
     const int64_t sr = trans ? ldx : 1, sk = trans ? 1 : ldx;
     const int64_t Rp = round_up(rows, (int64_t)OBM), Kp = round_up(k, (int64_t)OBK);
@@ -901,7 +905,7 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     REQUIRE(!pb || (pb->digits == digits && pb->rows == n && pb->k == k), CCSD_GPU_EINVAL,
             "ozaki_gemm: prepared B does not match");
     REQUIRE(m < (1ll << 31) && n < (1ll << 31) && k < (1ll << 31), CCSD_GPU_EINVAL, "ozaki_gemm: size too large");
-    REQUIRE(digits >= 2 && digits <= SLOTS, CCSD_GPU_EINVAL, "ozaki_gemm: 2 to 7 digits");
+    REQUIRE(digits >= 4 && digits <= SLOTS, CCSD_GPU_EINVAL, "ozaki_gemm: 4 to 7 digits");
     REQUIRE(ex.gemm_err != nullptr, CCSD_GPU_EINVAL, "ozaki_gemm: no error word");
     const int64_t Mp = round_up(m, OBM), Np = round_up(n, OBN);
     // op(A)(r, kk): A[r + lda kk] (N) or A[kk + lda r] (T); op(B)(kk, c) rows c: B[kk + ldb c] (N) or B[c + ldb kk] (T)
@@ -916,8 +920,7 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     }();
     const bool pair = pairs_on && m > OBM;
     auto kernel = digits == 7 ? ozaki_gemm_kernel<7> : digits == 6 ? ozaki_gemm_kernel<6>
-                : digits == 5 ? ozaki_gemm_kernel<5> : digits == 4 ? ozaki_gemm_kernel<4>
-                : digits == 3 ? ozaki_gemm_kernel<3> : ozaki_gemm_kernel<2>;
+                : digits == 5 ? ozaki_gemm_kernel<5> : ozaki_gemm_kernel<4>;
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OSMEM));
     CU_CHECK(cudaFuncSetAttribute(ozaki_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WSMEM));
     const int nsm = num_sms();
