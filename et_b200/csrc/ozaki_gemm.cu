@@ -299,31 +299,36 @@ ozaki_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
 }
 
-// The digit GEMM on a pair of CTAs (a cluster of two) with 256-wide N tiles: one cta_group::2 MMA of
-// M = 256 (each CTA's 128 rows of A) and N up to 256 (half of B's rows staged by each CTA).
+// The digit GEMM on a pair of CTAs (a cluster of two) with N tiles of up to 256 columns: one cta_group::2 MMA of
+// M = 256 (each CTA's 128 rows of A) and N = bn (half of B's rows staged by each CTA).
 //
 // What bounds it is shared memory, 128 bytes a cycle: an MMA of N = bn reads 4 KB of A and 32 bn bytes of B in
 // bn / 2 cycles, so a 128-wide tile, its two passes staging ten digit tiles a K block on top, kept the int8
 // pipe 67 % active.  At 256 columns the MMAs need 96 bytes a cycle and the staging 37, but TMEM then holds two
-// accumulators: the diagonals are taken two at a time, each such unit staging the digits up to its higher
-// diagonal (2 + 4 + 6 digit tiles a K block for six digits); tiles of at most 128 columns keep four.  What
-// keeps that rate up at L2's latency is bytes in flight: the ring's slots hold one digit of A and of B, the
-// products of a K block run from its highest digit down, and a slot is freed when its digit has taken part for
-// the last time (freeing a whole K block at once left 96 of the 192 KB idle: 2.1 instead of 2.7 POPS at
-// 4000^3).  Eight epilogue warps drain a unit (the accumulators are not double-buffered), old values a step
-// ahead.
+// accumulators: wide tiles (more than 128 columns) take the diagonals two at a time, each such unit staging the
+// digits up to its higher diagonal (2 + 4 + 6 digit tiles a K block for six digits); narrow ones four.  What
+// keeps the rate of wide tiles up at L2's latency is bytes in flight: their ring's slots hold one digit of A and
+// of B, the products of a K block run from its highest digit down, and a slot is freed when its digit has taken
+// part for the last time (freeing a whole K block at once left 96 of the 192 KB idle: 2.1 instead of 2.7 POPS
+// at 4000^3).  Narrow tiles have too few cycles of products per digit to hide ten waits and commits a K block:
+// their slots hold all its digits (4000 x 400 x 40000 1.68 ms with a slot per digit, 1.27 so).  Eight epilogue
+// warps drain a unit (the accumulators are not double-buffered), old values a step ahead.
 //
 // The sums keep the order of the single-CTA kernel, diagonals 0..3 and then 4..S-1 per K chunk: the sum of a
 // pass is exact in FP64 (four diagonals span 52 bits), so the units of a pass before its last leave their
 // share in a scratch of the CTA and the last adds it, and only then the scaled sum is rounded into the output.
-// With 6 digits, against the 128-wide pair kernel before it: 10240 x 10240 x 1200 2.65 ms (3.94), 4000^3 1.00 ms
-// (1.20), 4400 x 400 x 40000 1.64 ms (1.63 on single CTAs).
+// With 6 digits, against 128-wide pair tiles with one K block a stage: 10240 x 10240 x 1200 2.70 ms (3.94), 4000^3
+// 1.02 ms (1.27), 4000 x 400 x 40000 1.27 ms (1.36), 2304 x 256 x 16384 0.48 ms (0.51).
 constexpr int WBN = 256;
-constexpr int WRING = 12 * (A_TILE + (WBN / 2) * OBK);           // bytes of the ring of slots
-constexpr int WSLOTS = 20;                                        // slots at most (16 of a 128-wide tile)
+constexpr int WSLOTS = 20;                                        // slots at most
 constexpr int WEPI_WARPS = 8, WTHREADS = 64 + 32 * WEPI_WARPS;
-constexpr int WSMEM = WRING + 1024 + 512 + WEPI_WARPS * (WBN / 2) * 8;
-static_assert(WSMEM <= 232448, "shared memory of the wide digit GEMM");
+// WIDE: tiles of more than 128 columns
+template <bool WIDE>
+struct PairRing {
+    static constexpr int BYTES = WIDE ? 12 * (A_TILE + (WBN / 2) * OBK) : 18 * (A_TILE + (WBN / 4) * OBK);
+    static constexpr int SMEM = BYTES + 1024 + 512 + WEPI_WARPS * (WBN / 2) * 8;
+};
+static_assert(PairRing<true>::SMEM <= 232448 && PairRing<false>::SMEM <= 232448, "shared memory of the pair digit GEMM");
 constexpr uint32_t WIDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 4) << 24);
 
 __device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -358,29 +363,39 @@ struct Ring {
     }
 };
 
-// Waits for the slots of one K block (from ring position r) and issues its products of the NDIAG diagonals
+// Waits for one K block (from ring position r) and issues its products of the NDIAG diagonals
 // ND - NDIAG .. ND - 1 (accumulator d - (ND - NDIAG), each `width` columns), from the products of the highest
 // digit down: step k pairs digit ND - 1 - k with the lower ones, so digit ND - 1 - k is free after step k and
-// digit j after step j + NDIAG - 1.  False when a wait ran out.
-template <int ND, int NDIAG>
-__device__ __forceinline__ bool issue_unit(uint32_t tmem, uint32_t width, uint64_t desc0, int slot_bytes, uint64_t *full, uint64_t *empty,
-                                           const Ring &r, uint32_t idesc, bool first_kb, long long limit) {
+// digit j after step j + NDIAG - 1.  BLOCK: the K block's digits share one slot, slot_bytes apart; else each has
+// its own.  False when a wait ran out.
+template <int ND, int NDIAG, bool BLOCK>
+__device__ __forceinline__ bool issue_unit(uint32_t tmem, uint32_t width, uint64_t desc0, int slot_bytes, int digit_bytes,
+                                           uint64_t *full, uint64_t *empty, const Ring &r, uint32_t idesc, bool first_kb,
+                                           long long limit) {
     constexpr int D1 = ND - 1, D0 = ND - NDIAG, STEPS = D1 - (D0 + 1) / 2 + 1;
     uint64_t da[ND];
     bool ok = true;
+    if constexpr (BLOCK) {
+        ok = mbar_wait(&full[r.slot], r.phase, limit);
+#pragma unroll
+        for (int pos = 0; pos < ND; pos++)
+            da[digit_at(pos, ND)] = desc0 + (uint64_t)((r.slot * slot_bytes + pos * digit_bytes) >> 4);
+    }
 #pragma unroll
     for (int step = 0; step < STEPS; step++) {
         const int hi = D1 - step;
+        if constexpr (!BLOCK) {
 #pragma unroll
-        for (int pos = 2 * step; pos < 2 * step + 2; pos++) {
-            if (pos < ND) {
-                const Ring p = r.ahead(pos);
-                ok = ok && mbar_wait(&full[p.slot], p.phase, limit);
-                da[digit_at(pos, ND)] = desc0 + (uint64_t)(p.slot * (slot_bytes >> 4));
+            for (int pos = 2 * step; pos < 2 * step + 2; pos++) {
+                if (pos < ND) {
+                    const Ring p = r.ahead(pos);
+                    ok = ok && mbar_wait(&full[p.slot], p.phase, limit);
+                    da[digit_at(pos, ND)] = desc0 + (uint64_t)(p.slot * (slot_bytes >> 4));
+                }
             }
         }
         if (!ok) return false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (step == 0 || !BLOCK) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int d = D1; d >= D0; d--) {
             const int lo = d - hi;
@@ -395,37 +410,46 @@ __device__ __forceinline__ bool issue_unit(uint32_t tmem, uint32_t width, uint64
                     mma_i8_pair(acc, da[lo] + (uint64_t)(kk * 2), da[hi] + (uint64_t)((A_TILE >> 4) + kk * 2), idesc, 1u);
             }
         }
-        // positions 2 step (digit ND - 1 - step) and 2 (step - NDIAG + 1) + 1 (digit step - NDIAG + 1)
-        if (2 * step < ND) mma_commit_pair(&empty[r.ahead(2 * step).slot]);
-        const int low = 2 * (step - NDIAG + 1) + 1;
-        if (low > 0 && low < ND) mma_commit_pair(&empty[r.ahead(low).slot]);
+        if constexpr (!BLOCK) {
+            // positions 2 step (digit ND - 1 - step) and 2 (step - NDIAG + 1) + 1 (digit step - NDIAG + 1)
+            if (2 * step < ND) mma_commit_pair(&empty[r.ahead(2 * step).slot]);
+            const int low = 2 * (step - NDIAG + 1) + 1;
+            if (low > 0 && low < ND) mma_commit_pair(&empty[r.ahead(low).slot]);
+        }
     }
-    // what the last step leaves
+    if constexpr (BLOCK) {
+        mma_commit_pair(&empty[r.slot]);
+    } else {
+        // what the last step leaves
 #pragma unroll
-    for (int pos = 0; pos < ND; pos++) {
-        const bool freed = pos % 2 == 0 ? pos / 2 < STEPS : pos / 2 + NDIAG - 1 < STEPS;
-        if (!freed) mma_commit_pair(&empty[r.ahead(pos).slot]);
+        for (int pos = 0; pos < ND; pos++) {
+            const bool freed = pos % 2 == 0 ? pos / 2 < STEPS : pos / 2 + NDIAG - 1 < STEPS;
+            if (!freed) mma_commit_pair(&empty[r.ahead(pos).slot]);
+        }
     }
     return true;
 }
 
-// Units of an S-digit product: `wide` tiles (more than 128 columns) take the diagonals two at a time, others
-// four at a time; unit u stages the digits up to its highest diagonal.
-__device__ __forceinline__ int unit_digits(int u, int digits, bool wide) { return min((wide ? 2 : 4) * (u + 1), digits); }
+// Units of an S-digit product: wide tiles take the diagonals two at a time, others four at a time; unit u stages
+// the digits up to its highest diagonal.
+template <bool WIDE>
+__device__ __forceinline__ int unit_digits(int u, int digits) { return min((WIDE ? 2 : 4) * (u + 1), digits); }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(WTHREADS, 1)
 ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, OzMap map,
                   int num_tiles, double *__restrict__ scratch) {
+    constexpr int RING = PairRing<WIDE>::BYTES, WIDTH = WIDE ? WBN : WBN / 2;   // columns of an accumulator
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + WRING);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + RING);
     uint64_t *empty = full + WSLOTS;
     uint64_t *acc_full = empty + WSLOTS;
     uint64_t *acc_empty = acc_full + 1;   // used on CTA 0
     uint64_t *done = acc_empty + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    double *col_scales = reinterpret_cast<double *>(smem + WRING + 512);
+    double *col_scales = reinterpret_cast<double *>(smem + RING + 512);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const bool lead = rank == 0;
@@ -453,14 +477,16 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     cluster_sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const bool wide = map.bn > WBN / 2;
-    const int half = map.bn / 2, per = wide ? 2 : 4, units = (map.digits + per - 1) / per;
-    const int slot_bytes = A_TILE + half * OBK, n_slots = min(WSLOTS, WRING / slot_bytes);   // a slot: one digit of both
+    constexpr int per = WIDE ? 2 : 4;   // diagonals of a unit
+    const int half = map.bn / 2, units = (map.digits + per - 1) / per;
+    // a slot holds one digit of both operands, or all digits of a K block of a narrow tile
+    const int digit_bytes = A_TILE + half * OBK, slot_bytes = WIDE ? digit_bytes : map.digits * digit_bytes;
+    const int n_slots = min(WSLOTS, RING / slot_bytes);
 
     if (warp == 0) {
         if (lane == 0) {
-            // producer of this CTA: for every (tile, chunk, unit) the digits of each K block, a slot each
-            const uint32_t bytes = 2u * (uint32_t)(A_TILE + half * OBK);
+            // producer of this CTA: for every (tile, chunk, unit) the digits of each K block
+            const uint32_t bytes = 2u * (uint32_t)digit_bytes;
             Ring r{n_slots};
             int g = 0;
             for (int t = pair; t < num_tiles && !*abort_flag; t += npairs) {
@@ -470,19 +496,21 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 for (int c = 0; c < map.nchunks && !*abort_flag; c++) {
                     const int kb0 = c * map.kc, kb1 = min(map.nk_all, kb0 + map.kc);
                     for (int u = 0; u < units && !*abort_flag; u++) {
-                        const int nd = unit_digits(u, map.digits, wide);
+                        const int nd = unit_digits<WIDE>(u, map.digits), per_slot = WIDE ? 1 : nd;
                         for (int kb = kb0; kb < kb1 && !*abort_flag; kb++) {
-                            for (int pos = 0; pos < nd; pos++) {
+                            for (int pos = 0; pos < nd; pos += per_slot) {
                                 if (!mbar_wait(&empty[r.slot], r.phase ^ 1, map.wait_cycles)) {
                                     record_error(map.err, ERR_PRODUCER);
                                     *abort_flag = 1;
                                     break;
                                 }
                                 uint8_t *st = smem + r.slot * slot_bytes;
-                                const int q = digit_at(pos, nd);
-                                if (lead) mbar_expect_tx(&full[r.slot], bytes);
-                                tma_load_3d_pair(&tmA, &full[r.slot], st, kb * OBK, ma, q);
-                                tma_load_3d_pair(&tmB, &full[r.slot], st + A_TILE, kb * OBK, nb, q);
+                                if (lead) mbar_expect_tx(&full[r.slot], (uint32_t)per_slot * bytes);
+                                for (int p = pos; p < pos + per_slot; p++, st += digit_bytes) {
+                                    const int q = digit_at(p, nd);
+                                    tma_load_3d_pair(&tmA, &full[r.slot], st, kb * OBK, ma, q);
+                                    tma_load_3d_pair(&tmB, &full[r.slot], st + A_TILE, kb * OBK, nb, q);
+                                }
                                 r.advance(1);
                                 g++;
                             }
@@ -506,7 +534,7 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 for (int c = 0; c < map.nchunks && !*abort_flag; c++) {
                     const int kb0 = c * map.kc, kb1 = min(map.nk_all, kb0 + map.kc);
                     for (int u = 0; u < units && !*abort_flag; u++, uc++) {
-                        const int nd = unit_digits(u, map.digits, wide), diags = nd - per * u;
+                        const int nd = unit_digits<WIDE>(u, map.digits), diags = nd - per * u;
                         if (!mbar_wait(acc_empty, (uc & 1) ^ 1, map.wait_cycles)) {
                             record_error(map.err, ERR_MMA_ACC);
                             *abort_flag = 1;
@@ -518,14 +546,17 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                             bool ok = false;
 #define OZ_UNIT(ND, NDIAG)                                                                                        \
     case 8 * ND + NDIAG:                                                                                          \
-        ok = issue_unit<ND, NDIAG>(tmem, wide ? WBN : WBN / 2, desc0, slot_bytes, full, empty, r, idesc, first,   \
-                                   map.wait_cycles);                                                              \
+        ok = issue_unit<ND, NDIAG, !WIDE>(tmem, WIDTH, desc0, slot_bytes, digit_bytes, full, empty, r, idesc,     \
+                                          first, map.wait_cycles);                                                \
         break;
-                            switch (8 * nd + diags) {
-                                // two at a time: 2, 4, 6 digits, or the last diagonal of 5, 7
-                                OZ_UNIT(2, 2) OZ_UNIT(4, 2) OZ_UNIT(6, 2) OZ_UNIT(5, 1) OZ_UNIT(7, 1)
-                                // four at a time: four digits, then the rest of 6 or 7
-                                OZ_UNIT(4, 4) OZ_UNIT(7, 3)
+                            if constexpr (WIDE) {
+                                switch (8 * nd + diags) {   // 2, 4, 6 digits, or the last diagonal of 5, 7
+                                    OZ_UNIT(2, 2) OZ_UNIT(4, 2) OZ_UNIT(6, 2) OZ_UNIT(5, 1) OZ_UNIT(7, 1)
+                                }
+                            } else {
+                                switch (8 * nd + diags) {   // four digits, then the rest of 5, 6 or 7
+                                    OZ_UNIT(4, 4) OZ_UNIT(5, 1) OZ_UNIT(6, 2) OZ_UNIT(7, 3)
+                                }
                             }
 #undef OZ_UNIT
                             if (!ok || *abort_flag) {
@@ -533,7 +564,7 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                                 *abort_flag = 1;
                                 break;
                             }
-                            r.advance(nd);
+                            r.advance(WIDE ? nd : 1);
                         }
                         mma_commit_pair(acc_full);
                     }
@@ -573,13 +604,12 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const int d_lo = per * u, diags = unit_digits(u, map.digits, wide) - d_lo;
+                    const int d_lo = per * u, diags = unit_digits<WIDE>(u, map.digits) - d_lo;
                     // of a pass of four diagonals, the first unit and the last
                     const bool opens = d_lo % MAX_DIAG_PER_PASS == 0;
-                    const bool closes = !wide || u == units - 1 || u == 1;
+                    const bool closes = !WIDE || u == units - 1 || u == 1;
                     const bool first = c == 0 && d_lo < MAX_DIAG_PER_PASS;      // beta applies to the first pass
                     const bool read_c = closes && live && (!first || map.beta != 0.0);
-                    const uint32_t width = wide ? WBN : WBN / 2;
                     const double w0 = exp2(-7.0 * (double)(d_lo + 2));
                     const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16);
                     double ca[8], cb[8], pa[8], pb[8];   // output and scratch values of this step and the next
@@ -594,7 +624,7 @@ ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                         uint32_t acc[MAX_DIAG_PER_PASS][8];
 #pragma unroll
                         for (int h = 0; h < MAX_DIAG_PER_PASS; h++)   // diags is the same for every lane
-                            if (h < diags) tmem_ld8u_async(base + h * width + (uint32_t)cc, acc[h]);
+                            if (h < diags) tmem_ld8u_async(base + (uint32_t)(h * WIDTH + cc), acc[h]);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                         double v[8], w = w0;
 #pragma unroll
@@ -911,8 +941,9 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     // op(A)(r, kk): A[r + lda kk] (N) or A[kk + lda r] (T); op(B)(kk, c) rows c: B[kk + ldb c] (N) or B[c + ldb kk] (T)
     const int64_t a_sr = transA ? lda : 1, a_sk = transA ? 1 : lda;
     const int64_t b_sr = transB ? 1 : ldb, b_sk = transB ? ldb : 1;
-    // CTA pairs for every op(A) of more than one 128-row tile: a 256 x 256 pair tile stages half the bytes per
-    // product that four 128 x 128 tiles do, so that even a pair tile half empty costs no more than they.
+    // CTA pairs for every op(A) of more than one 128-row tile: a pair tile stages half the bytes per product that
+    // 128 x 128 tiles do, so that even one half empty costs less than they (six digits, single CTAs behind it:
+    // 129 x 4000 x 4000 0.14 ms, 0.22; 384 x 4000 x 4000 0.16, 0.23; 4400 x 400 x 40000 1.32, 1.66).
     // CCSD_GPU_PAIR_DIGITS=0 keeps single CTAs
     static const bool pairs_on = [] {
         const char *e = std::getenv("CCSD_GPU_PAIR_DIGITS");
@@ -922,7 +953,10 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     auto kernel = digits == 7 ? ozaki_gemm_kernel<7> : digits == 6 ? ozaki_gemm_kernel<6>
                 : digits == 5 ? ozaki_gemm_kernel<5> : ozaki_gemm_kernel<4>;
     CU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OSMEM));
-    CU_CHECK(cudaFuncSetAttribute(ozaki_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WSMEM));
+    CU_CHECK(cudaFuncSetAttribute(ozaki_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  PairRing<true>::SMEM));
+    CU_CHECK(cudaFuncSetAttribute(ozaki_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  PairRing<false>::SMEM));
     const int nsm = num_sms();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -931,7 +965,7 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(WTHREADS);
-    cfg.dynamicSmemBytes = WSMEM;
+    cfg.dynamicSmemBytes = PairRing<true>::SMEM;
     cfg.stream = ex.stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -944,7 +978,7 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
         if (mp == 0) {
             cfg.gridDim = dim3((unsigned)(2 * (nsm / 2)));
             int n = 0;
-            CU_CHECK(cudaOccupancyMaxActiveClusters(&n, ozaki_pair_kernel, &cfg));
+            CU_CHECK(cudaOccupancyMaxActiveClusters(&n, ozaki_pair_kernel<true>, &cfg));
             mp = std::max(1, n);
         }
         max_pairs = mp;
@@ -982,6 +1016,9 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
     else row_exponents(ex, B, b_sr, b_sk, n, k, Np, eb);
     const int64_t num_mt = pair ? round_up(m, (int64_t)(2 * OBM)) / (2 * OBM) : Mp / OBM;
     const int bn = pair ? pair_n_tile(num_mt, n, digits, max_pairs) : OBN;
+    const bool wide = bn > WBN / 2;
+    auto pkernel = wide ? ozaki_pair_kernel<true> : ozaki_pair_kernel<false>;
+    cfg.dynamicSmemBytes = wide ? PairRing<true>::SMEM : PairRing<false>::SMEM;
     for (int64_t k0 = 0; k0 < k; k0 += kslab) {
         const int64_t kk = std::min(kslab, k - k0), Kp = round_up(kk, OBK);
         if (!pa) slab_digits(ex, A + k0 * a_sk, a_sr, a_sk, m, kk, Mp, Kp, digits, ea, da);
@@ -1026,7 +1063,7 @@ void ozaki_gemm(Exec &ex, bool transA, bool transB, int64_t m, int64_t n, int64_
         }
         if (pair) {
             cfg.gridDim = dim3((unsigned)(2 * grid));
-            CU_CHECK(cudaLaunchKernelEx(&cfg, ozaki_pair_kernel, ta, tb, map, num_tiles, scratch));
+            CU_CHECK(cudaLaunchKernelEx(&cfg, pkernel, ta, tb, map, num_tiles, scratch));
         } else {
             kernel<<<grid, OTHREADS, OSMEM, ex.stream>>>(ta, tb, map, num_tiles);
             CU_CHECK(cudaGetLastError());
