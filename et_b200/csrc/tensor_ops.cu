@@ -755,9 +755,9 @@ void run_batch(Exec &ex, const BatchPlan &p, const TV &A, const TV &B, const TV 
     const TV Au = p.copyA ? make_contiguous(ex, A, p.a1, p.a2, bufA) : A;
     const TV Bu = p.copyB ? make_contiguous(ex, B, p.b1, p.b2, bufB) : B;
     if (trace_level() >= 2)
-        std::fprintf(stderr, "ccsd_gpu gemm [%s] fp64 batch %lld x %lld m %lld n %lld k %lld\n",
+        std::fprintf(stderr, "ccsd_gpu gemm [%s] fp64 batch %lld x %lld m %lld n %lld k %lld%s%s%s\n",
                      g_perm_tag ? g_perm_tag : "direct", (long long)p.nw, (long long)p.nz, (long long)p.m, (long long)p.n,
-                     (long long)p.k);
+                     (long long)p.k, p.swap ? " swap" : "", p.copyA ? " copyA" : "", p.copyB ? " copyB" : "");
     for (int64_t w = 0; w < p.nw; w++) {
         const double *a = Au.p + w * p.wA, *b = Bu.p + w * p.wB;
         double *c = C.p + w * p.wC;
