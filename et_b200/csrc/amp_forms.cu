@@ -167,11 +167,6 @@ __device__ __forceinline__ void put_planes(double x, int np, int64_t plane, __nv
     }
 }
 
-// An occupied pair i >= j and a 32 x 32 tile of (c, d), c >= d: t_cidj lies along d in its packed row
-// (c, i), t_cjdi along c in row (d, i), turned in shared memory; both forms are stored along d.  Bound by
-// HBM: n_t2 read, the forms written; each thread of the element-wise version found its four indices by two
-// square roots and read two elements whose neighbours lay a packed row apart.  bf16 planes at o=32, v=320
-// 0.34 ms (1.9 TB/s; 0.38 with the padding), 0.54 without MIN_BLOCKS.
 // The padding of one form's planes: K positions beyond the k pairs cd and rows beyond the used ones (ld is a
 // multiple of 8), shared out over the whole grid.  As up to four 2-D memsets before the kernel a residual at o=13,
 // v=107 took 1.081 ms, so 1.067; from o=16, v=128 on it makes no difference.
@@ -190,6 +185,11 @@ __device__ __forceinline__ void clear_pads(__nv_bfloat16 *t, int np, int64_t row
     }
 }
 
+// An occupied pair i >= j and a 32 x 32 tile of (c, d), c >= d: t_cidj lies along d in its packed row
+// (c, i), t_cjdi along c in row (d, i), turned in shared memory; both forms are stored along d.  Bound by
+// HBM: n_t2 read, the forms written; each thread of the element-wise version found its four indices by two
+// square roots and read two elements whose neighbours lay a packed row apart.  bf16 planes at o=32, v=320
+// 0.34 ms (1.9 TB/s; 0.38 with the padding), 0.54 without MIN_BLOCKS.
 template <bool PLANES>
 __global__ void __launch_bounds__(TILE * ROWS, MIN_BLOCKS)
 tpm_forms_kernel(const double *__restrict__ packed, int no, int nv, int64_t nvec, TpmOut o) {

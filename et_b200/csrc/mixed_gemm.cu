@@ -1007,10 +1007,9 @@ void launch_pair(Exec &ex, const __nv_bfloat16 *A, int64_t a_rows, int64_t a_pla
     }
 }
 
-// CTA pairs for two-plane FP64-output products with at least one full pair tile of rows, when
-// CCSD_GPU_PAIR_GEMM=1.  Off by default: at 10240^3 the pair runs at the single-CTA kernel's speed
-// (4.77 vs 4.75 ms, both near the power-capped bf16 rate), and the 256-row tiles pad the ladder's
-// 528-row operand further than 128-row tiles do.
+// CCSD_GPU_PAIR_GEMM=1 puts every two-plane FP64-output product of at least 256 rows on CTA pairs.  Off by default:
+// at 10240^3 the pair runs at the single-CTA kernel's speed (4.77 vs 4.75 ms, both near the power-capped bf16
+// rate); the measured routes and the ladder's rule (tc_tall_route) take pairs where they are faster.
 bool pair_gemm_on() {
     static const bool on = [] {
         const char *e = std::getenv("CCSD_GPU_PAIR_GEMM");

@@ -53,10 +53,11 @@ __global__ void permute_simple_kernel(PermArgs a, int64_t total, double alpha, c
     }
 }
 
-// Rows of the output-fastest dim (dim 0, at least 16 long): a warp takes a row or a segment of a long one, so the division chain that locates it in the other dims runs once per row instead of once per element,
-// and both sides stream along dim 0 (this kernel serves permutations whose input-fastest dim is dim
-// 0 as well, or whose other dims are too short for the tiled transpose).  Bound by HBM or, for rows of a few
-// hundred, by loads in flight: four per lane.
+// Rows of the output-fastest dim (dim 0, at least 16 long): a warp takes a row or a segment of a long one, so the
+// division chain that locates it in the other dims runs once per row instead of once per element, and both sides
+// stream along dim 0 (this kernel serves permutations whose input-fastest dim is dim 0 as well, or whose other
+// dims are too short for the tiled transpose).  Bound by HBM or, for rows of a few hundred, by loads in flight:
+// four per lane.
 template <class I>
 __global__ void __launch_bounds__(256) permute_rows_kernel(PermArgs a, int64_t nwork, int nseg, int seg, double alpha,
                                                            const double *__restrict__ in, double beta,
