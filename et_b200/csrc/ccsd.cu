@@ -834,7 +834,9 @@ bool Context::f64_ladder_planes(int digits) {
     if (f.version == f64_version && f.digits == digits) return f.held;
     not_captured();
     const int64_t nvp = nv * (nv + 1) / 2, nvm = nv * (nv - 1) / 2;
-    for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig}) p->buf.release();
+    // the planes of g_kcpd are decided again after these: both share the bound
+    for (OzPlanes *p : {&f64_gp_dig, &f64_gm_dig, &f64_ovvv_dig}) p->buf.release();
+    f64_ovvv_fit = DigitFit{};
     size_t free_b = 0, total_b = 0;
     CU_CHECK(cudaMemGetInfo(&free_b, &total_b));
     const double need = digit_bytes(digits, nvp, nvp) + (nvm > 0 ? digit_bytes(digits, nvm, nvm) : 0.0);
